@@ -287,17 +287,18 @@ __global__ void __launch_bounds__(kScanWarps * 32) k_scan(EncParams p) {
 }
 
 // Table builders by leaf count (k_leafTiers sorts the tables, k_tableBuild
-// builds them): the heap merge is a latency-bound chain on one thread, so a
+// builds them): the heap merge is a latency-bound chain on one warp, so a
 // smaller table gets a smaller CTA and heap and more of them share an SM.
-//   tier 0: up to 256 leaves, a warp, 5 KB of heap (32 per SM)
-//   tier 1: up to 1024 leaves, 64 threads, 20 KB (11 per SM)
-//   tier 2: up to 2048 leaves, 256 threads, 41 KB (5 per SM)
+//   tier 0: up to 256 leaves, a warp, 3 KB of heap (32 per SM)
+//   tier 1: up to 1024 leaves, 64 threads, 12 KB (16 per SM)
+//   tier 2: up to 2048 leaves, 256 threads, 25 KB (8 per SM)
 //   tier 3: more, 256 threads, the full heap (one per SM)
 constexpr u32 kTinyLeaves = 256;
 constexpr u32 kSmallLeaves = 1024;
 constexpr u32 kBuildSplitLeaves = 2048;
 constexpr int kTinySegs = int(kTinyLeaves / 17u) + 1;    // sort segments longer than 16 keys
 constexpr int kSmallSegs = int(kSmallLeaves / 17u) + 1;
+constexpr int kMidSegs = int(kBuildSplitLeaves / 17u) + 1;
 constexpr u32 kBuildEach = 0xFFFFFFFFu;                  // buildTier: one table per CTA
 constexpr u32 kTierMinTables = 64;                       // calls of more tables use the tiers
 
@@ -712,21 +713,23 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     // i that word is the low half of a device pointer when 2+2i < S (nonzero),
     // else the all-zero run-length scan output.
     const bool quirkLeaf = isZc && sAllEmpty && (2u + 2u * (td.stream - es.groupFirst) < es.groupSize);
-    // 2. leaves in symbol order: heap keys go straight to the shared-memory
-    //    heap (1-based, see table_build.cuh) when the table fits
+    // 2. leaves in symbol order: straight into the shared-memory heap
+    //    (1-based, see heap_merge.cuh) when the table fits
     u32* leafSym = p.leafSymWork + meta.leafOff;
     u64* heapG = p.leafWork + meta.leafOff;
-    u64* H = reinterpret_cast<u64*>(dyn);                                        // [heapCap + 2]
-    u32* parentS = reinterpret_cast<u32*>(dyn + sizeof(u64) * (p.heapCap + 2));  // [2 heapCap]
-    u32* orderS = parentS + 2 * p.heapCap;                                       // [heapCap]
+    const hm::Layout at(p.heapCap);
+    u32* heapP = reinterpret_cast<u32*>(dyn);
+    u16* heapI = reinterpret_cast<u16*>(dyn + at.ids);
+    const u16* parentS = reinterpret_cast<const u16*>(dyn + at.parents);
+    u32* orderS = heapP;   // takes the probabilities' place after the merge
+    const u32 smemLeaves = count < hm::kInf - 1u ? p.heapCap : 0u;
     u32 L;
     if (quirkLeaf) {
         L = 1;
         if (L < p.buildLo || L > p.buildHi) return;   // uniform: the other build launch has it
         if (threadIdx.x == 0) {
             leafSym[0] = 0;
-            const u64 key = (u64(1) << 32) | 0u;
-            if (L <= p.heapCap) H[1] = key; else heapG[0] = key;
+            if (L > smemLeaves) heapG[0] = u64(1) << 32;
         }
     } else if (count == 0) {
         L = 0;
@@ -741,28 +744,30 @@ __device__ void buildTable(const EncParams& p, u32 t) {
         u32 off = blockExclusiveSum<kThreads>(c, sScan, &tot);
         L = tot;
         if (L < p.buildLo || L > p.buildHi) return;
-        const bool toSmem = L <= p.heapCap;
+        const bool toSmem = L <= smemLeaves;
         const bool quirk65535 = p.symBytes == 2 && p.bins == 65536u && symbolMax == 65535u;
         for (u32 b = b0; b < b1; ++b) {
             u32 h = hist[b];
             if (h) {
                 if (quirk65535 && b == 65535u) h += count & 1u;   // HistogramKernels.cui:165,200 padding word
                 leafSym[off] = b;
-                const u64 key = (u64(h) << 32) | off;
-                if (toSmem) H[off + 1] = key; else heapG[off] = key;
+                if (toSmem) {
+                    heapP[off + 1] = h;
+                    heapI[off + 1] = u16(off);
+                } else {
+                    heapG[off] = (u64(h) << 32) | off;
+                }
                 ++off;
             }
         }
     }
-    const bool inSmem = L <= p.heapCap;
+    const bool inSmem = L <= smemLeaves;
     u32* order = inSmem ? orderS : p.orderWork + meta.leafOff;
     if (threadIdx.x == 0) sMaxLen = 0;
     __syncthreads();
     // 3. tree, depths and sort
     if (inSmem) {
-        if (L >= 2) tb::blockMakeHeap(H, int(L));
-        if (threadIdx.x == 0 && L >= 2) tb::buildTree(H, parentS, int(L));
-        __syncthreads();
+        if (L >= 2) tb::blockBuildTree(dyn, p.heapCap, L);
         const u32 root = L >= 2 ? 2 * L - 2 : 0;
         u32 localMax = 0;
         for (u32 i = threadIdx.x; i < L; i += kThreads) {
@@ -774,9 +779,10 @@ __device__ void buildTable(const EncParams& p, u32 t) {
         if (localMax) atomicMax(&sMaxLen, localMax);
         __syncthreads();
         if (sMaxLen <= 31) {
-            u16* lList = reinterpret_cast<u16*>(dyn);            // reuses the heap area (5 bytes per key)
-            u16* rList = lList + p.heapCap;
-            u8* mark = reinterpret_cast<u8*>(rList + p.heapCap);
+            // the ids', tails' and parents' places (9 bytes per key with the order)
+            u16* lList = heapI;
+            u16* rList = reinterpret_cast<u16*>(dyn + at.tails);
+            u8* mark = dyn + at.parents;
             tb::blockIntrosort<kThreads>(order, int(L), lList, rList, mark, sSegA, sSegB, sSegCount);
         }
     } else if (threadIdx.x == 0) {
@@ -1320,7 +1326,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         k_write<Sym><<<p.totalTiles, kRleThreads, writeSmem<Sym>(), st>>>(p);
         countLaunch();
     }
-    size_t buildSmem = sizeof(u64) * (p.heapCap + 2) + 3 * sizeof(u32) * size_t(p.heapCap);
+    size_t buildSmem = hm::Layout(p.heapCap).bytes;
     // an instance whose tables run beside other kernels (the batched codec's
     // lowpass encode) may ask for an SM of its own per table: the sequential
     // heap merge is latency-bound and loses issue slots to co-resident CTAs
@@ -1337,7 +1343,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         q.buildTier = kBuildEach;
         const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
         const bool solo = I->tableBuildSoloSM && p.T <= sms;
-        auto heapBytes = [](u32 cap) { return sizeof(u64) * (cap + 2) + 3 * sizeof(u32) * size_t(cap); };
+        auto heapBytes = [](u32 cap) { return size_t(hm::Layout(cap).bytes); };
         // a call of few tables builds them in one launch, a CTA each (the
         // tiers' pre-pass, launches and stream forks would cost it more than
         // they save)
@@ -1357,7 +1363,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
                 small.buildHi = kSmallLeaves;
                 small.heapCap = std::min(p.heapCap, kSmallLeaves);
                 k_tableBuild<64u, kSmallSegs>
-                    <<<std::min(p.T, 10u * sms), 64, heapBytes(small.heapCap), I->buildSide2>>>(small);
+                    <<<std::min(p.T, 16u * sms), 64, heapBytes(small.heapCap), I->buildSide2>>>(small);
                 countLaunch();
                 CC_TRY_CUDA(cudaEventRecord(I->buildJoin2, I->buildSide2), "table build join");
             }
@@ -1376,8 +1382,8 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
                 mid.buildLo = kSmallLeaves + 1;
                 mid.buildHi = kBuildSplitLeaves;
                 mid.heapCap = std::min(p.heapCap, kBuildSplitLeaves);
-                k_tableBuild<kBuildThreads, tb::kMaxSegs>
-                    <<<std::min(p.T, 5u * sms), kBuildThreads, heapBytes(mid.heapCap), I->buildSide>>>(mid);
+                k_tableBuild<kBuildThreads, kMidSegs>
+                    <<<std::min(p.T, 8u * sms), kBuildThreads, heapBytes(mid.heapCap), I->buildSide>>>(mid);
                 countLaunch();
                 CC_TRY_CUDA(cudaEventRecord(I->buildJoin, I->buildSide), "table build join");
             }
@@ -1442,7 +1448,7 @@ int prepareDecodeAttributes(cc_instance* I);
 
 int prepareKernelAttributes(cc_instance* I) {
     const u32 heapCap = std::min<u32>(I->leavesMax, kBuildSmemLeaves);
-    size_t buildSmem = sizeof(u64) * (heapCap + 2) + 3 * sizeof(u32) * size_t(heapCap);
+    size_t buildSmem = hm::Layout(heapCap).bytes;
     if (I->tableBuildSoloSM) buildSmem = std::max(buildSmem, tableBuildSoloSmem(I->device));
     CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, tb::kMaxSegs>),
                                     kAttrTableBuild, I->device, buildSmem),

@@ -2,11 +2,115 @@
 // exported for the CPU unit tests (tests/test_table_build_host.py), which
 // compare it with the oracle on many histograms.  Not part of the product
 // library: it is built into _lib/libcc_selftest.so and loaded only by tests.
+#include <algorithm>
 #include <cstring>
 #include <vector>
+#include "heap_merge.cuh"
 #include "huffman_build.cuh"
 
 using namespace ccb;
+
+namespace {
+
+// heap_merge.cuh's warp as 32-element arrays over a bounds-checked memory.
+struct LaneU { u32 v[32]; };
+struct LaneB { bool v[32]; };
+
+struct HostWarp {
+    using U = LaneU;
+    using B = LaneB;
+    u8* mem;
+    u32 bytes;
+    bool* bad;
+    template <class F> static U each(F f) { U r; for (u32 i = 0; i < 32; ++i) r.v[i] = f(i); return r; }
+    template <class F> static B test(F f) { B r; for (u32 i = 0; i < 32; ++i) r.v[i] = f(i); return r; }
+    U lane() const { return each([](u32 i) { return i; }); }
+    U all(u32 x) const { return each([=](u32) { return x; }); }
+    u32 first(const U& a) const { return a.v[0]; }
+    B le(const U& a, const U& b) const { return test([&](u32 i) { return a.v[i] <= b.v[i]; }); }
+    B lt(const U& a, const U& b) const { return test([&](u32 i) { return a.v[i] < b.v[i]; }); }
+    B eq(const U& a, const U& b) const { return test([&](u32 i) { return a.v[i] == b.v[i]; }); }
+    B nz(const U& a) const { return test([&](u32 i) { return a.v[i] != 0; }); }
+    B both(const B& a, const B& b) const { return test([&](u32 i) { return a.v[i] && b.v[i]; }); }
+    U sel(const B& c, const U& a, const U& b) const { return each([&](u32 i) { return c.v[i] ? a.v[i] : b.v[i]; }); }
+    U min(const U& a, const U& b) const { return each([&](u32 i) { return std::min(a.v[i], b.v[i]); }); }
+    U max(const U& a, const U& b) const { return each([&](u32 i) { return std::max(a.v[i], b.v[i]); }); }
+    U sub(const U& a, const U& b) const { return each([&](u32 i) { return a.v[i] - b.v[i]; }); }
+    U add(const U& a, const U& b) const { return each([&](u32 i) { return a.v[i] + b.v[i]; }); }
+    U shr(const U& a, const U& n) const { return each([&](u32 i) { return a.v[i] >> n.v[i]; }); }
+    U shr(const U& a, u32 n) const { return each([&](u32 i) { return a.v[i] >> n; }); }
+    U shl(const U& a, u32 n) const { return each([&](u32 i) { return a.v[i] << n; }); }
+    U shlv(const U& a, const U& n) const { return each([&](u32 i) { return a.v[i] << n.v[i]; }); }
+    U lo16(const U& a) const { return each([&](u32 i) { return a.v[i] & 0xFFFFu; }); }
+    U hi16(const U& a) const { return each([&](u32 i) { return a.v[i] >> 16; }); }
+    U andv(const U& a, const U& b) const { return each([&](u32 i) { return a.v[i] & b.v[i]; }); }
+    U orv(const U& a, const U& b) const { return each([&](u32 i) { return a.v[i] | b.v[i]; }); }
+    U xorv(const U& a, const U& b) const { return each([&](u32 i) { return a.v[i] ^ b.v[i]; }); }
+    U lastSet(const U& m) const { return each([&](u32 i) { return m.v[i] ? 31u - u32(__builtin_clz(m.v[i])) : ~0u; }); }
+    u32 ballot(const B& c) const { u32 m = 0; for (u32 i = 0; i < 32; ++i) m |= u32(c.v[i]) << i; return m; }
+    u32 reduceMin(const U& a) const { return *std::min_element(a.v, a.v + 32); }
+    U shfl(const U& a, const U& from) const { return each([&](u32 i) { return a.v[from.v[i] & 31u]; }); }
+    void fence() const {}
+    template <class T> T* at(u32 off) const {
+        static u64 sink;
+        if (u64(off) + sizeof(T) > bytes || off % sizeof(T)) { *bad = true; return reinterpret_cast<T*>(&sink); }
+        return reinterpret_cast<T*>(mem + off);
+    }
+    void ldPair(const U& o, U& x, U& y) const {
+        for (u32 i = 0; i < 32; ++i) if (o.v[i] % 8) *bad = true;
+        x = ld32(o);
+        y = ld32(add(o, all(4)));
+    }
+    U ld32(const U& o) const { return each([&](u32 i) { return *at<u32>(o.v[i]); }); }
+    U ld16(u32 array, const U& o) const { return each([&](u32 i) { return u32(*at<u16>(array + o.v[i])); }); }
+    U ld16Pair(u32 array, const U& o) const { return each([&](u32 i) { return *at<u32>(array + o.v[i]); }); }
+    u32 ldOne32(u32 o) const { return *at<u32>(o); }
+    u32 ldOne16(u32 o) const { return *at<u16>(o); }
+    void st32(const U& o, const U& x, const B& c) const {
+        for (u32 i = 0; i < 32; ++i) if (c.v[i]) *at<u32>(o.v[i]) = x.v[i];
+    }
+    void st16(u32 array, const U& o, const U& x, const B& c) const {
+        for (u32 i = 0; i < 32; ++i) {
+            if (!c.v[i]) continue;
+            if (x.v[i] > 0xFFFFu) *bad = true;
+            *at<u16>(array + o.v[i]) = u16(x.v[i]);
+        }
+    }
+    void stParent(u32 array, const U& id, u32 x) const { *at<u16>(array + 2u * id.v[31]) = u16(x); }
+};
+
+}  // namespace
+
+// Parent links of the tree over L >= 2 leaf probabilities, by the warp's merge
+// loop (warpParents) and by the sequential libstdc++ replay (seqParents); 0,
+// or -1 after an access outside the layout's area.
+extern "C" int ccst_heap_merge(const u32* probs, u32 L, u32* warpParents, u32* seqParents) {
+    std::vector<u64> heap(L);
+    for (u32 i = 0; i < L; ++i) heap[i] = (u64(probs[i]) << 32) | i;
+    std::vector<u64> seq(heap);
+    std::vector<u32> par(2 * L, 0);
+    hb::buildTree(seq.data(), par.data(), int(L));
+    hb::makeHeap(heap.data(), int(L), hb::ProbInvLess());
+    const hm::Layout at(L);
+    std::vector<u64> area(at.bytes / 8 + 1, 0xAAAAAAAAAAAAAAAAull);
+    u8* m = reinterpret_cast<u8*>(area.data());
+    u32* P = reinterpret_cast<u32*>(m);
+    u16* I = reinterpret_cast<u16*>(m + at.ids);
+    u16* T = reinterpret_cast<u16*>(m + at.tails);
+    const u16* up = reinterpret_cast<const u16*>(m + at.parents);
+    P[0] = hm::kInf;
+    for (u32 i = 0; i < L; ++i) { P[i + 1] = u32(heap[i] >> 32); I[i + 1] = u16(heap[i]); }
+    const u32 D = hm::log2Floor(L);
+    for (u32 k = L; k >= 1; --k) {
+        const u32 c = 2 * k;
+        T[k] = c > L ? u16(k << (D - hm::log2Floor(k))) : (c == L || P[c] < P[c + 1]) ? T[c] : T[c + 1];
+    }
+    bool bad = false;
+    hm::Merge<HostWarp> merge(HostWarp{m, at.bytes, &bad}, L, L);
+    merge.run(L);
+    for (u32 i = 0; i + 2 < 2 * L; ++i) { warpParents[i] = up[i]; seqParents[i] = par[i]; }
+    return bad ? -1 : 0;
+}
 
 extern "C" int ccst_huffman_build(const u32* hist, u32 bins, u32 symbolMax, u32 log2Max, u32* codewords,
                                   u32* lengths, u32* tableWords, u32 cap, u32* tableBits) {

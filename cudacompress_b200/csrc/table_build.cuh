@@ -3,10 +3,9 @@
 // 487-596, libstdc++ priority_queue + std::sort) with the work a block can
 // share done by the block.
 //
-//  * tree: make_heap runs level by level over the block; the merge loop
-//    stays sequential (one thread) on a shared-memory heap laid out 1-based
-//    so that the two children of a node are one aligned 16-byte load, with
-//    the grandchildren loaded speculatively beside them;
+//  * tree: make_heap runs level by level over the block; the merge loop, a
+//    chain of pops and pushes, runs on one warp with a lane per heap level
+//    (heap_merge.cuh);
 //  * depths: one thread per leaf walks to the root;
 //  * sort: std::sort's introsort is replayed exactly, but every partition
 //    step runs on a warp: the left scan stops at the k-th element not less
@@ -19,148 +18,86 @@
 //    it and the insertion only moves past strictly greater elements).
 #pragma once
 
+#include "heap_merge.cuh"
 #include "huffman_build.cuh"
 
 namespace ccb {
 namespace tb {
 
 // ---------------------------------------------------------------------------
-// Tree (HuffmanTable.cu:507-529).  H[i + 1] holds heap element i, i.e. the
-// heap is 1-based inside H; H must be 16-byte aligned and hold L + 2 entries.
-// Elements: (probability << 32) | node id; "less(a, b)" is b.prob < a.prob
-// (the top is the smallest probability; ties are not broken by id, so the
-// result depends on the exact libstdc++ heap moves, which are replayed).
-// Writes parent[id] for every node except the root.
+// Tree (HuffmanTable.cu:507-529): probabilities P and ids I of heap_merge.cuh's
+// layout, 1-based (node k holds heap element k - 1).  "less(a, b)" is b.prob <
+// a.prob (the top is the smallest probability; ties are not broken by id, so
+// the result depends on the exact libstdc++ heap moves, which are replayed).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ u32 probOf(u64 v) { return u32(v >> 32); }
 
 // make_heap (libstdc++ __make_heap): __adjust_heap of every parent from
-// (len-2)/2 down to 0.  Parents at one depth have disjoint subtrees and all
+// len / 2 down to 1.  Parents at one depth have disjoint subtrees and all
 // deeper parents come first in that order, so the parents of one depth are
-// adjusted in parallel, deepest depth first, with the same result.  All
-// threads of the block.
-__device__ void blockMakeHeap(u64* H, int len) {
-    if (len < 2) return;
-    const int lastParent = (len - 2) / 2;
-    for (int d = 31 - __clz(lastParent + 1); d >= 0; --d) {
-        const int first = (1 << d) - 1, last = min(2 * first, lastParent);
-        for (int p = first + int(threadIdx.x); p <= last; p += int(blockDim.x))
-            hb::adjustHeap(H + 1, p, len, H[p + 1], hb::ProbInvLess());
+// adjusted in parallel, deepest depth first, with the same result.  The hole
+// of an adjustment sinks along the smaller children and the value rises again
+// from the leaf; that path ascends, so stopping at the first child above the
+// value places it the same.  All threads of the block.
+__device__ void blockMakeHeap(u32* P, u16* I, u32 len) {
+    for (int d = 31 - __clz(len / 2); d >= 0; --d) {
+        const u32 first = 1u << d, last = min(2u * first - 1u, len / 2u);
+        for (u32 node = first + threadIdx.x; node <= last; node += blockDim.x) {
+            const u32 v = P[node];
+            const u16 id = I[node];
+            u32 hole = node;
+            while (2u * hole <= len) {
+                u32 c = 2u * hole;
+                if (c < len && !(P[c] < P[c + 1])) ++c;   // the right child unless the left is strictly smaller
+                const u32 cp = P[c];
+                if (v < cp) break;
+                P[hole] = cp;
+                I[hole] = I[c];
+                hole = c;
+            }
+            P[hole] = v;
+            I[hole] = id;
+        }
         __syncthreads();
     }
 }
 
-__device__ __forceinline__ ulonglong2 ld2(const u64* H, int i) { return *reinterpret_cast<const ulonglong2*>(H + i); }
-
-// pop_heap on H[1..n+1] (libstdc++ __pop_heap: the last element v goes
-// through __adjust_heap(first, 0, n, v) and __push_heap); returns the top.
-// One thread.  The sift-down resolves two levels per step: the children and
-// both grandchild pairs are loaded together (capEven: the largest even index
-// e with H[e + 1] inside the array clamps the speculative loads).  The
-// push-up compares v with the last two values moved up, still in registers.
-__device__ __forceinline__ u64 popTop(u64* H, int n, int capEven) {
-    const u64 top = H[1];
-    if (n <= 0) return top;
-    const u64 v = H[n + 1];
-    const u32 pv = probOf(v);
-    const int lim = (n - 1) / 2;
-    int hole = 0;
-    u64 w1 = 0, w2 = 0;   // values moved into the hole's parent and grandparent
-    while (hole < lim) {
-        const int c = 2 * hole + 2;   // right child; the pair (c-1, c) is H[c], H[c+1]
-        const ulonglong2 pr = ld2(H, c);
-        const ulonglong2 gl = ld2(H, min(2 * c, capEven));
-        const ulonglong2 gr = ld2(H, min(2 * c + 2, capEven));
-        const bool left = probOf(pr.x) < probOf(pr.y);   // less(right, left)
-        const u64 cv = left ? pr.x : pr.y;
-        H[hole + 1] = cv;
-        hole = left ? c - 1 : c;
-        w2 = w1;
-        w1 = cv;
-        if (hole >= lim) break;
-        const ulonglong2 q = left ? gl : gr;
-        const bool left2 = probOf(q.x) < probOf(q.y);
-        const u64 cv2 = left2 ? q.x : q.y;
-        H[hole + 1] = cv2;
-        hole = 2 * hole + (left2 ? 1 : 2);
-        w2 = w1;
-        w1 = cv2;
-    }
-    if ((n & 1) == 0 && hole == (n - 2) / 2) {
-        const u64 cv = H[2 * hole + 2];
-        H[hole + 1] = cv;
-        hole = 2 * hole + 1;
-        w2 = w1;
-        w1 = cv;
-    }
-    if (hole > 0 && pv < probOf(w1)) {
-        H[hole + 1] = w1;
-        hole = (hole - 1) / 2;
-        if (hole > 0 && pv < probOf(w2)) {
-            H[hole + 1] = w2;
-            hole = (hole - 1) / 2;
-            while (hole > 0) {
-                const int parent = (hole - 1) / 2;
-                const u64 pe = H[parent + 1];
-                if (!(pv < probOf(pe))) break;
-                H[hole + 1] = pe;
-                hole = parent;
-            }
+// The tails of a heap: the bottom end of every node's path of smaller children.
+__device__ void blockTails(const u32* P, u16* T, u32 len) {
+    const u32 D = hm::log2Floor(len);
+    for (int d = int(D); d >= 0; --d) {
+        const u32 first = 1u << d, last = min(2u * first - 1u, len);
+        for (u32 node = first + threadIdx.x; node <= last; node += blockDim.x) {
+            const u32 c = 2u * node;
+            T[node] = c > len ? u16(node << (D - d)) : (c == len || P[c] < P[c + 1]) ? T[c] : T[c + 1];
         }
+        __syncthreads();
     }
-    H[hole + 1] = v;
-    return top;
 }
 
-// push_heap of v as element len-1 (__push_heap); three ancestors per step are
-// loaded together.
-__device__ __forceinline__ void pushLast(u64* H, int len, u64 v) {
-    int hole = len - 1;
-    const u32 pv = probOf(v);
-    while (hole > 0) {
-        const int p1 = (hole - 1) / 2, p2 = p1 > 0 ? (p1 - 1) / 2 : 0, p3 = p2 > 0 ? (p2 - 1) / 2 : 0;
-        const u64 e1 = H[p1 + 1], e2 = H[p2 + 1], e3 = H[p3 + 1];
-        if (!(pv < probOf(e1))) break;
-        H[hole + 1] = e1;
-        hole = p1;
-        if (hole == 0 || !(pv < probOf(e2))) break;
-        H[hole + 1] = e2;
-        hole = p2;
-        if (hole == 0 || !(pv < probOf(e3))) break;
-        H[hole + 1] = e3;
-        hole = p3;
+// The tree of L >= 2 leaves (P and I of nodes 1 .. L in symbol order): parent
+// links in the layout's parents.  All threads of the block.
+__device__ void blockBuildTree(unsigned char* area, u32 leavesCap, u32 L) {
+    const hm::Layout at(leavesCap);
+    u32* P = reinterpret_cast<u32*>(area);
+    if (threadIdx.x == 0) P[0] = hm::kInf;
+    blockMakeHeap(P, reinterpret_cast<u16*>(area + at.ids), L);
+    blockTails(P, reinterpret_cast<u16*>(area + at.tails), L);
+    if (threadIdx.x < 32) {
+        hm::Merge<hm::DeviceWarp> m(hm::DeviceWarp(area), leavesCap, L);
+        m.run(L);
     }
-    H[hole + 1] = v;
-}
-
-// The merge loop (HuffmanTable.cu:512-529) on a heap made by blockMakeHeap.
-// One thread; H holds L + 2 entries.
-__device__ void buildTree(u64* H, u32* parent, int L) {
-    const int capEven = L & ~1;
-    int len = L;
-    u32 next = u32(L);
-    while (len > 1) {
-        const u64 a = popTop(H, len - 1, capEven);
-        --len;
-        const u64 b = popTop(H, len - 1, capEven);
-        --len;
-        parent[u32(a)] = next;
-        parent[u32(b)] = next;
-        const u64 node = (u64(probOf(a) + probOf(b)) << 32) | next;
-        ++next;
-        ++len;
-        pushLast(H, len, node);
-    }
+    __syncthreads();
 }
 
 // ---------------------------------------------------------------------------
 // Sort (HuffmanTable.cu:538, libstdc++ std::sort) of keys (len << 27 | leaf).
 // ---------------------------------------------------------------------------
 struct Seg {
-    int f, l, d;
+    u16 f, l;
+    int d;
 };
 constexpr int kSortThreshold = 16;
-constexpr int kMaxSegs = 512;   // segments longer than 16 of up to 8192 keys
+constexpr int kMaxSegs = int(hm::kMergeLeavesMax) / 17 + 1;   // segments longer than 16 keys
 
 __device__ __forceinline__ u32 keyOf(u32 v) { return v >> 27; }
 
@@ -211,7 +148,7 @@ __device__ int warpPartition(u32* a, int f, int l, u16* lList, u16* rList) {
     return cut;
 }
 
-// Block-cooperative introsort of a[0, n) (n <= 8192).  Scratch: lList, rList
+// Block-cooperative introsort of a[0, n) (n <= 16384).  Scratch: lList, rList
 // (n u16 each), mark (n bytes), two segment queues.  All threads call it.
 template <int kThreads>
 __device__ void blockIntrosort(u32* a, int n, u16* lList, u16* rList, u8* mark, Seg* qA, Seg* qB, int* counters) {
@@ -221,7 +158,7 @@ __device__ void blockIntrosort(u32* a, int n, u16* lList, u16* rList, u8* mark, 
     if (threadIdx.x == 0) {
         counters[0] = 0;
         if (n > kSortThreshold) {
-            qA[0] = Seg{0, n, 2 * hb::floorLog2(n)};
+            qA[0] = Seg{0, u16(n), 2 * hb::floorLog2(n)};
             counters[0] = 1;
         }
     }
@@ -252,7 +189,7 @@ __device__ void blockIntrosort(u32* a, int n, u16* lList, u16* rList, u8* mark, 
             __syncwarp();
             const int cut = warpPartition(a, g.f, g.l, lList, rList);
             if (lane == 0) {
-                const Seg kids[2] = {Seg{g.f, cut, g.d - 1}, Seg{cut, g.l, g.d - 1}};
+                const Seg kids[2] = {Seg{g.f, u16(cut), g.d - 1}, Seg{u16(cut), g.l, g.d - 1}};
                 for (int k = 0; k < 2; ++k) {
                     if (kids[k].l - kids[k].f > kSortThreshold) nxt[atomicAdd(&counters[1], 1)] = kids[k];
                     else if (kids[k].l > kids[k].f) mark[kids[k].f] = 1;
