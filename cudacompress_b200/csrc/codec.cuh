@@ -36,10 +36,10 @@ constexpr u32 kRunSymbols = 1024;
 constexpr u32 kPlanChunk = 4096;
 constexpr u64 planPartWords(u64 tables) { return 8 * ((tables + kPlanChunk - 1) / kPlanChunk + 1); }
 
-// Leaves of a table whose Huffman build runs in shared memory (12 bytes per
-// leaf: heap_merge.cuh's layout, whose place the sort takes afterwards); larger
-// tables use global memory.
-constexpr u32 kBuildSmemLeaves = 16384;
+// Leaves of a table whose Huffman build runs in shared memory (heap_merge.cuh's
+// layout, 213 KB, whose place the sort takes afterwards); larger tables use
+// global memory.
+constexpr u32 kBuildSmemLeaves = 12288;
 
 // Words of a serialized table with `leaves` symbols (HuffmanTable.cu:470-485
 // field sizes at their maxima: 31 codeword lengths, 24-bit symbols) plus two

@@ -53,7 +53,7 @@ struct EncParams {
     u32* leafSymWork;
     u32* tierTables;  // [4][T]: the tables of each leaf-count tier (k_leafTiers); counts in totals[4..7]
     u64* planPart;    // [8 per chunk]: sums of each plan chunk (k_histPlan)
-    u32 heapCap;      // leaves that fit the shared-memory builder of tableBuild
+    u32 heapCap;      // bound of the call's leaf counts (at most kBuildSmemLeaves)
     u32 buildLo, buildHi;   // k_tableBuild builds the tables with buildLo <= leaves <= buildHi
     u32 buildTier;    // k_tableBuild: kBuildEach (table blockIdx.x) or the tier whose list its CTAs walk
 };
@@ -289,16 +289,13 @@ __global__ void __launch_bounds__(kScanWarps * 32) k_scan(EncParams p) {
 // Table builders by leaf count (k_leafTiers sorts the tables, k_tableBuild
 // builds them): the heap merge is a latency-bound chain on one warp, so a
 // smaller table gets a smaller CTA and heap and more of them share an SM.
-//   tier 0: up to 256 leaves, a warp, 3 KB of heap (32 per SM)
-//   tier 1: up to 1024 leaves, 64 threads, 12 KB (16 per SM)
-//   tier 2: up to 2048 leaves, 256 threads, 25 KB (8 per SM)
+//   tier 0: up to 256 leaves, a warp, 5 KB of heap (32 per SM)
+//   tier 1: up to 1024 leaves, 64 threads, 20 KB (10 per SM)
+//   tier 2: up to 2048 leaves, 256 threads, 41 KB (5 per SM)
 //   tier 3: more, 256 threads, the full heap (one per SM)
 constexpr u32 kTinyLeaves = 256;
 constexpr u32 kSmallLeaves = 1024;
 constexpr u32 kBuildSplitLeaves = 2048;
-constexpr int kTinySegs = int(kTinyLeaves / 17u) + 1;    // sort segments longer than 16 keys
-constexpr int kSmallSegs = int(kSmallLeaves / 17u) + 1;
-constexpr int kMidSegs = int(kBuildSplitLeaves / 17u) + 1;
 constexpr u32 kBuildEach = 0xFFFFFFFFu;                  // buildTier: one table per CTA
 constexpr u32 kTierMinTables = 64;                       // calls of more tables use the tiers
 
@@ -678,10 +675,10 @@ __device__ __forceinline__ void putBits(u32* words, u32 pos, u32 value, u32 coun
 }
 
 // Builds table t (all kThreads threads of the block; returns uniformly).
-// kSegs: the sort's segment queue (segments longer than 16 keys in a round:
-// at most heapCap / 17).
-template <u32 kThreads, int kSegs>
+// Tables of up to kCap leaves are built in shared memory.
+template <u32 kThreads, u32 kCap>
 __device__ void buildTable(const EncParams& p, u32 t) {
+    constexpr int kSegs = int(kCap / 17u) + 1;   // the sort's queue: segments longer than 16 keys
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ u32 sScan[40];
     __shared__ u32 sMax, sMaxLen, sAllEmpty;
@@ -717,12 +714,12 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     //    (1-based, see heap_merge.cuh) when the table fits
     u32* leafSym = p.leafSymWork + meta.leafOff;
     u64* heapG = p.leafWork + meta.leafOff;
-    const hm::Layout at(p.heapCap);
+    using At = hm::Layout<kCap>;
     u32* heapP = reinterpret_cast<u32*>(dyn);
-    u16* heapI = reinterpret_cast<u16*>(dyn + at.ids);
-    const u16* parentS = reinterpret_cast<const u16*>(dyn + at.parents);
+    u32* heapI = reinterpret_cast<u32*>(dyn + At::kIds);
+    const u16* parentS = reinterpret_cast<const u16*>(dyn + At::kParents);
     u32* orderS = heapP;   // takes the probabilities' place after the merge
-    const u32 smemLeaves = count < hm::kInf - 1u ? p.heapCap : 0u;
+    const u32 smemLeaves = count < hm::kInf - 1u ? kCap : 0u;
     u32 L;
     if (quirkLeaf) {
         L = 1;
@@ -753,7 +750,7 @@ __device__ void buildTable(const EncParams& p, u32 t) {
                 leafSym[off] = b;
                 if (toSmem) {
                     heapP[off + 1] = h;
-                    heapI[off + 1] = u16(off);
+                    heapI[off + 1] = 2u * off;
                 } else {
                     heapG[off] = (u64(h) << 32) | off;
                 }
@@ -767,7 +764,7 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     __syncthreads();
     // 3. tree, depths and sort
     if (inSmem) {
-        if (L >= 2) tb::blockBuildTree(dyn, p.heapCap, L);
+        if (L >= 2) tb::blockBuildTree<kCap>(dyn, L);
         const u32 root = L >= 2 ? 2 * L - 2 : 0;
         u32 localMax = 0;
         for (u32 i = threadIdx.x; i < L; i += kThreads) {
@@ -779,10 +776,10 @@ __device__ void buildTable(const EncParams& p, u32 t) {
         if (localMax) atomicMax(&sMaxLen, localMax);
         __syncthreads();
         if (sMaxLen <= 31) {
-            // the ids', tails' and parents' places (9 bytes per key with the order)
-            u16* lList = heapI;
-            u16* rList = reinterpret_cast<u16*>(dyn + at.tails);
-            u8* mark = dyn + at.parents;
+            // the ids' and the tails' places
+            u16* lList = reinterpret_cast<u16*>(heapI);
+            u16* rList = lList + kCap;
+            u8* mark = dyn + At::kTails;
             tb::blockIntrosort<kThreads>(order, int(L), lList, rList, mark, sSegA, sSegB, sSegCount);
         }
     } else if (threadIdx.x == 0) {
@@ -865,16 +862,16 @@ __device__ void buildTable(const EncParams& p, u32 t) {
 }
 
 // One table per CTA (kBuildEach), or the CTAs walk the list of one tier.
-template <u32 kThreads, int kSegs>
+template <u32 kThreads, u32 kCap>
 __global__ void __launch_bounds__(kThreads) k_tableBuild(EncParams p) {
     if (p.buildTier == kBuildEach) {
-        buildTable<kThreads, kSegs>(p, blockIdx.x);
+        buildTable<kThreads, kCap>(p, blockIdx.x);
         return;
     }
     const u32 n = u32(p.totals[4 + p.buildTier]);
     const u32* list = p.tierTables + u64(p.buildTier) * p.T;
     for (u32 i = blockIdx.x; i < n; i += gridDim.x) {
-        buildTable<kThreads, kSegs>(p, list[i]);
+        buildTable<kThreads, kCap>(p, list[i]);
         __syncthreads();   // the next table reuses the shared memory
     }
 }
@@ -889,7 +886,7 @@ static size_t tableBuildSoloSmem(int device) {
         int optin = 0;
         cudaFuncAttributes fa{};
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-        cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, tb::kMaxSegs>));
+        cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, kBuildSmemLeaves>));
         cached[device] = optin > int(fa.sharedSizeBytes) ? size_t(optin) - fa.sharedSizeBytes : 0;
     }
     return cached[device];
@@ -1326,13 +1323,14 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         k_write<Sym><<<p.totalTiles, kRleThreads, writeSmem<Sym>(), st>>>(p);
         countLaunch();
     }
-    size_t buildSmem = hm::Layout(p.heapCap).bytes;
+    const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
     // an instance whose tables run beside other kernels (the batched codec's
     // lowpass encode) may ask for an SM of its own per table: the sequential
     // heap merge is latency-bound and loses issue slots to co-resident CTAs
-    if (I->tableBuildSoloSM && p.T <= u32(std::max(1, I->smCount > 0 ? I->smCount : 148)))
-        buildSmem = std::max(buildSmem, tableBuildSoloSmem(I->device));
-    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, tb::kMaxSegs>),
+    const bool solo = I->tableBuildSoloSM && p.T <= sms;
+    size_t buildSmem = hm::Layout<kBuildSmemLeaves>::kBytes;
+    if (solo) buildSmem = std::max(buildSmem, tableBuildSoloSmem(I->device));
+    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, kBuildSmemLeaves>),
                                     kAttrTableBuild, I->device, buildSmem),
                 "tableBuild smem");
     {
@@ -1341,9 +1339,6 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         q.buildLo = 0;
         q.buildHi = ~0u;
         q.buildTier = kBuildEach;
-        const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
-        const bool solo = I->tableBuildSoloSM && p.T <= sms;
-        auto heapBytes = [](u32 cap) { return size_t(hm::Layout(cap).bytes); };
         // a call of few tables builds them in one launch, a CTA each (the
         // tiers' pre-pass, launches and stream forks would cost it more than
         // they save)
@@ -1361,9 +1356,8 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
                 small.buildTier = 1;
                 small.buildLo = kTinyLeaves + 1;
                 small.buildHi = kSmallLeaves;
-                small.heapCap = std::min(p.heapCap, kSmallLeaves);
-                k_tableBuild<64u, kSmallSegs>
-                    <<<std::min(p.T, 16u * sms), 64, heapBytes(small.heapCap), I->buildSide2>>>(small);
+                k_tableBuild<64u, kSmallLeaves>
+                    <<<std::min(p.T, 10u * sms), 64, hm::Layout<kSmallLeaves>::kBytes, I->buildSide2>>>(small);
                 countLaunch();
                 CC_TRY_CUDA(cudaEventRecord(I->buildJoin2, I->buildSide2), "table build join");
             }
@@ -1373,7 +1367,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
                     EncParams big = q;
                     big.buildTier = 3;
                     big.buildLo = kBuildSplitLeaves + 1;
-                    k_tableBuild<kBuildThreads, tb::kMaxSegs>
+                    k_tableBuild<kBuildThreads, kBuildSmemLeaves>
                         <<<std::min(p.T, sms), kBuildThreads, buildSmem, I->buildSide>>>(big);
                     countLaunch();
                 }
@@ -1381,22 +1375,28 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
                 mid.buildTier = 2;
                 mid.buildLo = kSmallLeaves + 1;
                 mid.buildHi = kBuildSplitLeaves;
-                mid.heapCap = std::min(p.heapCap, kBuildSplitLeaves);
-                k_tableBuild<kBuildThreads, kMidSegs>
-                    <<<std::min(p.T, 8u * sms), kBuildThreads, heapBytes(mid.heapCap), I->buildSide>>>(mid);
+                k_tableBuild<kBuildThreads, kBuildSplitLeaves>
+                    <<<std::min(p.T, 5u * sms), kBuildThreads, hm::Layout<kBuildSplitLeaves>::kBytes, I->buildSide>>>(mid);
                 countLaunch();
                 CC_TRY_CUDA(cudaEventRecord(I->buildJoin, I->buildSide), "table build join");
             }
             EncParams tiny = q;
             tiny.buildTier = 0;
             tiny.buildHi = kTinyLeaves;
-            tiny.heapCap = std::min(p.heapCap, kTinyLeaves);
-            k_tableBuild<32u, kTinySegs><<<std::min(p.T, 32u * sms), 32, heapBytes(tiny.heapCap), st>>>(tiny);
+            k_tableBuild<32u, kTinyLeaves>
+                <<<std::min(p.T, 32u * sms), 32, hm::Layout<kTinyLeaves>::kBytes, st>>>(tiny);
             countLaunch();
             if (side2) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->buildJoin2, 0), "table build join");
             if (side) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->buildJoin, 0), "table build join");
         } else {
-            k_tableBuild<kBuildThreads, tb::kMaxSegs><<<p.T, kBuildThreads, buildSmem, st>>>(q);
+            if (!solo && p.heapCap <= kSmallLeaves)
+                k_tableBuild<kBuildThreads, kSmallLeaves>
+                    <<<p.T, kBuildThreads, hm::Layout<kSmallLeaves>::kBytes, st>>>(q);
+            else if (!solo && p.heapCap <= kBuildSplitLeaves)
+                k_tableBuild<kBuildThreads, kBuildSplitLeaves>
+                    <<<p.T, kBuildThreads, hm::Layout<kBuildSplitLeaves>::kBytes, st>>>(q);
+            else
+                k_tableBuild<kBuildThreads, kBuildSmemLeaves><<<p.T, kBuildThreads, buildSmem, st>>>(q);
             countLaunch();
         }
     }
@@ -1447,10 +1447,9 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
 int prepareDecodeAttributes(cc_instance* I);
 
 int prepareKernelAttributes(cc_instance* I) {
-    const u32 heapCap = std::min<u32>(I->leavesMax, kBuildSmemLeaves);
-    size_t buildSmem = hm::Layout(heapCap).bytes;
+    size_t buildSmem = hm::Layout<kBuildSmemLeaves>::kBytes;
     if (I->tableBuildSoloSM) buildSmem = std::max(buildSmem, tableBuildSoloSmem(I->device));
-    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, tb::kMaxSegs>),
+    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, kBuildSmemLeaves>),
                                     kAttrTableBuild, I->device, buildSmem),
                 "tableBuild smem");
     if (I->symBytes == 2)

@@ -41,8 +41,8 @@ struct HostWarp {
     U shr(const U& a, u32 n) const { return each([&](u32 i) { return a.v[i] >> n; }); }
     U shl(const U& a, u32 n) const { return each([&](u32 i) { return a.v[i] << n; }); }
     U shlv(const U& a, const U& n) const { return each([&](u32 i) { return a.v[i] << n.v[i]; }); }
-    U lo16(const U& a) const { return each([&](u32 i) { return a.v[i] & 0xFFFFu; }); }
-    U hi16(const U& a) const { return each([&](u32 i) { return a.v[i] >> 16; }); }
+    U min3(const U& a, const U& b, const U& c) const { return min(a, min(b, c)); }
+    U below(const U& a) const { return each([&](u32 i) { return a.v[i] - 1u + (a.v[i] >> 31); }); }
     U andv(const U& a, const U& b) const { return each([&](u32 i) { return a.v[i] & b.v[i]; }); }
     U orv(const U& a, const U& b) const { return each([&](u32 i) { return a.v[i] | b.v[i]; }); }
     U xorv(const U& a, const U& b) const { return each([&](u32 i) { return a.v[i] ^ b.v[i]; }); }
@@ -56,60 +56,67 @@ struct HostWarp {
         if (u64(off) + sizeof(T) > bytes || off % sizeof(T)) { *bad = true; return reinterpret_cast<T*>(&sink); }
         return reinterpret_cast<T*>(mem + off);
     }
-    void ldPair(const U& o, U& x, U& y) const {
-        for (u32 i = 0; i < 32; ++i) if (o.v[i] % 8) *bad = true;
-        x = ld32(o);
-        y = ld32(add(o, all(4)));
+    template <u32 A> void ldPair(const U& o, U& x, U& y) const {
+        for (u32 i = 0; i < 32; ++i) if ((A + o.v[i]) % 8) *bad = true;
+        x = ld<A>(o);
+        y = ld<A + 4u>(o);
     }
-    U ld32(const U& o) const { return each([&](u32 i) { return *at<u32>(o.v[i]); }); }
-    U ld16(u32 array, const U& o) const { return each([&](u32 i) { return u32(*at<u16>(array + o.v[i])); }); }
-    U ld16Pair(u32 array, const U& o) const { return each([&](u32 i) { return *at<u32>(array + o.v[i]); }); }
-    u32 ldOne32(u32 o) const { return *at<u32>(o); }
-    u32 ldOne16(u32 o) const { return *at<u16>(o); }
-    void st32(const U& o, const U& x, const B& c) const {
-        for (u32 i = 0; i < 32; ++i) if (c.v[i]) *at<u32>(o.v[i]) = x.v[i];
+    template <u32 A> U ld(const U& o) const { return each([&](u32 i) { return *at<u32>(A + o.v[i]); }); }
+    template <u32 A> u32 ldOne(u32 o) const { return *at<u32>(A + o); }
+    template <u32 A> void st(const U& o, const U& x, const B& c) const {
+        for (u32 i = 0; i < 32; ++i) if (c.v[i]) *at<u32>(A + o.v[i]) = x.v[i];
     }
-    void st16(u32 array, const U& o, const U& x, const B& c) const {
-        for (u32 i = 0; i < 32; ++i) {
-            if (!c.v[i]) continue;
-            if (x.v[i] > 0xFFFFu) *bad = true;
-            *at<u16>(array + o.v[i]) = u16(x.v[i]);
-        }
-    }
-    void stParent(u32 array, const U& id, u32 x) const { *at<u16>(array + 2u * id.v[31]) = u16(x); }
+    template <u32 A> void stAll(u32 o, u32 x) const { *at<u32>(A + o) = x; }
+    template <u32 A> void stParent(const U& id2, u32 x) const { *at<u16>(A + id2.v[31]) = u16(x); }
 };
 
 }  // namespace
 
+// The warp's merge loop over a heap of L leaves in a layout of kCap.
+template <u32 kCap>
+static bool warpMerge(const std::vector<u64>& heap, u32 L, u32* parents) {
+    using At = hm::Layout<kCap>;
+    std::vector<u64> area(At::kBytes / 8 + 1, 0xAAAAAAAAAAAAAAAAull);
+    u8* m = reinterpret_cast<u8*>(area.data());
+    u32* P = reinterpret_cast<u32*>(m);
+    u32* I = reinterpret_cast<u32*>(m + At::kIds);
+    u32* T = reinterpret_cast<u32*>(m + At::kTails);
+    const u16* up = reinterpret_cast<const u16*>(m + At::kParents);
+    const u32 D = hm::log2Floor(L);
+    for (u32 i = 0; i < (2u << D); ++i) P[i] = hm::kInf;
+    P[At::kNodes] = P[At::kNodes + 1] = hm::kInf;
+    for (u32 i = 0; i < L; ++i) { P[i + 1] = u32(heap[i] >> 32); I[i + 1] = 2u * u32(heap[i]); }
+    for (u32 k = L; k >= 1; --k) {
+        const u32 c = 2 * k;
+        T[k] = c > L ? 4u * (k << (D - hm::log2Floor(k))) : (c == L || P[c] < P[c + 1]) ? T[c] : T[c + 1];
+    }
+    bool bad = false;
+    hm::Merge<HostWarp, kCap> merge(HostWarp{m, At::kBytes, &bad}, L);
+    merge.run(L);
+    for (u32 i = 0; i + 2 < 2 * L; ++i) parents[i] = up[i];
+    return bad;
+}
+
 // Parent links of the tree over L >= 2 leaf probabilities, by the warp's merge
-// loop (warpParents) and by the sequential libstdc++ replay (seqParents); 0,
-// or -1 after an access outside the layout's area.
-extern "C" int ccst_heap_merge(const u32* probs, u32 L, u32* warpParents, u32* seqParents) {
+// loop in a layout of `cap` leaves (warpParents) and by the sequential
+// libstdc++ replay (seqParents); 0, -1 after an access outside the layout's
+// area, -2 for a capacity that is not built.
+extern "C" int ccst_heap_merge(const u32* probs, u32 L, u32 cap, u32* warpParents, u32* seqParents) {
     std::vector<u64> heap(L);
     for (u32 i = 0; i < L; ++i) heap[i] = (u64(probs[i]) << 32) | i;
     std::vector<u64> seq(heap);
     std::vector<u32> par(2 * L, 0);
     hb::buildTree(seq.data(), par.data(), int(L));
+    std::memcpy(seqParents, par.data(), sizeof(u32) * (2 * L - 2));
     hb::makeHeap(heap.data(), int(L), hb::ProbInvLess());
-    const hm::Layout at(L);
-    std::vector<u64> area(at.bytes / 8 + 1, 0xAAAAAAAAAAAAAAAAull);
-    u8* m = reinterpret_cast<u8*>(area.data());
-    u32* P = reinterpret_cast<u32*>(m);
-    u16* I = reinterpret_cast<u16*>(m + at.ids);
-    u16* T = reinterpret_cast<u16*>(m + at.tails);
-    const u16* up = reinterpret_cast<const u16*>(m + at.parents);
-    P[0] = hm::kInf;
-    for (u32 i = 0; i < L; ++i) { P[i + 1] = u32(heap[i] >> 32); I[i + 1] = u16(heap[i]); }
-    const u32 D = hm::log2Floor(L);
-    for (u32 k = L; k >= 1; --k) {
-        const u32 c = 2 * k;
-        T[k] = c > L ? u16(k << (D - hm::log2Floor(k))) : (c == L || P[c] < P[c + 1]) ? T[c] : T[c + 1];
+    if (L > cap) return -2;
+    switch (cap) {
+        case 256: return -int(warpMerge<256>(heap, L, warpParents));
+        case 1024: return -int(warpMerge<1024>(heap, L, warpParents));
+        case 2048: return -int(warpMerge<2048>(heap, L, warpParents));
+        case 12288: return -int(warpMerge<12288>(heap, L, warpParents));
+        default: return -2;
     }
-    bool bad = false;
-    hm::Merge<HostWarp> merge(HostWarp{m, at.bytes, &bad}, L, L);
-    merge.run(L);
-    for (u32 i = 0; i + 2 < 2 * L; ++i) { warpParents[i] = up[i]; seqParents[i] = par[i]; }
-    return bad ? -1 : 0;
 }
 
 extern "C" int ccst_huffman_build(const u32* hist, u32 bins, u32 symbolMax, u32 log2Max, u32* codewords,

@@ -38,12 +38,12 @@ namespace tb {
 // of an adjustment sinks along the smaller children and the value rises again
 // from the leaf; that path ascends, so stopping at the first child above the
 // value places it the same.  All threads of the block.
-__device__ void blockMakeHeap(u32* P, u16* I, u32 len) {
+__device__ void blockMakeHeap(u32* P, u32* I, u32 len) {
     for (int d = 31 - __clz(len / 2); d >= 0; --d) {
         const u32 first = 1u << d, last = min(2u * first - 1u, len / 2u);
         for (u32 node = first + threadIdx.x; node <= last; node += blockDim.x) {
             const u32 v = P[node];
-            const u16 id = I[node];
+            const u32 id = I[node];
             u32 hole = node;
             while (2u * hole <= len) {
                 u32 c = 2u * hole;
@@ -61,29 +61,34 @@ __device__ void blockMakeHeap(u32* P, u16* I, u32 len) {
     }
 }
 
-// The tails of a heap: the bottom end of every node's path of smaller children.
-__device__ void blockTails(const u32* P, u16* T, u32 len) {
+// The tails (x 4) of a heap: the bottom end of every node's path of smaller
+// children.
+__device__ void blockTails(const u32* P, u32* T, u32 len) {
     const u32 D = hm::log2Floor(len);
     for (int d = int(D); d >= 0; --d) {
         const u32 first = 1u << d, last = min(2u * first - 1u, len);
         for (u32 node = first + threadIdx.x; node <= last; node += blockDim.x) {
             const u32 c = 2u * node;
-            T[node] = c > len ? u16(node << (D - d)) : (c == len || P[c] < P[c + 1]) ? T[c] : T[c + 1];
+            T[node] = c > len ? 4u * (node << (D - d)) : (c == len || P[c] < P[c + 1]) ? T[c] : T[c + 1];
         }
         __syncthreads();
     }
 }
 
-// The tree of L >= 2 leaves (P and I of nodes 1 .. L in symbol order): parent
-// links in the layout's parents.  All threads of the block.
-__device__ void blockBuildTree(unsigned char* area, u32 leavesCap, u32 L) {
-    const hm::Layout at(leavesCap);
-    u32* P = reinterpret_cast<u32*>(area);
+// The tree of 2 <= L <= kCap leaves (P and I of nodes 1 .. L in symbol order,
+// in the block's dynamic shared memory): parent links in the layout's parents.
+// All threads of the block.
+template <u32 kCap>
+__device__ void blockBuildTree(unsigned char* dyn, u32 L) {
+    using At = hm::Layout<kCap>;
+    u32* P = reinterpret_cast<u32*>(dyn);
+    for (u32 i = L + 1 + threadIdx.x; i < (2u << hm::log2Floor(L)); i += blockDim.x) P[i] = hm::kInf;
+    if (threadIdx.x < 2) P[At::kNodes + threadIdx.x] = hm::kInf;
     if (threadIdx.x == 0) P[0] = hm::kInf;
-    blockMakeHeap(P, reinterpret_cast<u16*>(area + at.ids), L);
-    blockTails(P, reinterpret_cast<u16*>(area + at.tails), L);
+    blockMakeHeap(P, reinterpret_cast<u32*>(dyn + At::kIds), L);
+    blockTails(P, reinterpret_cast<u32*>(dyn + At::kTails), L);
     if (threadIdx.x < 32) {
-        hm::Merge<hm::DeviceWarp> m(hm::DeviceWarp(area), leavesCap, L);
+        hm::Merge<hm::DeviceWarp, kCap> m(hm::DeviceWarp(), L);
         m.run(L);
     }
     __syncthreads();
@@ -97,7 +102,6 @@ struct Seg {
     int d;
 };
 constexpr int kSortThreshold = 16;
-constexpr int kMaxSegs = int(hm::kMergeLeavesMax) / 17 + 1;   // segments longer than 16 keys
 
 __device__ __forceinline__ u32 keyOf(u32 v) { return v >> 27; }
 

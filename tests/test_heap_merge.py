@@ -26,15 +26,18 @@ def test_warp_merge_matches_sequential_replay(pattern):
         pytest.skip("self-test library not built")
     f = st.ccst_heap_merge
     u32p = ctypes.POINTER(ctypes.c_uint32)
-    f.argtypes = [u32p, ctypes.c_uint32, u32p, u32p]
+    f.argtypes = [u32p, ctypes.c_uint32, ctypes.c_uint32, u32p, u32p]
     rng = np.random.default_rng(5)
     # around every tree depth's edge, odd sizes, and the largest heap
     sizes = list(range(2, 70)) + [127, 128, 129, 255, 256, 257, 1000, 1023, 1024, 1025, 2047, 2048, 4097]
     if pattern in ("few values", "log-uniform"):
-        sizes += [8191, 8192, 8193, 16383, 16384]
+        sizes += [8191, 8192, 8193, 12287, 12288]
     for n in sizes:
         p = np.ascontiguousarray(PATTERNS[pattern](rng, n), np.uint32)
-        got, want = np.zeros(2 * n, np.uint32), np.zeros(2 * n, np.uint32)
-        rc = f(p.ctypes.data_as(u32p), n, got.ctypes.data_as(u32p), want.ctypes.data_as(u32p))
-        assert rc == 0, n
-        assert np.array_equal(got, want), n
+        for cap in (256, 1024, 2048, 12288):     # the builders' capacities
+            if n > cap or (cap == 12288 and n < 1000 and n % 7):
+                continue
+            got, want = np.zeros(2 * n, np.uint32), np.zeros(2 * n, np.uint32)
+            rc = f(p.ctypes.data_as(u32p), n, cap, got.ctypes.data_as(u32p), want.ctypes.data_as(u32p))
+            assert rc == 0, (n, cap)
+            assert np.array_equal(got, want), (n, cap)
