@@ -929,7 +929,7 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
                     T += 2; blocks += 2 * nb; ++nRl; rlB += nb;
                     ++hS; hT += 2; hTiles += nt; hBlocks += 2 * nb;
                 } else {
-                    T += 1; blocks += nb; ++nH; hB += nb;
+                    T += 1; blocks += nb; ++nH; hB += huffBlocksPlanned(nb);
                     lTiles += nt; lBlocks += nb;
                 }
             }

@@ -147,7 +147,8 @@ enum SmemAttrKernel {
     kAttrDecHuff32,
     kAttrWrite16,
     kAttrWrite32,
-    kAttrCount
+    kAttrDecRl,   // 8 variants
+    kAttrCount = kAttrDecRl + 8
 };
 cudaError_t ensureSmemAttribute(const void* kernel, int which, int device, size_t bytes);
 // Sets the largest shared memory the encoder and decoder kernels may ask for

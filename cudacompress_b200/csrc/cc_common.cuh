@@ -37,6 +37,8 @@ CC_HD u32 requiredBits(u32 v) { return v ? 32u - u32(__builtin_clz(v)) : 0u; }
 
 CC_HD u64 ceilDiv(u64 a, u64 b) { return (a + b - 1) / b; }
 CC_HD u64 alignUp(u64 a, u64 b) { return (a + b - 1) / b * b; }
+// Coding blocks of n symbols, 2^log each (kernels take no 64-bit division for them).
+CC_HD u32 blocksOf(u32 n, u32 log) { return (n >> log) + ((n & ((1u << log) - 1u)) ? 1u : 0u); }
 
 #ifdef __CUDACC__
 // Inclusive warp scan (sum).
@@ -104,6 +106,31 @@ __device__ __forceinline__ u32 blockExclusiveSum(u32 v, u32* scratch, u32* total
     if (total) *total = scratch[32];
     __syncthreads();
     return r;
+}
+
+// Exclusive scan of in[0, n) by a whole CTA, each thread summing eight
+// consecutive elements per step; returns the total (all threads).  `scratch`
+// holds >= 33 u32.
+template <int kThreads>
+__device__ __forceinline__ u32 blockExclusiveScan8(const u32* in, u32* out, u32 n, u32* scratch) {
+    u32 carry = 0;
+    for (u32 base = 0; base < n; base += 8u * kThreads) {
+        const u32 i0 = base + 8u * threadIdx.x;
+        u32 v[8], sum = 0, tot;
+#pragma unroll
+        for (u32 k = 0; k < 8; ++k) {
+            v[k] = i0 + k < n ? in[i0 + k] : 0u;
+            sum += v[k];
+        }
+        u32 run = carry + blockExclusiveSum<kThreads>(sum, scratch, &tot);
+#pragma unroll
+        for (u32 k = 0; k < 8; ++k) {
+            if (i0 + k < n) out[i0 + k] = run;
+            run += v[k];
+        }
+        carry += tot;
+    }
+    return carry;
 }
 
 // Block-wide exclusive scans of N values per thread at once (two barriers

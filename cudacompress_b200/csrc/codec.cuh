@@ -28,7 +28,8 @@ constexpr u32 kRlePerThread = 32;
 constexpr u32 kRleTile = kRleThreads * kRlePerThread;
 // The Huffman block kernels take coding blocks in runs of kRunSymbols symbols
 // of one table (32 per lane of a warp): 1024 / codingBlockSize blocks.
-constexpr u32 kRunSymbols = 1024;
+constexpr u32 kRunLog = 10;
+constexpr u32 kRunSymbols = 1u << kRunLog;
 
 // Tables planned by one CTA of the encode's and decode's table plans (1024
 // threads, four tables each); a call of more tables runs one CTA per chunk
@@ -174,6 +175,10 @@ struct DecStreamDesc {
     u32 blockFirst;   // first of its blocks among the streams of its kind
 };
 
+// Numbers the plan of a decode gives a Huff stream of `blocks` coding blocks:
+// whole warps of 32.
+CC_HD u32 huffBlocksPlanned(u32 blocks) { return (blocks + 31u) / 32u * 32u; }
+
 // Decode tables in device memory: canonical description + fast lookup.
 constexpr u32 kLutBits = 10;
 struct DecTable {
@@ -199,7 +204,8 @@ struct cc_instance {
     // the small-table launch on `stream` (fork / join by the two events)
     cudaStream_t buildSide = nullptr, buildSide2 = nullptr;   // the table builders' other streams
     cudaEvent_t buildFork = nullptr, buildJoin = nullptr, buildJoin2 = nullptr;
-    cudaEvent_t decFork = nullptr, decJoin = nullptr;   // the decode's Huff branch on buildSide2
+    // the decode's zero fill and Huff branch on buildSide2
+    cudaEvent_t decFork = nullptr, decZeroed = nullptr, decTablesReady = nullptr, decJoin = nullptr;
 
     // derived sizes
     ccb::u32 bins = 0;          // 1 << log2Max

@@ -9,7 +9,7 @@
 //    decode parses them on the host too and returns before the GPU work is
 //    done - and stages the touched words once;
 //  * decodePrepare / decodeLaunch (batched volume codec, device-resident bit
-//    streams): one thread per bit stream walks its headers on the device, so
+//    streams): one warp per bit stream walks its headers on the device, so
 //    nothing goes through the host and the launches can be replayed.
 // Back end, one launch per stage over the whole batch (coding blocks are
 // numbered across the streams of a kind and found back by binary search):
@@ -28,7 +28,7 @@ struct DecParams {
     u32 S, T, nSrc, nRl, nH;
     u32 rlBlocks, hBlocks;     // coding blocks (upper bounds) of the RLHuff / Huff streams
     u32 rlMaxN;                // largest output of an RLHuff stream
-    u32 cb, log2Max, symBytes, leavesMax;
+    u32 cb, cbLog, log2Max, symBytes, leavesMax;   // cb = 2^cbLog
     u64 capLeaves;
     DecStreamDesc* streams;
     DecTableDesc* tables;
@@ -87,55 +87,103 @@ __device__ __forceinline__ u32 streamOfBlock(const DecParams& p, const u32* list
 // Device walk (HuffmanTable.cu:117-151 header fields, Encode.cpp:473-646 /
 // 792-917 stream layout, BitStream.h:290-308 alignment).
 // ---------------------------------------------------------------------------
+// A bit stream's reader: the walk is a chain of short reads, so the calling
+// warp (every lane with the same values) reads through a window of 128 words
+// in shared memory, loaded 16 bytes per lane wherever a read leaves it - one
+// round trip per header for most tables, whose code lengths, symbols and code
+// word count then come out of the window.  Word indices are 32-bit (a stream
+// holds at most 2^31 symbols of 31 bits).  Three 256^3 streams (43 tables
+// each): 37 us, against 56 with 64-bit positions and divisions by the coding
+// block, and 81 for a thread per stream reading word by word.
+constexpr u32 kWalkWindow = 128;
+
 struct DevReader {
-    const u32* w;
-    u64 nWords, size, pos;
-    bool ok;
-    __device__ u32 read(u32 n) {
-        if (n == 0) return 0;
-        if (pos + n > size) { ok = false; pos = size; return 0; }
-        const u64 wi = pos >> 5;
-        const u32 b = u32(pos & 31u);
-        const u64 window = (u64(wi < nWords ? w[wi] : 0u) << 32) | (wi + 1 < nWords ? w[wi + 1] : 0u);
-        pos += n;
-        return u32((window << b) >> (64 - n));
+    const u32* aligned;   // the 16-byte aligned word at or below the stream's first
+    u32 skew;             // words from it to the stream's first
+    u32 end;              // one past the stream's last word, from `aligned`
+    u64 size;             // readable bits
+    u32* win;             // kWalkWindow words of shared memory
+    u32 base;             // first word in it, from `aligned` (a multiple of 4)
+
+    __device__ u32 word(u32 i) {
+        const u32 a = i + skew;
+        if (a >= end || a < skew) return 0u;
+        if (a - base >= kWalkWindow) {   // also when the window lies behind (unsigned)
+            base = a & ~3u;
+            const u32 q = base + 4u * (threadIdx.x & 31u);   // this lane's four words, where they belong to the stream
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (q >= skew && q + 4 <= end) {
+                v = *reinterpret_cast<const uint4*>(aligned + q);
+            } else {
+                if (q >= skew && q < end) v.x = aligned[q];
+                if (q + 1 >= skew && q + 1 < end) v.y = aligned[q + 1];
+                if (q + 2 >= skew && q + 2 < end) v.z = aligned[q + 2];
+                if (q + 3 >= skew && q + 3 < end) v.w = aligned[q + 3];
+            }
+            __syncwarp();
+            *reinterpret_cast<uint4*>(win + 4u * (threadIdx.x & 31u)) = v;
+            __syncwarp();
+        }
+        return win[a - base];
     }
-    __device__ void align() {
-        const u64 a = (pos + 31) / 32 * 32;
-        pos = a < size ? a : size;
+    // n <= 32 bits at bit `bit` after word w; false past the end
+    __device__ bool bits(u32 w, u32 bit, u32 n, u32& v) {
+        if (u64(w) * 32u + bit + n > size) return false;
+        w += bit >> 5;
+        bit &= 31u;
+        const u32 hi = word(w), lo = bit + n > 32u ? word(w + 1) : 0u;
+        v = __funnelshift_l(lo, hi, bit) >> (32u - n);
+        return true;
     }
-    __device__ void skip(u64 n) { pos = pos + n < size ? pos + n : size; }
 };
 
-__device__ bool walkTableDev(DevReader& r, u32 log2Max, u32 leavesMax, DecTableDesc& d) {
-    d.hdrBit = r.pos;
-    d.nLen = r.read(5);
-    r.skip(u64(d.nLen) * log2Max);
-    d.nSym = r.read(log2Max);
+// Walks a table and its payload from bit `bit` of word w; w moves behind them.
+__device__ bool walkTableDev(DevReader& r, u32& w, u32 bit, u32 count, u32 log2Max, u32 leavesMax, u32 cbLog,
+                             DecTableDesc& d) {
+    d.hdrBit = u64(w) * 32u + bit;
+    if (!r.bits(w, bit, 5, d.nLen)) return false;
+    bit += 5 + d.nLen * log2Max;
+    if (!r.bits(w, bit, log2Max, d.nSym)) return false;
+    bit += log2Max;
     const bool longSym = log2Max > 16;
-    d.symbolBits = r.read(longSym ? 5 : 4);
+    if (!r.bits(w, bit, longSym ? 5 : 4, d.symbolBits)) return false;
+    bit += longSym ? 5 : 4;
     if (!longSym && d.symbolBits == 0 && d.nSym > 1) d.symbolBits = 16;   // HuffmanTable.cu:138-139
-    r.skip(u64(d.nSym) * d.symbolBits);
-    return r.ok && d.nSym <= leavesMax && d.nLen <= 31;
-}
-
-__device__ bool walkPayloadDev(DevReader& r, u32 count, u32 cb, DecTableDesc& d) {
-    r.align();
-    d.cwBits = r.read(32);
-    d.cwWord = r.pos / 32;
-    r.skip(ceilDiv(d.cwBits, 32) * 32);
-    r.align();
-    d.offWord = r.pos / 32;
-    r.skip(ceilDiv(count, cb) * 16);
-    r.align();
+    if (d.nSym > leavesMax || d.nLen > 31) return false;
+    const u64 symEnd = bit + u64(d.nSym) * d.symbolBits;
+    w += u32((symEnd + 31) >> 5);
+    if (!r.bits(w, 0, 32, d.cwBits)) return false;
+    ++w;
+    d.cwWord = w;
+    w += (d.cwBits >> 5) + ((d.cwBits & 31u) ? 1u : 0u);
+    d.offWord = w;
+    w += (blocksOf(count, cbLog) + 1u) / 2u;
     d.count = count;
-    return r.ok;
+    return true;
 }
 
-__global__ void __launch_bounds__(64) k_decWalk(DecParams p) {
-    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+// The walked fields of a table's descriptor (by one lane; blockOff and stream
+// are the plan's).
+__device__ __forceinline__ void storeWalked(DecTableDesc& to, const DecTableDesc& d) {
+    to.hdrBit = d.hdrBit;
+    to.cwWord = d.cwWord;
+    to.offWord = d.offWord;
+    to.cwBits = d.cwBits;
+    to.count = d.count;
+    to.symbolBits = d.symbolBits;
+    to.nLen = d.nLen;
+    to.nSym = d.nSym;
+}
+
+// A warp per source.
+constexpr u32 kWalkWarps = 2;
+
+__global__ void __launch_bounds__(kWalkWarps * 32) k_decWalk(DecParams p) {
+    __shared__ __align__(16) u32 sWin[kWalkWarps][kWalkWindow];
+    const u32 i = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
     if (i >= p.nSrc) return;
-    DecSource& src = p.sources[i];
+    const bool first = (threadIdx.x & 31u) == 0;
+    DecSource src = p.sources[i];
     if (p.wordOff) {
         const u64 bits = p.bitSize[i];
         src.words = p.wordsBase + p.wordOff[i];
@@ -143,25 +191,49 @@ __global__ void __launch_bounds__(64) k_decWalk(DecParams p) {
         src.wordCount = ceilDiv(bits, 32);
     }
     const u64 wordBits = src.wordCount * 32ull;
-    DevReader r{src.words, src.wordCount, src.bitSize < wordBits ? src.bitSize : wordBits, src.startBit, true};
-    bool ok = true;
+    const u32 skew = u32(reinterpret_cast<uintptr_t>(src.words) & 15u) / 4u;
+    DevReader r{src.words - skew, skew, u32(src.wordCount) + skew, src.bitSize < wordBits ? src.bitSize : wordBits,
+                sWin[threadIdx.x >> 5], 0u - kWalkWindow};
+    bool ok = src.wordCount < 0xFFFFFF00ull;
+    u32 w = u32(src.startBit >> 5), bit = u32(src.startBit & 31u);
+    u32 ns = 0, kinds = 0, firsts = 0;   // of this lane's stream of 32
     for (u32 k = 0; k < src.streamCount && ok; ++k) {
-        const u32 s = src.firstStream + k;
-        DecStreamDesc& sd = p.streams[s];
-        DecTableDesc& t0 = p.tables[sd.tableFirst];
-        if (sd.kind == KIND_RLHUFF) {
-            r.align();
-            const u32 m = r.read(32);
-            ok = r.ok && m <= sd.n;
-            sd.m = ok ? m : 0u;
-            DecTableDesc& t1 = p.tables[sd.tableFirst + 1];
-            ok = ok && walkTableDev(r, p.log2Max, p.leavesMax, t0) && walkPayloadDev(r, m, p.cb, t0);
-            ok = ok && walkTableDev(r, p.log2Max, p.leavesMax, t1) && walkPayloadDev(r, m, p.cb, t1);
+        if ((k & 31u) == 0) {
+            const u32 q = k + (threadIdx.x & 31u);
+            if (q < src.streamCount) {
+                const DecStreamDesc& mine = p.streams[src.firstStream + q];
+                ns = mine.n;
+                kinds = mine.kind;
+                firsts = mine.tableFirst;
+            }
+        }
+        DecStreamDesc& sd = p.streams[src.firstStream + k];
+        const u32 n = __shfl_sync(0xffffffffu, ns, int(k & 31u)), t0 = __shfl_sync(0xffffffffu, firsts, int(k & 31u));
+        const u32 kind = __shfl_sync(0xffffffffu, kinds, int(k & 31u));
+        DecTableDesc d0{}, d1{};
+        if (kind == KIND_RLHUFF) {
+            w += bit ? 1u : 0u;   // word aligned
+            bit = 0;
+            u32 m = 0;
+            ok = r.bits(w, 0, 32, m) && m <= n;
+            ++w;
+            if (first) sd.m = ok ? m : 0u;
+            ok = ok && walkTableDev(r, w, 0, m, p.log2Max, p.leavesMax, p.cbLog, d0) &&
+                 walkTableDev(r, w, 0, m, p.log2Max, p.leavesMax, p.cbLog, d1);
+            if (first) {
+                storeWalked(p.tables[t0], d0);
+                storeWalked(p.tables[t0 + 1], d1);
+            }
         } else {
-            sd.m = sd.n;
-            ok = walkTableDev(r, p.log2Max, p.leavesMax, t0) && walkPayloadDev(r, sd.n, p.cb, t0);
+            ok = walkTableDev(r, w, bit, n, p.log2Max, p.leavesMax, p.cbLog, d0);
+            bit = 0;
+            if (first) {
+                sd.m = n;
+                storeWalked(p.tables[t0], d0);
+            }
         }
     }
+    if (!first) return;
     if (!ok) {
         atomicOr(p.errors, DEV_ERR_CORRUPT);
         // nothing of this source is decoded
@@ -169,28 +241,20 @@ __global__ void __launch_bounds__(64) k_decWalk(DecParams p) {
             DecStreamDesc& sd = p.streams[src.firstStream + k];
             sd.m = 0;
             const u32 parts = sd.kind == KIND_RLHUFF ? 2u : 1u;
-            for (u32 w = 0; w < parts; ++w) {
-                DecTableDesc& t = p.tables[sd.tableFirst + w];
-                t.count = 0;
-                t.nSym = 0;
-                t.nLen = 0;
-                t.hdrBit = t.cwWord = t.offWord = 0;
-                t.cwBits = 0;
-                t.symbolBits = 0;
-            }
+            for (u32 w = 0; w < parts; ++w) storeWalked(p.tables[sd.tableFirst + w], DecTableDesc{});
         }
     }
-    src.endBit = r.pos;
+    src.endBit = min(u64(w) * 32u + bit, r.size);
+    p.sources[i] = src;
 }
 
 // Symbol array offsets of the tables (prefix of nSym) and capacity check.
 // CTA b takes the kPlanChunk tables of chunk b (four consecutive per thread):
 // offsets within the chunk and the chunk's sum (planPart); with more than one
 // chunk, k_decSymPlanCarry adds the chunks before each one.
-__global__ void __launch_bounds__(1024) k_decSymPlan(DecParams p) {
+__device__ __forceinline__ void symPlanChunk(const DecParams& p, u32 b, u32 chunks, u32* scratch) {
     constexpr u32 kPer = kPlanChunk / 1024;
-    __shared__ u32 scratch[40];
-    const u32 t0 = blockIdx.x * kPlanChunk + threadIdx.x * kPer;
+    const u32 t0 = b * kPlanChunk + threadIdx.x * kPer;
     u32 v[kPer], sum = 0;
 #pragma unroll
     for (u32 j = 0; j < kPer; ++j) {
@@ -205,12 +269,17 @@ __global__ void __launch_bounds__(1024) k_decSymPlan(DecParams p) {
         at += v[j];
     }
     if (threadIdx.x == 0) {
-        if (gridDim.x == 1) {
+        if (chunks == 1) {
             if (tot > p.capLeaves) atomicOr(p.errors, DEV_ERR_TABLE_CAPACITY);
         } else {
-            p.planPart[blockIdx.x] = tot;
+            p.planPart[b] = tot;
         }
     }
+}
+
+__global__ void __launch_bounds__(1024) k_decSymPlan(DecParams p) {
+    __shared__ u32 scratch[40];
+    symPlanChunk(p, blockIdx.x, gridDim.x, scratch);
 }
 
 // Chunk b = blockIdx.x + 1 of a symbol plan of more than one chunk: the sum
@@ -240,10 +309,14 @@ __global__ void __launch_bounds__(1024) k_decSymPlanCarry(DecParams p) {
 // ---------------------------------------------------------------------------
 // Table parse and decode structures (HuffmanTable.cu:117-151, :205-266).
 // ---------------------------------------------------------------------------
-// One 64-thread CTA per table (up to 32 tables per SM: the work per table is
-// a short chain of dependent steps).
-constexpr u32 kDecThreads = 64;
+// One CTA per table: 64 threads in calls of many tables (up to 32 tables per
+// SM: the work per table is a short chain of dependent steps), 512 in calls of
+// few, where the offsets of a long stream's blocks - 8 per thread and step -
+// and the lookup table take the time (129 tables of 256^3 streams: 35 -> 18 us).
+constexpr u32 kDecThreads = 64, kDecThreadsWide = 512;
+constexpr u32 kDecWideTables = 4 * 148;   // tables of a call that the wide CTAs hold at once
 
+template <u32 kDecThreads>
 __global__ void __launch_bounds__(kDecThreads) k_decTables(DecParams p) {
     __shared__ u32 cpl[32];
     __shared__ int sFirst[32], sMin[32], sMax[32];
@@ -338,7 +411,7 @@ __global__ void __launch_bounds__(kDecThreads) k_decTables(DecParams p) {
     }
     // absolute block offsets: inclusive prefix of the u16 increments
     // (PackInc.cu:220-229), eight blocks (four words) per thread per step
-    const u32 blocks = u32(ceilDiv(d.count, p.cb));
+    const u32 blocks = blocksOf(d.count, p.cbLog);
     u32* bo = p.blockOff + d.blockOff;
     __syncthreads();
     for (u32 base = 0; base < blocks; base += 8 * kDecThreads) {
@@ -368,143 +441,165 @@ __global__ void __launch_bounds__(kDecThreads) k_decTables(DecParams p) {
     }
 }
 
-// Decodes up to `cnt` symbols of one coding block starting at absolute bit
-// `bit`, calling emit(i, symbol).  kValueLut: lookup entries hold symbol
-// values (16-bit symbols), else symbol indices.  The 64-bit window is two
-// words, read with a funnel shift.
-template <bool kValueLut, class Src, class Emit>
-__device__ __forceinline__ void decodeBlock(const Src& ws, const DecTable& D, const u32* syms, const u32* lut,
-                                            u64 bit, u32 cnt, bool& corrupt, Emit emit) {
-    const u32 nSym = D.nSym;
-    if (nSym == 0xFFFFFFFFu) { corrupt = true; return; }
-    if (nSym <= 1) {
-        const u32 single = D.single;
-        for (u32 i = 0; i < cnt; ++i) emit(i, single);
-        return;
-    }
-    u64 w = bit >> 5;
-    u32 bpos = u32(bit & 31u);
-    u32 hi = ws.at(w), lo = ws.at(w + 1);
-    w += 2;
-    for (u32 i = 0; i < cnt; ++i) {
-        const u32 v = __funnelshift_l(lo, hi, bpos);
-        const u32 e = lut[v >> (32 - kLutBits)];
-        u32 len, val;
-        if (e) {
-            len = e >> 24;
-            val = e & 0xFFFFFFu;
-            if (!kValueLut) {
-                if (val >= nSym) { corrupt = true; return; }
-                val = syms[val];
-            }
-        } else {
-            len = kLutBits + 1;
-            while (len <= 31 && int(v >> (32 - len)) > D.maxCode[len - 1]) ++len;
-            if (len > 31) { corrupt = true; return; }
-            const u32 idx = u32(D.firstIndex[len - 1] + int(v >> (32 - len)) - D.minCode[len - 1]);
-            if (idx >= nSym) { corrupt = true; return; }
-            val = syms[idx];
-        }
-        emit(i, val);
-        bpos += len;
-        if (bpos >= 32) {
-            hi = lo;
-            lo = ws.at(w);
-            ++w;
-            bpos -= 32;
-        }
-    }
-}
-
-// One table's decode data in shared memory: the lookup table, and for codes
-// longer than it the left-justified limits - lim[l] = (maxCode[l] + 1) <<
-// (32 - l), carried over lengths without codes, so a 32-bit window v holds a
-// code longer than l iff v >= lim[l] (the canonical codes of one length are
-// consecutive and each length starts where the shorter ones end, so lim never
-// decreases) - and the first index / first code of each length.
+// One table's data for codes longer than the lookup table, in shared memory:
+// last[l] = (maxCode[l] + 1 << (32 - l)) - 1, carried over lengths without
+// codes, so a 32-bit window v holds a code longer than l iff v > last[l] (the
+// canonical codes of one length are consecutive and each length starts where
+// the shorter ones end, so last never decreases), for l from the shortest
+// code's length on; off[l - 1]: first index - first code.
 struct CanonSmem {
-    u32 lut[1u << kLutBits];
-    unsigned long long lim[36];   // lengths 1..31; 32..35 above every window
-    int first[32], minc[32];
+    u32 last[32];
+    int off[32];
+};
+// The same for the lengths met in earnest, in registers: codes of more than
+// kLutBits bits are `start` bits long or more; lengths kLutBits + 1 .. + 4 as
+// in last[] (never exceeded below the shortest code, which start leaves out).
+struct LongCodes {
+    u32 start, l0, l1, l2, l3;
 };
 
-// Stages table t into cs (all 32 lanes of the calling warp).
-__device__ __forceinline__ void stageCanon(CanonSmem& cs, const DecParams& p, u32 t) {
+// Stages table t's long codes into cs (all 32 lanes of the calling warp; the
+// caller synchronizes).
+__device__ __forceinline__ LongCodes stageLongCodes(CanonSmem& cs, const DecParams& p, u32 t) {
     const u32 lane = threadIdx.x & 31u;
-    const u32* g = p.lut + (u64(t) << kLutBits);
-    for (u32 e = lane; e < (1u << kLutBits); e += 32) cs.lut[e] = g[e];
     const DecTable& D = p.dec[t];
     const int mc = D.maxCode[lane];
-    const u32 l = lane + 1;
-    unsigned long long lim = l <= 31 && mc >= 0 ? (unsigned long long)(u32(mc) + 1u) << (32 - l) : 0ull;
+    cs.off[lane] = D.firstIndex[lane] - D.minCode[lane];
+    // lane l holds length l + 1
+    const u32 has = __ballot_sync(0xffffffffu, mc >= 0 && lane < 31u);
+    const u32 upTo = has & (0xFFFFFFFFu >> (31u - lane));
+    const u32 from = upTo ? 31u - u32(__clz(int(upTo))) : 0u;   // nearest length with codes
+    u32 last = mc >= 0 && lane < 31u ? ((u32(mc) + 1u) << (31u - lane)) - 1u : 0xFFFFFFFFu;
+    last = __shfl_sync(0xffffffffu, last, int(from));
+    if (!upTo) last = 0xFFFFFFFFu;
+    cs.last[lane] = last;
+    LongCodes lc;
+    const u32 shortest = has ? u32(__ffs(int(has))) : 32u;      // length of the shortest code
+    lc.start = max(kLutBits + 1u, shortest);
+    lc.l0 = __shfl_sync(0xffffffffu, last, int(kLutBits));
+    lc.l1 = __shfl_sync(0xffffffffu, last, int(kLutBits + 1));
+    lc.l2 = __shfl_sync(0xffffffffu, last, int(kLutBits + 2));
+    lc.l3 = __shfl_sync(0xffffffffu, last, int(kLutBits + 3));
+    return lc;
+}
+// Stages table t's lookup table, one of `threads` threads calling (the caller
+// synchronizes).
+__device__ __forceinline__ void stageLut(u32* lut, const DecParams& p, u32 t, u32 thread, u32 threads) {
+    const uint4* g = reinterpret_cast<const uint4*>(p.lut + (u64(t) << kLutBits));
+    for (u32 k = thread; k < (1u << kLutBits) / 4u; k += threads) reinterpret_cast<uint4*>(lut)[k] = g[k];
+}
+
+// Length and symbol index of a window holding a code longer than the lookup
+// table; false past the longest.
+__device__ __forceinline__ bool longCode(u32 v, const LongCodes& lc, const CanonSmem& cs, u32 nSym, u32& len,
+                                         u32& idx) {
+    len = lc.start + (v > lc.l0 ? 1u : 0u) + (v > lc.l1 ? 1u : 0u) + (v > lc.l2 ? 1u : 0u) + (v > lc.l3 ? 1u : 0u);
+    if (len > kLutBits + 4u)
+        while (len <= 31u && v > cs.last[len - 1]) ++len;
+    if (len > 31u) return false;
+    idx = (v >> (32u - len)) + u32(cs.off[len - 1]);
+    return idx < nSym;
+}
+
+// The code words of a warp's coding blocks, which are consecutive: staged in
+// shared memory by coalesced loads when they fit, else read where they are.  A
+// lane that fetches its words from global memory as it goes waits for a cache
+// miss, or for 31 other lanes' lines, about every other symbol.
+struct StagedWords {   // s[n] = 0
+    const u32* s;
+    u32 n;
+    __device__ __forceinline__ u32 at(u32 i) const { return s[min(i, n)]; }
+};
+struct SourceWords {
+    WordSrc ws;
+    u64 first;
+    __device__ __forceinline__ u32 at(u32 i) const { return ws.at(first + i); }
+};
+
+// Copies words [first, first + n) of ws to stage (all lanes of the warp).
+__device__ __forceinline__ void stageWords(u32* stage, const WordSrc& ws, u64 first, u32 n) {
+    for (u32 base = 0; base < n; base += 256) {
+        u32 v[8];
 #pragma unroll
-    for (u32 d = 1; d < 32; d <<= 1) {
-        const unsigned long long o = __shfl_up_sync(0xffffffffu, lim, d);
-        if (lane >= d) lim = o > lim ? o : lim;   // running maximum
-    }
-    cs.lim[l] = l <= 31 ? lim : ~0ull;
-    if (lane < 4) cs.lim[32 + lane] = ~0ull;
-    if (lane == 0) cs.lim[0] = 0;
-    cs.first[lane] = D.firstIndex[lane];
-    cs.minc[lane] = D.minCode[lane];
-    __syncwarp();
-}
-
-// decodeBlock with the table in shared memory: the length of a code longer
-// than the lookup table is found four lengths per step.
-template <bool kValueLut, class Emit>
-__device__ __forceinline__ void decodeBlockStaged(const WordSrc& ws, const DecTable& D, const CanonSmem& cs,
-                                                  const u32* syms, u64 bit, u32 cnt, bool& corrupt, Emit emit) {
-    const u32 nSym = D.nSym;
-    if (nSym == 0xFFFFFFFFu) { corrupt = true; return; }
-    if (nSym <= 1) {
-        const u32 single = D.single;
-        for (u32 i = 0; i < cnt; ++i) emit(i, single);
-        return;
-    }
-    u64 w = bit >> 5;
-    u32 bpos = u32(bit & 31u);
-    u32 hi = ws.at(w), lo = ws.at(w + 1);
-    w += 2;
-    for (u32 i = 0; i < cnt; ++i) {
-        const u32 v = __funnelshift_l(lo, hi, bpos);
-        const u32 e = cs.lut[v >> (32 - kLutBits)];
-        u32 len, val;
-        if (e) {
-            len = e >> 24;
-            val = e & 0xFFFFFFu;
-            if (!kValueLut) {
-                if (val >= nSym) { corrupt = true; return; }
-                val = syms[val];
-            }
-        } else {
-            const unsigned long long vv = v;
-            len = kLutBits + 1;
-            for (;;) {
-                const u32 c = (vv >= cs.lim[len] ? 1u : 0u) + (vv >= cs.lim[len + 1] ? 1u : 0u) +
-                              (vv >= cs.lim[len + 2] ? 1u : 0u) + (vv >= cs.lim[len + 3] ? 1u : 0u);
-                len += c;
-                if (c < 4 || len > 31) break;
-            }
-            if (len > 31) { corrupt = true; return; }
-            const u32 idx = u32(cs.first[len - 1] + int(v >> (32 - len)) - cs.minc[len - 1]);
-            if (idx >= nSym) { corrupt = true; return; }
-            val = syms[idx];
+        for (u32 k = 0; k < 8; ++k) {
+            const u32 i = base + 32 * k + (threadIdx.x & 31u);
+            v[k] = i < n ? ws.at(first + i) : 0u;
         }
-        emit(i, val);
-        bpos += len;
-        if (bpos >= 32) {
-            hi = lo;
-            lo = ws.at(w);
-            ++w;
-            bpos -= 32;
+#pragma unroll
+        for (u32 k = 0; k < 8; ++k) {
+            const u32 i = base + 32 * k + (threadIdx.x & 31u);
+            if (i < n) stage[i] = v[k];
         }
     }
+    if ((threadIdx.x & 31u) == 0) stage[n] = 0;
 }
 
-// decodeHuff: one thread per coding block; when a warp's 32 blocks belong to
-// one stream its table is staged in shared memory and its output staged
-// there too and written coalesced.
+// A lane's place in its words: two words in hand and the next on its way, so
+// that a step waits for the lookup only.
+struct BitReader {
+    u32 w;          // index of the word after nx
+    u32 bpos;       // bit position in hi
+    u32 hi, lo, nx;
+    template <class Words>
+    __device__ __forceinline__ void start(const Words& ws, u32 bit) {
+        w = bit >> 5;
+        bpos = bit & 31u;
+        hi = ws.at(w);
+        lo = ws.at(w + 1);
+        nx = ws.at(w + 2);
+        w += 3;
+    }
+};
+
+// One symbol from r: a lookup, or for a code longer than the lookup table its
+// length from the limits.  A window that holds no code sets corrupt and moves
+// on by a bit.  kValueLut: lookup entries hold symbol values (16-bit symbols),
+// else symbol indices.
+template <bool kValueLut, class Words>
+__device__ __forceinline__ u32 decodeOne(const Words& ws, const u32* lut, const CanonSmem& cs, const LongCodes& lc,
+                                         u32 nSym, const u32* syms, BitReader& r, bool& corrupt) {
+    const u32 v = __funnelshift_l(r.lo, r.hi, r.bpos);
+    const u32 e = lut[v >> (32 - kLutBits)];
+    u32 len = e >> 24, val = e & 0xFFFFFFu;
+    if (kValueLut) {
+        if (!e) {
+            u32 idx;
+            if (longCode(v, lc, cs, nSym, len, idx)) val = syms[idx];
+            else { corrupt = true; len = 1; }
+        }
+    } else {
+        bool ok = val < nSym;
+        if (!e) ok = longCode(v, lc, cs, nSym, len, val);
+        if (ok) val = syms[val];
+        else { corrupt = true; len = 1; }
+    }
+    r.bpos += len;
+    const bool next = r.bpos >= 32u;
+    r.hi = next ? r.lo : r.hi;
+    r.lo = next ? r.nx : r.lo;
+    if (next) r.nx = ws.at(r.w);
+    r.w += next ? 1u : 0u;
+    r.bpos &= 31u;
+    return val;
+}
+
+// decodeHuff: one thread per coding block, a warp per 32 blocks of a stream
+// (the plan numbers the streams' blocks from multiples of 32), its table and
+// code words staged in shared memory (huffStageWords at most), its output too,
+// and written coalesced.  The
+// lane's serial chain per block bounds it: a lookup and a few selects per
+// symbol, and for codes longer than the lookup table - half of a lowpass
+// band's - the register limits, an offset and the symbol from L1.  24 warps of
+// 256^3 lowpass streams: 79 us with words read from global memory, 47 with
+// words staged, 39 with the limits in registers; six warps of 4675-symbol
+// streams 93 -> 32, most of whose warps held blocks of two streams before.
+CC_HD u32 huffStageWords(u32 cb) { return 12u * cb; }   // 12 bits per symbol
+CC_HD u32 huffPitch(u32 cb, u32 symBytes) { return cb + (symBytes == 2 ? 2 : 1); }
+template <class Sym>
+CC_HD size_t huffSmem(u32 cb) {
+    return 4 * size_t((1u << kLutBits) + huffStageWords(cb) + 4) + size_t(32) * huffPitch(cb, sizeof(Sym)) * sizeof(Sym);
+}
+
 template <class Sym>
 __global__ void __launch_bounds__(32) k_decHuff(DecParams p) {
     extern __shared__ __align__(16) unsigned char stage[];
@@ -512,51 +607,72 @@ __global__ void __launch_bounds__(32) k_decHuff(DecParams p) {
     if (__any_sync(0xffffffffu, capacityFailed(p))) return;
     const u32 lane = threadIdx.x;
     const u32 b0 = blockIdx.x * 32;
-    const u32 gb = b0 + lane;
-    const bool valid = gb < p.hBlocks;
-    const u32 s = streamOfBlock(p, p.hList, p.nH, valid ? gb : p.hBlocks - 1);
-    const u32 s0 = __shfl_sync(0xffffffffu, s, 0);
-    const bool uniform = __all_sync(0xffffffffu, !valid || s == s0);
+    const u32 s = streamOfBlock(p, p.hList, p.nH, b0);
     const DecStreamDesc sd = p.streams[s];
-    const u32 b = gb - sd.blockFirst;
-    const u32 blocks = u32(ceilDiv(sd.n, p.cb));
-    const u32 rowPitch = p.cb + (sizeof(Sym) == 2 ? 2 : 1);
-    Sym* rows = reinterpret_cast<Sym*>(stage);
-    Sym* out = reinterpret_cast<Sym*>(sd.out);
-    bool corrupt = false;
-    const bool mine = valid && b < blocks;
-    const u32 i0 = b * p.cb;
-    if (uniform) stageCanon(cs, p, p.streams[s0].tableFirst);   // the warp's one table
-    if (mine) {
-        const u32 t = sd.tableFirst;
-        const DecTableDesc& td = p.tables[t];
-        const WordSrc ws = srcOf(p, s);
-        const u32 cnt = min(p.cb, sd.n - i0);
-        const u64 bit = td.cwWord * 32ull + p.blockOff[td.blockOff + b];
-        if (uniform)
-            decodeBlockStaged<sizeof(Sym) == 2>(ws, p.dec[t], cs, p.syms + td.symOff, bit, cnt, corrupt,
-                        [&](u32 i, u32 v) { rows[lane * rowPitch + i] = Sym(v); });
-        else
-            decodeBlock<sizeof(Sym) == 2>(ws, p.dec[t], p.syms + td.symOff, p.lut + (u64(t) << kLutBits), bit, cnt, corrupt,
-                        [&](u32 i, u32 v) { out[i0 + i] = Sym(v); });
-    }
-    if (corrupt) atomicOr(p.errors, DEV_ERR_CORRUPT);
-    if (!uniform) return;
-    __syncwarp();
-    // every lane's sd is the stream of block b0 here
     const u32 bFirst = b0 - sd.blockFirst;
+    const u32 blocks = blocksOf(sd.n, p.cbLog);
     if (bFirst >= blocks) return;
     const u32 nb = min(32u, blocks - bFirst);
+    const u32 b = bFirst + lane;
+    const u32 rowPitch = huffPitch(p.cb, sizeof(Sym));
+    u32* lut = reinterpret_cast<u32*>(stage);
+    u32* words = lut + (1u << kLutBits);
+    Sym* rows = reinterpret_cast<Sym*>(words + huffStageWords(p.cb) + 4);
+    Sym* out = reinterpret_cast<Sym*>(sd.out);
+    bool corrupt = false;
+    const bool mine = lane < nb;
+    const u32 t = sd.tableFirst;
+    const DecTableDesc td = p.tables[t];
+    const u32* syms = p.syms + td.symOff;
+    const u32 cnt = mine ? min(p.cb, sd.n - b * p.cb) : 0u;
+    const u32 blockBit = mine ? p.blockOff[td.blockOff + b] : 0u;
+    const WordSrc ws = srcOf(p, s);
+    // the warp's words: from its first block's to the next warp's first, or the stream's end
+    const u32 bit0 = __shfl_sync(0xffffffffu, blockBit, 0);
+    const u32 bit1 = bFirst + 32 < blocks ? p.blockOff[td.blockOff + bFirst + 32] : td.cwBits;
+    const u32 w0 = bit0 >> 5;
+    const u32 nw = bit1 > bit0 ? (bit1 - 1) / 32 - w0 + 1 : 0u;
+    const bool staged = nw <= huffStageWords(p.cb);   // warp-uniform
+    const DecTable& D = p.dec[t];
+    const u32 nSym = D.nSym;
+    if (staged) stageWords(words, ws, td.cwWord + w0, nw);
+    stageLut(lut, p, t, lane, 32);
+    const LongCodes lc = stageLongCodes(cs, p, t);
+    __syncwarp();
+    if (mine) {
+        Sym* row = rows + lane * rowPitch;
+        if (nSym == 0xFFFFFFFFu) {
+            corrupt = true;
+        } else if (nSym <= 1) {
+            const u32 single = D.single;
+            for (u32 i = 0; i < cnt; ++i) row[i] = Sym(single);
+        } else {
+            BitReader rd;
+            if (staged) {
+                const StagedWords sw{words, nw};
+                rd.start(sw, blockBit - 32u * w0);
+                for (u32 i = 0; i < cnt; ++i)
+                    row[i] = Sym(decodeOne<sizeof(Sym) == 2>(sw, lut, cs, lc, nSym, syms, rd, corrupt));
+            } else {
+                const SourceWords gw{ws, td.cwWord + w0};
+                rd.start(gw, blockBit - 32u * w0);
+                for (u32 i = 0; i < cnt; ++i)
+                    row[i] = Sym(decodeOne<sizeof(Sym) == 2>(gw, lut, cs, lc, nSym, syms, rd, corrupt));
+            }
+        }
+    }
+    if (corrupt) atomicOr(p.errors, DEV_ERR_CORRUPT);
+    __syncwarp();
     const u64 base = u64(bFirst) * p.cb;
     const u64 lim = u64(sd.n) - base;
     const u64 total = u64(nb) * p.cb < lim ? u64(nb) * p.cb : lim;
-    for (u64 k = lane; k < total; k += 32) out[base + k] = rows[(k / p.cb) * rowPitch + (k % p.cb)];
+    for (u32 k = lane; k < u32(total); k += 32) out[base + k] = rows[(k >> p.cbLog) * rowPitch + (k & (p.cb - 1u))];
 }
 
 // Coding blocks of RLHuff stream s that a decode covers: its run-length
 // symbol count in blocks, within the blocks planned for its length.
 __device__ __forceinline__ u32 rlBlocksOf(const DecParams& p, const DecStreamDesc& sd) {
-    return u32(min(ceilDiv(u64(sd.m), p.cb), ceilDiv(u64(sd.n), p.cb)));
+    return blocksOf(min(sd.m, sd.n), p.cbLog);
 }
 
 // Warp tasks of the run-length decode, once the headers are walked: every
@@ -569,7 +685,7 @@ __device__ __forceinline__ u32 rlTaskWarps(const DecParams& p, u32 k, u32& s) {
     s = 0;
     if (k >= p.nRl) return 0;
     s = p.rlList[k];
-    return u32(ceilDiv(rlBlocksOf(p, p.streams[s]), 32));
+    return (rlBlocksOf(p, p.streams[s]) + 31u) / 32u;
 }
 
 __global__ void __launch_bounds__(1024) k_decRlTaskCounts(DecParams p) {
@@ -580,11 +696,9 @@ __global__ void __launch_bounds__(1024) k_decRlTaskCounts(DecParams p) {
     if (threadIdx.x == 0) p.planPart[blockIdx.x] = tot;
 }
 
-__global__ void __launch_bounds__(1024) k_decRlTasks(DecParams p) {
-    __shared__ u32 scratch[40];
+__device__ __forceinline__ void rlTasksChunk(const DecParams& p, u32 b, u32 chunks, u32* scratch) {
     __shared__ u32 sOff[1024], sStr[1024];   // the chunk's streams: first task, stream index
     __shared__ u32 sCarry;
-    const u32 b = blockIdx.x;
     if (threadIdx.x < 32) {
         // tasks of the chunks before this one
         u32 c = 0;
@@ -614,8 +728,20 @@ __global__ void __launch_bounds__(1024) k_decRlTasks(DecParams p) {
         const u32 at = carry + i;
         if (at < p.rlTaskCap) p.rlTasks[at] = (u64(sStr[lo]) << 32) | (32u * (i - sOff[lo]));
     }
-    if (b + 1 == gridDim.x && threadIdx.x == 0)
+    if (b + 1 == chunks && threadIdx.x == 0)
         reinterpret_cast<u32*>(p.rlTasks + p.rlTaskCap)[0] = min(carry + tot, p.rlTaskCap);
+}
+
+__global__ void __launch_bounds__(1024) k_decRlTasks(DecParams p) {
+    __shared__ u32 scratch[40];
+    rlTasksChunk(p, blockIdx.x, gridDim.x, scratch);
+}
+
+// Both plans of a call of one chunk each: CTA 0 the symbols', CTA 1 the tasks.
+__global__ void __launch_bounds__(1024) k_decPlans(DecParams p) {
+    __shared__ u32 scratch[40];
+    if (blockIdx.x == 0) symPlanChunk(p, 0, 1, scratch);
+    else rlTasksChunk(p, 0, 1, scratch);
 }
 
 // The RLHuff streams' outputs, zeroed before the symbol pass writes the
@@ -642,173 +768,250 @@ __global__ void __launch_bounds__(256) k_decZero(DecParams p) {
 }
 
 // decodeRLHuff (RunLengthKernels.cui:56-66 for the scatter): one lane per
-// coding block, 32 consecutive blocks of one stream per warp (k_decRlTasks).
+// coding block, 32 consecutive blocks of one stream per warp (k_decRlTasks),
+// the warp's code words and long codes staged in its shared memory; the lookup
+// table is the CTA's (kSharedLut: its first warp's, warps of another table
+// read theirs from global memory - calls of long streams) or each warp's.
 // Each lane decodes its block in rounds of kRlRound symbols into its row of
-// the warp's shared rows, its bit reader staying in registers between
-// rounds; after a round the warp moves the rows out block by block, lane k
-// taking the block's element k of the round.  Zero counts (kSymbols false)
-// are stored and their (zc + 1) summed per block.  Symbols are scattered to
-// out[block start + sum of (zc + 1) before the element + zc]: the round's
-// zero counts of the warp's blocks are staged with coalesced loads and a
-// warp scan gives the positions.  Lanes read their code words through L1;
-// the CTA stages the lookup table of its first warp's stream in shared
-// memory (a warp decoding another stream reads its table from global
-// memory).  About 13 KB of shared memory per CTA of four warps.
+// the warp's shared rows, its bit reader staying in registers between rounds;
+// after a round the warp moves the rows out block by block, lane k taking the
+// block's element k of the round.  Zero counts (kSymbols false) are stored, 16
+// bytes per lane, and their (zc + 1) summed per block.  Symbols are scattered
+// to out[block start + sum of (zc + 1) before the element + zc]: the round's
+// zero counts, fetched before its symbols are decoded, become positions in the
+// round by the lane of the block, four per step beside its 31 neighbours.
+// Rows are 36 elements: four 16-bit (8 bytes) per lane are free of conflicts.
+// Bound: instruction issue and shared memory (27 instructions per 32 zero
+// counts, 54 per 32 symbols, 64% and 49% of the issue slots), and the lane's
+// chain per symbol (lookup, length, next word) where a call has few blocks.
+// Three 256^3 streams (26 million entries): zero counts 61 -> 53, symbols 145
+// -> 126 us against words read from global memory, a scan over the warp per
+// block and round, and the limits searched in global memory; seven streams of
+// 100003 symbols 33 -> 26 and 73 -> 38.
 constexpr u32 kRlRound = 32;
+constexpr u32 kRlWarps = 4;
+constexpr u32 kRlPitch = 36;
+constexpr u32 kRlSharedTasks = 8;   // mean warp tasks per stream from which a CTA shares one lookup table
 
-struct BitReader {
-    u64 w;      // next word
-    u32 bpos;   // bit position in hi
-    u32 hi, lo;
-};
-
-// Decodes cnt symbols from r, calling emit(i, symbol) (decodeBlock's steps).
-template <bool kValueLut, class Lut, class Emit>
-__device__ __forceinline__ void decodeRun(const WordSrc& ws, const DecTable& D, u32 nSym, const u32* syms,
-                                          const Lut& lut, BitReader& r, u32 cnt, bool& corrupt, Emit emit) {
-    for (u32 i = 0; i < cnt; ++i) {
-        const u32 v = __funnelshift_l(r.lo, r.hi, r.bpos);
-        const u32 e = lut(v >> (32 - kLutBits));
-        u32 len, val;
-        if (e) {
-            len = e >> 24;
-            val = e & 0xFFFFFFu;
-            if (!kValueLut) {
-                if (val >= nSym) { corrupt = true; return; }
-                val = syms[val];
-            }
-        } else {
-            len = kLutBits + 1;
-            while (len <= 31 && int(v >> (32 - len)) > D.maxCode[len - 1]) ++len;
-            if (len > 31) { corrupt = true; return; }
-            const u32 idx = u32(D.firstIndex[len - 1] + int(v >> (32 - len)) - D.minCode[len - 1]);
-            if (idx >= nSym) { corrupt = true; return; }
-            val = syms[idx];
-        }
-        emit(i, val);
-        r.bpos += len;
-        if (r.bpos >= 32) {
-            r.hi = r.lo;
-            r.lo = ws.at(r.w);
-            ++r.w;
-            r.bpos -= 32;
-        }
-    }
+CC_HD u32 rlStageWords(u32 cb) { return 6u * cb; }   // 6 bits per symbol
+// Bytes of a warp's shared memory: long codes, rows, zero counts, words (and one behind them).
+template <class Sym, bool kSymbols>
+CC_HD size_t rlWarpSmem(u32 cb) {
+    return sizeof(CanonSmem) + (kSymbols ? 2 : 1) * 32 * kRlPitch * sizeof(Sym) + 4 * size_t(rlStageWords(cb) + 4);
+}
+template <class Sym, bool kSymbols, bool kSharedLut>
+CC_HD size_t rlSmem(u32 cb) {
+    return kRlWarps * rlWarpSmem<Sym, kSymbols>(cb) + (kSharedLut ? 1 : kRlWarps) * (4u << kLutBits);
 }
 
-template <class Sym, bool kSymbols>
-__global__ void __launch_bounds__(128) k_decRl(DecParams p) {
-    constexpr u32 kPitch = kRlRound + (sizeof(Sym) == 2 ? 2 : 1);
-    __shared__ Sym sRows[4][32 * kPitch];
-    __shared__ Sym sZc[kSymbols ? 4 : 1][32 * kRlRound];
-    __shared__ u32 sLut[1u << kLutBits];
-    __shared__ u32 sLutTable, sFail;
+// Four consecutive elements of a row.
+__device__ __forceinline__ void putFour(u16* row, u32 a, u32 b, u32 c, u32 d) {
+    *reinterpret_cast<uint2*>(row) = make_uint2((a & 0xFFFFu) | (b << 16), (c & 0xFFFFu) | (d << 16));
+}
+__device__ __forceinline__ void putFour(u32* row, u32 a, u32 b, u32 c, u32 d) {
+    *reinterpret_cast<uint4*>(row) = make_uint4(a, b, c, d);
+}
+__device__ __forceinline__ void getFour(const u16* row, u32 (&v)[4]) {
+    const uint2 x = *reinterpret_cast<const uint2*>(row);
+    v[0] = x.x & 0xFFFFu; v[1] = x.x >> 16; v[2] = x.y & 0xFFFFu; v[3] = x.y >> 16;
+}
+__device__ __forceinline__ void getFour(const u32* row, u32 (&v)[4]) {
+    const uint4 x = *reinterpret_cast<const uint4*>(row);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+// 16 bytes of a row, 8-byte aligned.
+__device__ __forceinline__ uint4 rowVec(const void* q) {
+    const uint2* h = reinterpret_cast<const uint2*>(q);
+    const uint2 a = h[0], b = h[1];
+    return make_uint4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void rowVec(void* q, uint4 v) {
+    uint2* h = reinterpret_cast<uint2*>(q);
+    h[0] = make_uint2(v.x, v.y);
+    h[1] = make_uint2(v.z, v.w);
+}
+
+template <class Sym, bool kSymbols, bool kSharedLut>
+__global__ void __launch_bounds__(kRlWarps * 32) k_decRl(DecParams p) {
+    constexpr u32 kVec = 16 / sizeof(Sym);        // elements of a 16-byte access
+    constexpr u32 kParts = kRlRound / kVec;       // accesses per block and round
+    constexpr u32 kWordsPer = 4 / sizeof(Sym);    // elements per 32-bit word
+    constexpr bool kValueLut = sizeof(Sym) == 2;
+    extern __shared__ __align__(16) unsigned char stage[];
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const u32 wt = blockIdx.x * 4u + warp;
-    const bool hasTask = wt < reinterpret_cast<const u32*>(p.rlTasks + p.rlTaskCap)[0];
-    u32 s = 0, bFirst = 0, t = 0;
-    if (hasTask) {
-        const u64 task = p.rlTasks[wt];
-        s = u32(task >> 32);
-        bFirst = u32(task);
-        t = p.streams[s].tableFirst + (kSymbols ? 0u : 1u);
+    const u32 tasks = reinterpret_cast<const u32*>(p.rlTasks + p.rlTaskCap)[0];
+    const u32 wt = blockIdx.x * kRlWarps + warp;
+    if (blockIdx.x * kRlWarps >= tasks) return;   // CTA-uniform
+    unsigned char* mem = stage + (kSharedLut ? 1 : kRlWarps) * (4u << kLutBits) + warp * rlWarpSmem<Sym, kSymbols>(p.cb);
+    CanonSmem& cs = *reinterpret_cast<CanonSmem*>(mem);
+    Sym* rows = reinterpret_cast<Sym*>(mem + sizeof(CanonSmem));
+    Sym* zs = rows + 32 * kRlPitch;
+    u32* words = reinterpret_cast<u32*>(rows + (kSymbols ? 2 : 1) * 32 * kRlPitch);
+    u32* lutS = reinterpret_cast<u32*>(stage) + (kSharedLut ? 0u : warp << kLutBits);
+    bool lutHere = true;   // warp-uniform: the warp's lookup table is in shared memory
+    if (kSharedLut) {
+        // the CTA's table: its first warp's
+        const u32 t0 = p.streams[u32(p.rlTasks[blockIdx.x * kRlWarps] >> 32)].tableFirst + (kSymbols ? 0u : 1u);
+        stageLut(lutS, p, t0, threadIdx.x, kRlWarps * 32);
+        if (wt < tasks)
+            lutHere = p.streams[u32(p.rlTasks[wt] >> 32)].tableFirst + (kSymbols ? 0u : 1u) == t0;
+        __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        sFail = capacityFailed(p) ? 1u : 0u;
-        sLutTable = hasTask ? t : 0xFFFFFFFFu;
-    }
-    __syncthreads();
-    if (sFail) return;   // CTA-uniform
-    const u32 lutT = sLutTable;
-    if (lutT != 0xFFFFFFFFu) {
-        const u32* g = p.lut + (u64(lutT) << kLutBits);
-        for (u32 e = threadIdx.x; e < (1u << kLutBits); e += 128) sLut[e] = g[e];
-    }
-    __syncthreads();
-    if (!hasTask) return;
+    if (wt >= tasks) return;   // no block-wide barriers below
+    if (__any_sync(0xffffffffu, capacityFailed(p))) return;
+    const u64 task = p.rlTasks[wt];
+    const u32 s = u32(task >> 32), bFirst = u32(task);
     const DecStreamDesc sd = p.streams[s];
-    const u32 b = bFirst + lane;
+    const u32 t = sd.tableFirst + (kSymbols ? 0u : 1u);
     const u32 blocks = rlBlocksOf(p, sd);
-    const bool mine = b < blocks;
-    const u32 nMine = __popc(__ballot_sync(0xffffffffu, mine));   // lanes 0 .. nMine-1
-    if (nMine == 0) return;
-    const DecTableDesc& td = p.tables[t];
+    if (bFirst >= blocks) return;
+    const u32 nMine = min(32u, blocks - bFirst);   // lanes 0 .. nMine-1 have a block
+    const u32 b = bFirst + lane;
+    const bool mine = lane < nMine;
+    const DecTableDesc td = p.tables[t];
     const WordSrc ws = srcOf(p, s);
     const u32* symv = p.syms + td.symOff;
-    const u32* lutG = p.lut + (u64(t) << kLutBits);
-    const bool lutShared = t == lutT;   // warp-uniform
     const DecTable& D = p.dec[t];
     const u32 nSym = D.nSym;
     const bool single = nSym <= 1;
     const u32 singleVal = D.single;
-    bool corrupt = nSym == 0xFFFFFFFFu;
+    const bool bad = nSym == 0xFFFFFFFFu;   // warp-uniform: nothing is decoded
+    bool corrupt = bad;
     const u32 cnt = mine ? min(p.cb, sd.m - b * p.cb) : 0u;
-    BitReader rd{0ull, 0u, 0u, 0u};
-    if (mine && !corrupt && !single) {
-        const u64 bit = td.cwWord * 32ull + p.blockOff[td.blockOff + b];
-        rd.w = bit >> 5;
-        rd.bpos = u32(bit & 31u);
-        rd.hi = ws.at(rd.w);
-        rd.lo = ws.at(rd.w + 1);
-        rd.w += 2;
+    const u32 blockBit = mine ? p.blockOff[td.blockOff + b] : 0u;
+    // the warp's words: from its first block's to the next warp's first, or the stream's end
+    const u32 bit0 = __shfl_sync(0xffffffffu, blockBit, 0);
+    const u32 bit1 = bFirst + 32 < blocks ? p.blockOff[td.blockOff + bFirst + 32] : td.cwBits;
+    const u32 w0 = bit0 >> 5;
+    const u32 nw = bit1 > bit0 ? (bit1 - 1) / 32 - w0 + 1 : 0u;
+    const bool staged = nw <= rlStageWords(p.cb);   // warp-uniform
+    if (staged) stageWords(words, ws, td.cwWord + w0, nw);
+    if (!kSharedLut) stageLut(lutS, p, t, lane, 32);
+    const LongCodes lc = stageLongCodes(cs, p, t);
+    __syncwarp();
+    const StagedWords sw{words, nw};
+    const SourceWords gw{ws, td.cwWord + w0};
+    BitReader rd{0u, 0u, 0u, 0u, 0u};
+    if (mine && !bad && !single) {
+        if (staged) rd.start(sw, blockBit - 32u * w0);
+        else rd.start(gw, blockBit - 32u * w0);
     }
     u32 sum = 0;   // zero counts: the block's sum of (zc + 1)
     // symbols: the block's next output position (its start from the zero-count scan)
     u32 pos = 0;
     if (kSymbols && mine) pos = p.blockSum[p.tables[t + 1].blockOff + b];
-    Sym* rows = sRows[warp];
+    Sym* row = rows + lane * kRlPitch;
+    Sym* zcG = reinterpret_cast<Sym*>(p.zc) + sd.zcOff;
+    Sym* out = reinterpret_cast<Sym*>(sd.out);
     const u32 cnt0 = __shfl_sync(0xffffffffu, cnt, 0);   // the first block is the longest
     for (u32 r0 = 0; r0 < cnt0; r0 += kRlRound) {
         const u32 n = cnt > r0 ? min(kRlRound, cnt - r0) : 0u;
-        if (!corrupt) {
-            auto emit = [&](u32 i, u32 v) {
-                rows[lane * kPitch + i] = Sym(v);
-                if (!kSymbols) sum += v + 1u;
-            };
-            if (single) {
-                for (u32 i = 0; i < n; ++i) emit(i, singleVal);
-            } else if (lutShared) {
-                decodeRun<sizeof(Sym) == 2>(ws, D, nSym, symv, [&](u32 k) { return sLut[k]; }, rd, n, corrupt, emit);
-            } else {
-                decodeRun<sizeof(Sym) == 2>(ws, D, nSym, symv, [&](u32 k) { return lutG[k]; }, rd, n, corrupt, emit);
+        const bool full = __all_sync(0xffffffffu, n == kRlRound || !mine);
+        // symbols: the round's zero counts of the warp's blocks, kVec elements
+        // per lane and step, zero past the stream's m (a part lies whole in
+        // them or is taken element by element)
+        uint4 z[kSymbols ? kParts : 1];
+        if (kSymbols) {
+#pragma unroll
+            for (u32 k = 0; k < kParts; ++k) {
+                const u32 c = k * 32 + lane, j = c / kParts, e = (c % kParts) * kVec;
+                const u32 at = (bFirst + j) * p.cb + r0 + e;
+                z[k] = make_uint4(0u, 0u, 0u, 0u);
+                if (at + kVec <= sd.m) {
+                    z[k] = *reinterpret_cast<const uint4*>(zcG + at);
+                } else if (at < sd.m) {
+                    u32 v[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                    for (u32 q = 0; q < kVec; ++q)
+                        if (at + q < sd.m) v[q / kWordsPer] |= u32(zcG[at + q]) << (16 * (q % kWordsPer));
+                    z[k] = make_uint4(v[0], v[1], v[2], v[3]);
+                }
             }
         }
-        __syncwarp();
-        const u32 k = r0 + lane;   // the element of every block this lane moves
+        if (!bad) {
+            if (full && staged && lutHere && !single) {
+                if (mine) {
+#pragma unroll 1
+                    for (u32 i = 0; i < kRlRound; i += 4) {
+                        u32 v[4];
+#pragma unroll
+                        for (u32 q = 0; q < 4; ++q)
+                            v[q] = decodeOne<kValueLut>(sw, lutS, cs, lc, nSym, symv, rd, corrupt);
+                        putFour(row + i, v[0], v[1], v[2], v[3]);
+                        if (!kSymbols) sum += v[0] + v[1] + v[2] + v[3] + 4u;
+                    }
+                }
+            } else {
+                const u32* lut = lutHere ? lutS : p.lut + (u64(t) << kLutBits);
+                for (u32 i = 0; i < n; ++i) {
+                    const u32 v = single ? singleVal
+                                : staged ? decodeOne<kValueLut>(sw, lut, cs, lc, nSym, symv, rd, corrupt)
+                                         : decodeOne<kValueLut>(gw, lut, cs, lc, nSym, symv, rd, corrupt);
+                    row[i] = Sym(v);
+                    if (!kSymbols) sum += v + 1u;
+                }
+            }
+        }
         if (!kSymbols) {
-            Sym* zc = reinterpret_cast<Sym*>(p.zc) + sd.zcOff;
-            for (u32 j = 0; j < nMine; ++j) {
-                const u32 c = min(p.cb, sd.m - (bFirst + j) * p.cb);
-                if (k < c) zc[u64(bFirst + j) * p.cb + k] = rows[j * kPitch + lane];
+            __syncwarp();
+#pragma unroll
+            for (u32 k = 0; k < kParts; ++k) {
+                const u32 c = k * 32 + lane, j = c / kParts, e = (c % kParts) * kVec;
+                const u32 at = (bFirst + j) * p.cb + r0 + e;
+                if (at + kVec <= sd.m) {
+                    *reinterpret_cast<uint4*>(zcG + at) = rowVec(rows + j * kRlPitch + e);
+                } else {
+                    for (u32 q = 0; q < kVec && at + q < sd.m; ++q) zcG[at + q] = rows[j * kRlPitch + e + q];
+                }
             }
         } else {
-            Sym* zs = sZc[warp];
-            const Sym* zcG = reinterpret_cast<const Sym*>(p.zc) + sd.zcOff;
-            for (u32 j = 0; j < nMine; ++j) {
-                const u32 c = min(p.cb, sd.m - (bFirst + j) * p.cb);
-                zs[j * kRlRound + lane] = k < c ? zcG[u64(bFirst + j) * p.cb + k] : Sym(0);
+#pragma unroll
+            for (u32 k = 0; k < kParts; ++k) {
+                const u32 c = k * 32 + lane, j = c / kParts, e = (c % kParts) * kVec;
+                rowVec(zs + j * kRlPitch + e, z[k]);
             }
             __syncwarp();
-            Sym* out = reinterpret_cast<Sym*>(sd.out);
-            for (u32 j = 0; j < nMine; ++j) {
-                const u32 c = min(p.cb, sd.m - (bFirst + j) * p.cb);
-                const bool act = k < c;
-                const u32 z = act ? u32(zs[j * kRlRound + lane]) : 0u;
-                const u32 v = act ? z + 1u : 0u;
-                u32 incl = v;
+            // positions within the round, in place of the zero counts
+            Sym* zrow = zs + lane * kRlPitch;
+            u32 run = 0;
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const u32 y = __shfl_up_sync(0xffffffffu, incl, d);
-                    if (int(lane) >= d) incl += y;
+            for (u32 i = 0; i < kRlRound; i += 4) {
+                u32 v[4];
+                getFour(zrow + i, v);
+                v[0] += run;
+                v[1] += v[0] + 1u;
+                v[2] += v[1] + 1u;
+                v[3] += v[2] + 1u;
+                run = v[3] + 1u;
+                putFour(zrow + i, v[0], v[1], v[2], v[3]);
+            }
+            run -= kRlRound - n;   // counts past n are zero
+            const bool fits = sizeof(Sym) == 4 || __all_sync(0xffffffffu, run <= 65536u);
+            __syncwarp();
+            if (fits) {
+#pragma unroll 4
+                for (u32 j = 0; j < nMine; ++j) {
+                    const u32 c = full ? kRlRound : __shfl_sync(0xffffffffu, n, j);
+                    const u32 start = __shfl_sync(0xffffffffu, pos, j);
+                    if (lane < c) {
+                        const u32 to = start + u32(zs[j * kRlPitch + lane]);
+                        if (to < sd.n) out[to] = rows[j * kRlPitch + lane];
+                        else corrupt = true;
+                    }
                 }
-                const u32 at = __shfl_sync(0xffffffffu, pos, j) + incl - v + z;
-                if (act) {
-                    if (at < sd.n) out[at] = rows[j * kPitch + lane];
+            } else {
+                // zero counts past the format's 255, positions kept modulo
+                // 2^16: the lane places its own, each count from the difference
+                u32 at = pos - 1u, before = 0xFFFFu;
+                for (u32 i = 0; i < n; ++i) {
+                    const u32 now = u32(zrow[i]);
+                    at += ((now - before - 1u) & 0xFFFFu) + 1u;
+                    before = now;
+                    if (at < sd.n) out[at] = row[i];
                     else corrupt = true;
                 }
-                const u32 tot = __shfl_sync(0xffffffffu, incl, 31);
-                if (lane == j) pos += tot;
             }
+            pos += run;
         }
         __syncwarp();
     }
@@ -821,11 +1024,22 @@ __global__ void __launch_bounds__(256) k_decScan(DecParams p) {
     const u32 k = blockIdx.x * 8u + (threadIdx.x >> 5);
     if (k >= p.nRl) return;
     const DecStreamDesc sd = p.streams[p.rlList[k]];
-    const u32 blocks = u32(ceilDiv(sd.m, p.cb));
+    const u32 blocks = blocksOf(sd.m, p.cbLog);
     u32* bs = p.blockSum + p.tables[sd.tableFirst + 1].blockOff;
     const u32 total = warpExclusiveScan8(bs, bs, blocks, 0u);
     // the last symbol's position must be < n: total length <= n
     if ((threadIdx.x & 31u) == 0 && total > sd.n) atomicOr(p.errors, DEV_ERR_CORRUPT);
+}
+
+// The same with a CTA per stream, for calls of few: a warp takes 38 us over the
+// 16384 blocks of a 256^3 volume's band, 512 threads 13.
+__global__ void __launch_bounds__(512) k_decScanWide(DecParams p) {
+    __shared__ u32 scratch[40];
+    const DecStreamDesc sd = p.streams[p.rlList[blockIdx.x]];
+    const u32 blocks = blocksOf(sd.m, p.cbLog);
+    u32* bs = p.blockSum + p.tables[sd.tableFirst + 1].blockOff;
+    const u32 total = blockExclusiveScan8<512>(bs, bs, blocks, scratch);
+    if (threadIdx.x == 0 && total > sd.n) atomicOr(p.errors, DEV_ERR_CORRUPT);
 }
 
 // ---------------------------------------------------------------------------
@@ -940,7 +1154,7 @@ static int planDecode(cc_instance* I, const u32* kinds, const u32* ns, void* con
             dc.rlMaxN = std::max<u32>(dc.rlMaxN, ns[s]);
         } else {
             d.blockFirst = u32(hBlocks);
-            hBlocks += nb;
+            hBlocks += huffBlocksPlanned(nb);
             hl[dc.nH++] = s;
         }
         sd[s] = d;
@@ -964,52 +1178,106 @@ static int planDecode(cc_instance* I, const u32* kinds, const u32* ns, void* con
     return CC_OK;
 }
 
+// The run-length decode kernels by symbol and lookup table place, with their
+// dynamic shared memory.
+template <class Sym, bool kSymbols, bool kSharedLut>
+static cudaError_t rlSmemAttribute(cc_instance* I) {
+    const int which = kAttrDecRl + (sizeof(Sym) == 4 ? 4 : 0) + (kSymbols ? 2 : 0) + (kSharedLut ? 1 : 0);
+    return ensureSmemAttribute(reinterpret_cast<const void*>(k_decRl<Sym, kSymbols, kSharedLut>), which, I->device,
+                               rlSmem<Sym, kSymbols, kSharedLut>(I->codingBlockSize));
+}
+
+template <class Sym>
+static cudaError_t decodeSmemAttributes(cc_instance* I) {
+    cudaError_t e = ensureSmemAttribute(reinterpret_cast<const void*>(k_decHuff<Sym>),
+                                        sizeof(Sym) == 4 ? kAttrDecHuff32 : kAttrDecHuff16, I->device,
+                                        huffSmem<Sym>(I->codingBlockSize));
+    if (e == cudaSuccess) e = rlSmemAttribute<Sym, false, false>(I);
+    if (e == cudaSuccess) e = rlSmemAttribute<Sym, false, true>(I);
+    if (e == cudaSuccess) e = rlSmemAttribute<Sym, true, false>(I);
+    if (e == cudaSuccess) e = rlSmemAttribute<Sym, true, true>(I);
+    return e;
+}
+
+template <class Sym, bool kSymbols>
+static void launchRl(const DecParams& p, u32 ctas, cudaStream_t st) {
+    if (p.rlBlocks / 32 >= u64(kRlSharedTasks) * p.nRl)
+        k_decRl<Sym, kSymbols, true><<<ctas, kRlWarps * 32, rlSmem<Sym, kSymbols, true>(p.cb), st>>>(p);
+    else
+        k_decRl<Sym, kSymbols, false><<<ctas, kRlWarps * 32, rlSmem<Sym, kSymbols, false>(p.cb), st>>>(p);
+    countLaunch();
+}
+
 template <class Sym>
 static int launchDecodeBackEnd(cc_instance* I, const DecParams& p) {
     cudaStream_t st = I->stream;
-    {
-        SectionTimer t(I, "dec.sym_plan", st);
-        const u32 chunks = std::max<u32>(1, u32(ceilDiv(p.T, kPlanChunk)));
-        k_decSymPlan<<<chunks, 1024, 0, st>>>(p);
-        countLaunch();
-        if (chunks > 1) { k_decSymPlanCarry<<<chunks - 1, 1024, 0, st>>>(p); countLaunch(); }
-    }
-    { SectionTimer t(I, "dec.tables", st); k_decTables<<<p.T, kDecThreads, 0, st>>>(p); countLaunch(); }
-    // the Huff streams decode on a side stream beside the RLHuff chain (they
-    // share only the read-only tables and the error flags), joined below
+    CC_TRY_CUDA(decodeSmemAttributes<Sym>(I), "decode smem");
+    // a side stream beside the RLHuff chain: the zero fill of its outputs,
+    // which it needs before the symbols, and the Huff streams' decode (the two
+    // share only the read-only tables and the error flags), joined at the end
     const bool fork = p.hBlocks && p.rlBlocks;
     cudaStream_t hs = fork ? I->buildSide2 : st;
+    auto zeroFill = [&](cudaStream_t q) {
+        SectionTimer t(I, "dec.zero_fill", q);
+        k_decZero<Sym><<<dim3(p.nRl, u32(ceilDiv(p.rlMaxN, kZeroChunk))), 256, 0, q>>>(p);
+        countLaunch();
+    };
     if (fork) {
         CC_TRY_CUDA(cudaEventRecord(I->decFork, st), "decode fork");
         CC_TRY_CUDA(cudaStreamWaitEvent(hs, I->decFork, 0), "decode fork");
+        zeroFill(hs);
+        CC_TRY_CUDA(cudaEventRecord(I->decZeroed, hs), "decode zero fill");
+    }
+    const u32 symChunks = std::max<u32>(1, u32(ceilDiv(p.T, kPlanChunk)));
+    const u32 rlChunks = std::max<u32>(1, u32(ceilDiv(p.nRl, 1024)));
+    const bool onePlan = symChunks == 1 && rlChunks == 1 && p.rlBlocks;
+    {
+        SectionTimer t(I, "dec.sym_plan", st);
+        if (onePlan) k_decPlans<<<2, 1024, 0, st>>>(p);
+        else k_decSymPlan<<<symChunks, 1024, 0, st>>>(p);
+        countLaunch();
+        if (symChunks > 1) { k_decSymPlanCarry<<<symChunks - 1, 1024, 0, st>>>(p); countLaunch(); }
+    }
+    {
+        SectionTimer t(I, "dec.tables", st);
+        if (p.T <= kDecWideTables) k_decTables<kDecThreadsWide><<<p.T, kDecThreadsWide, 0, st>>>(p);
+        else k_decTables<kDecThreads><<<p.T, kDecThreads, 0, st>>>(p);
+        countLaunch();
+    }
+    if (fork) {
+        CC_TRY_CUDA(cudaEventRecord(I->decTablesReady, st), "decode tables");
+        CC_TRY_CUDA(cudaStreamWaitEvent(hs, I->decTablesReady, 0), "decode tables");
     }
     if (p.hBlocks) {
-        const size_t smem = size_t(32) * (p.cb + 2) * sizeof(Sym);
-        CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_decHuff<Sym>),
-                                        sizeof(Sym) == 2 ? kAttrDecHuff16 : kAttrDecHuff32, I->device, smem),
-                    "decHuff smem");
         SectionTimer t(I, "dec.huffman", hs);
-        k_decHuff<Sym><<<u32(ceilDiv(p.hBlocks, 32)), 32, smem, hs>>>(p);
+        k_decHuff<Sym><<<u32(ceilDiv(p.hBlocks, 32)), 32, huffSmem<Sym>(p.cb), hs>>>(p);
         countLaunch();
     }
     if (fork) CC_TRY_CUDA(cudaEventRecord(I->decJoin, hs), "decode join");
     if (p.rlBlocks) {
-        const u32 g = u32(ceilDiv(u64(p.rlBlocks) / 32 + p.nRl, 4));   // warp tasks <= rlBlocks / 32 + nRl
-        {
+        const u32 g = u32(ceilDiv(u64(p.rlBlocks) / 32 + p.nRl, kRlWarps));   // warp tasks <= rlBlocks / 32 + nRl
+        if (!onePlan) {
             SectionTimer t(I, "dec.rl_tasks", st);
-            const u32 chunks = std::max<u32>(1, u32(ceilDiv(p.nRl, 1024)));
-            if (chunks > 1) { k_decRlTaskCounts<<<chunks, 1024, 0, st>>>(p); countLaunch(); }
-            k_decRlTasks<<<chunks, 1024, 0, st>>>(p);
+            if (rlChunks > 1) { k_decRlTaskCounts<<<rlChunks, 1024, 0, st>>>(p); countLaunch(); }
+            k_decRlTasks<<<rlChunks, 1024, 0, st>>>(p);
             countLaunch();
+        }
+        if (!fork) zeroFill(st);
+        {
+            SectionTimer t(I, "dec.zero_counts", st);
+            launchRl<Sym, false>(p, g, st);
         }
         {
-            SectionTimer t(I, "dec.zero_fill", st);
-            k_decZero<Sym><<<dim3(p.nRl, u32(ceilDiv(p.rlMaxN, kZeroChunk))), 256, 0, st>>>(p);
+            SectionTimer t(I, "dec.run_scan", st);
+            if (p.nRl <= kDecWideTables) k_decScanWide<<<p.nRl, 512, 0, st>>>(p);
+            else k_decScan<<<u32(ceilDiv(p.nRl, 8)), 256, 0, st>>>(p);
             countLaunch();
         }
-        { SectionTimer t(I, "dec.zero_counts", st); k_decRl<Sym, false><<<g, 128, 0, st>>>(p); countLaunch(); }
-        { SectionTimer t(I, "dec.run_scan", st); k_decScan<<<u32(ceilDiv(p.nRl, 8)), 256, 0, st>>>(p); countLaunch(); }
-        { SectionTimer t(I, "dec.symbols_scatter", st); k_decRl<Sym, true><<<g, 128, 0, st>>>(p); countLaunch(); }
+        if (fork) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->decZeroed, 0), "decode zero fill");
+        {
+            SectionTimer t(I, "dec.symbols_scatter", st);
+            launchRl<Sym, true>(p, g, st);
+        }
     }
     if (fork) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->decJoin, 0), "decode join");
     CC_TRY_CUDA(cudaGetLastError(), "decode launch");
@@ -1017,13 +1285,7 @@ static int launchDecodeBackEnd(cc_instance* I, const DecParams& p) {
 }
 
 int prepareDecodeAttributes(cc_instance* I) {
-    const size_t smem = size_t(32) * (I->codingBlockSize + 2) * I->symBytes;
-    const int dev = I->device;
-    if (I->symBytes == 2) {
-        CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_decHuff<u16>), kAttrDecHuff16, dev, smem), "decHuff smem");
-    } else {
-        CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_decHuff<u32>), kAttrDecHuff32, dev, smem), "decHuff smem");
-    }
+    CC_TRY_CUDA(I->symBytes == 2 ? decodeSmemAttributes<u16>(I) : decodeSmemAttributes<u32>(I), "decode smem");
     return CC_OK;
 }
 
@@ -1039,6 +1301,7 @@ static DecParams makeDecParams(cc_instance* I, const DecPlan& dc) {
     p.rlMaxN = dc.rlMaxN;
     p.hBlocks = dc.hBlocks;
     p.cb = I->codingBlockSize;
+    p.cbLog = 31u - u32(__builtin_clz(p.cb));
     p.log2Max = I->log2Max;
     p.symBytes = I->symBytes;
     p.leavesMax = I->leavesMax;
@@ -1178,7 +1441,7 @@ int decodeLaunch(cc_instance* I, const DecPlan& dc) {
     cudaStream_t st = I->stream;
     CC_TRY_CUDA(cudaMemsetAsync(I->errors + 4, 0, sizeof(u32), st), "memset errors");
     const DecParams p = makeDecParams(I, dc);
-    { SectionTimer t(I, "dec.walk", st); k_decWalk<<<u32(ceilDiv(dc.B, 64)), 64, 0, st>>>(p); countLaunch(); }
+    { SectionTimer t(I, "dec.walk", st); k_decWalk<<<u32(ceilDiv(dc.B, kWalkWarps)), kWalkWarps * 32, 0, st>>>(p); countLaunch(); }
     return I->symBytes == 2 ? launchDecodeBackEnd<u16>(I, p) : launchDecodeBackEnd<u32>(I, p);
 }
 

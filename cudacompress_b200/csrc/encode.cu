@@ -23,7 +23,7 @@ namespace ccb {
 struct EncParams {
     u32 S, T;
     u32 totalTiles, totalBlocks;
-    u32 cb, log2Max, bins, symBytes;
+    u32 cb, cbLog, log2Max, bins, symBytes;   // cb = 2^cbLog
     const EncStreamDev* streams;
     const EncTableDev* tables;
     char* compact;
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256) k_usedBlocks(EncParams p) {
     if (t >= p.T) return;
     const TableMeta& m = p.meta[t];
     for (u32 k = lane; k < m.blocks; k += 32) p.blockTable[m.actOff + k] = t;
-    const u32 runs = u32(ceilDiv(m.blocks, kRunSymbols / p.cb));
+    const u32 runs = blocksOf(m.blocks, kRunLog - p.cbLog);
     for (u32 k = lane; k < runs; k += 32) p.runTable[m.runOff + k] = t;
 }
 
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
             ws = headerWordsFor(ls, p.log2Max);
             m[j].count = count;
             m[j].histSize = hs;
-            m[j].blocks = u32(ceilDiv(count, p.cb));
+            m[j].blocks = blocksOf(count, p.cbLog);
         }
         v[j][0] = 0;
         v[j][1] = 0;
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
         v[j][3] = ls;
         v[j][4] = ws;
         v[j][5] = m[j].blocks;
-        v[j][6] = u32(ceilDiv(m[j].blocks, kRunSymbols / p.cb));
+        v[j][6] = blocksOf(m[j].blocks, kRunLog - p.cbLog);
     }
     u32 sum[7], ex[7], tot[7];
 #pragma unroll
@@ -941,7 +941,7 @@ __global__ void __launch_bounds__(kPackWarps * 32) k_blockBits(EncParams p) {
     const u32 lane = threadIdx.x & 31;
     if (warpFailed(p)) return;
     const u32 runs = u32(p.totals[3]);
-    const u32 lpb = p.cb / 32u, bpr = kRunSymbols / p.cb;
+    const u32 lpb = p.cb >> 5, bpr = kRunSymbols >> p.cbLog;
     const u32 stride = gridDim.x * kPackWarps;
     for (u32 r = blockIdx.x * kPackWarps + (threadIdx.x >> 5); r < runs; r += stride) {
         const u32 t = p.runTable[r];
@@ -960,8 +960,8 @@ __global__ void __launch_bounds__(kPackWarps * 32) k_blockBits(EncParams p) {
         for (u32 k = 0; k < 32; ++k)
             if (j0 + k < count) bits += enc[min(sv.at(k), hs - 1u)].y;
         for (u32 o = 1; o < lpb; o <<= 1) bits += __shfl_xor_sync(0xffffffffu, bits, o);
-        const u32 b = rb * bpr + lane / lpb;
-        if (lane % lpb == 0 && b < m.blocks) p.blockBits[td.blockOff + b] = bits;
+        const u32 b = rb * bpr + (lane >> (p.cbLog - 5u));
+        if ((lane & (lpb - 1u)) == 0 && b < m.blocks) p.blockBits[td.blockOff + b] = bits;
     }
 }
 
@@ -985,7 +985,7 @@ __global__ void __launch_bounds__(256) k_layoutSegments(EncParams p) {
     if (s >= p.S) return;
     SegmentLayout L{};
     const EncStreamDev sd = p.streams[s];
-    const u32 offW = u32(ceilDiv(ceilDiv(p.counts[s], p.cb), 2));
+    const u32 offW = (blocksOf(p.counts[s], p.cbLog) + 1u) / 2u;
     const TableMeta ms = p.meta[sd.tableFirst];
     u32 words;
     if (sd.kind == KIND_RLHUFF) {
@@ -1090,7 +1090,7 @@ __global__ void __launch_bounds__(kPackWarps * 32, 3) k_pack(EncParams p) {
     if (warpFailed(p)) return;
     u32* win = winAll + warp * kPackWindowWords;
     const u32 runs = u32(p.totals[3]);
-    const u32 bpr = kRunSymbols / p.cb;
+    const u32 bpr = kRunSymbols >> p.cbLog;
     const u32 stride = gridDim.x * kPackWarps;
     for (u32 r = blockIdx.x * kPackWarps + warp; r < runs; r += stride) {
         const u32 t = p.runTable[r];
@@ -1477,6 +1477,7 @@ int encodeLaunch(cc_instance* I, const EncPlan& hp, u32* out, u64 outCap) {
     p.totalTiles = hp.tiles;
     p.totalBlocks = hp.blocks;
     p.cb = I->codingBlockSize;
+    p.cbLog = 31u - u32(__builtin_clz(p.cb));
     p.log2Max = I->log2Max;
     p.bins = I->bins;
     p.symBytes = I->symBytes;

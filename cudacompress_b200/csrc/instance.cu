@@ -296,6 +296,8 @@ int createInstance(cc_instance** out, int cudaDevice, u32 streamCountMax, u32 el
         (e = cudaEventCreateWithFlags(&I->buildJoin, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&I->buildJoin2, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&I->decFork, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&I->decZeroed, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&I->decTablesReady, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&I->decJoin, cudaEventDisableTiming)) != cudaSuccess) {
         cc_destroy_instance(I);
         return cudaFail(e, "table build stream");
@@ -334,6 +336,8 @@ void cc_destroy_instance(cc_instance* I) {
     if (I->buildJoin) cudaEventDestroy(I->buildJoin);
     if (I->buildJoin2) cudaEventDestroy(I->buildJoin2);
     if (I->decFork) cudaEventDestroy(I->decFork);
+    if (I->decZeroed) cudaEventDestroy(I->decZeroed);
+    if (I->decTablesReady) cudaEventDestroy(I->decTablesReady);
     if (I->decJoin) cudaEventDestroy(I->decJoin);
     if (I->buildSide) cudaStreamDestroy(I->buildSide);
     if (I->buildSide2) cudaStreamDestroy(I->buildSide2);
