@@ -111,10 +111,7 @@ struct Arena {
 u64 vol3(u32 x, u32 y, u32 z) { return u64(x) * y * z; }
 
 void addRows(std::vector<BRowDesc>& v, u32& ctas, BRowDesc d) {
-    batchRowTiling(d.nx, d.W, d.R);
-    d.tilesX = int(ceilDiv(d.nx, d.W));
-    d.vec = (d.nx % 8 == 0 && d.W % 8 == 0 && d.srcRow % 4 == 0 && d.srcSlice % 4 == 0 && d.dstRow % 4 == 0 &&
-             d.dstSlice % 4 == 0) ? 1 : 0;
+    batchRowPlan(d);
     d.ctaOff = ctas;
     ctas += u32(d.tilesX) * u32(ceilDiv(u64(d.ny) * d.nz, d.R));
     v.push_back(d);

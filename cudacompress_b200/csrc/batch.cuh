@@ -107,6 +107,19 @@ inline void batchRowTiling(int nx, int& W, int& R) {
     if (R > kBRowMaxRows) R = kBRowMaxRows;
 }
 
+// Fills a row descriptor's tiling and vector flag from its extents and pitches.
+inline void batchRowPlan(BRowDesc& d) {
+    batchRowTiling(d.nx, d.W, d.R);
+    d.tilesX = int(ceilDiv(d.nx, d.W));
+    d.vec = (d.nx % 8 == 0 && d.W % 8 == 0 && d.srcRow % 4 == 0 && d.srcSlice % 4 == 0 && d.dstRow % 4 == 0 &&
+             d.dstSlice % 4 == 0) ? 1 : 0;
+}
+
+// One 2D level of the integer transform between samples and symbol bands (dwt.cu).
+void liftForwardToBands(i16* ll, u16* const (&band)[3], i16* tmp, const i16* src, int sx, int sy, int srcRow,
+                        cudaStream_t st);
+void liftInverseFromBands(i16* dst, u16* const (&band)[3], i16* tmp, const i16* ll, int sx, int sy, cudaStream_t st);
+
 // New quantization steps for a batch's volumes (batch.cu).
 int batchSetQuantSteps(cc_volume_batch* b, const float* q);
 // The error status of the batch's last compress (decode false) or decompress

@@ -643,31 +643,26 @@ int cc_compress_heightfield(cc_instance* I, const int16_t* img, uint32_t nx, uin
     i16* coefB = w.take<i16>(N0);
     i16* tmp = w.take<i16>(N0);
     u16* syms = w.take<u16>(N0 + 1024);
-    // level l: transform the (dense) lowpass of level l-1
-    std::vector<i16*> coef(levels);
+    // level l: transform the lowpass of level l-1 (dense; the two areas in
+    // turn), its highpass bands straight to symbols
     const i16* src = img;
     u16* next = syms;
     std::vector<std::vector<u16*>> bands(levels, std::vector<u16*>(3));
     for (u32 l = 0; l < levels; ++l) {
         const u32 sx = nx >> l, sy = ny >> l;
-        i16* dst = (l % 2 == 0) ? coefA : coefB;
-        rc = cc_dwt_int_forward(dst, tmp, src, int(sx), int(sy), 1, 0, 0, int(l == 0 ? nx : (nx >> (l - 1))), 0, st);
-        if (rc) return rc;
-        const u32 hx = sx / 2, hy = sy / 2;
-        for (u32 bi = 1; bi < 4; ++bi) {
-            const u32 x = bi % 2, y = bi / 2;
-            rc = cc_symbolize(next, dst + u64(y) * hy * sx + u64(x) * hx, hx, hy, 1, sx, 0, st);
-            if (rc) return rc;
-            bands[l][bi - 1] = next;
-            next += u64(hx) * hy;
-        }
-        coef[l] = dst;
-        src = dst;   // LL corner, row pitch sx (passed above as the next level's source pitch)
+        i16* ll = (l % 2 == 0) ? coefA : coefB;
+        const u64 bandN = u64(sx / 2) * (sy / 2);
+        u16* const band[3] = {next, next + bandN, next + 2 * bandN};
+        liftForwardToBands(ll, band, tmp, src, int(sx), int(sy), int(sx), st);
+        for (u32 i = 0; i < 3; ++i) bands[l][i] = band[i];
+        next += 3 * bandN;
+        src = ll;
     }
+    CC_TRY_CUDA(cudaGetLastError(), "compressHeightfield transform");
     const u32 L = levels;
     const u32 lx = nx >> L, ly = ny >> L;
     u16* lp = next;
-    rc = cc_symbolize(lp, coef[L - 1], lx, ly, 1, nx >> (L - 1), 0, st);
+    rc = cc_symbolize(lp, src, lx, ly, 1, lx, 0, st);
     if (rc) return rc;
     std::vector<EncStream> es;
     std::vector<EncGroup> groups;
@@ -758,13 +753,11 @@ int cc_decompress_heightfield(cc_instance* I, int16_t* out, uint32_t nx, uint32_
     Bump b{nullptr};
     b.take<i16>(N0);
     b.take<i16>(N0);
-    b.take<i16>(N0);
     b.take<u16>(N0 + 1024);
     int rc = ensurePipelineWork(I, b.off + 1024);
     if (rc) return rc;
     Bump w{I->pipeWork};
     i16* cur = w.take<i16>(N0);
-    i16* coef = w.take<i16>(N0);
     i16* tmp = w.take<i16>(N0);
     u16* syms = w.take<u16>(N0 + 1024);
     // every stream of every level in one device-walked decode: the LP stream
@@ -795,19 +788,12 @@ int cc_decompress_heightfield(cc_instance* I, int16_t* out, uint32_t nx, uint32_
     rc = cc_unsymbolize(cur, syms, lx, ly, 1, 0, 0, st);
     if (rc) return rc;
     for (int l = int(L) - 1; l >= 0; --l) {
-        const u32 sx = nx >> l, sy = ny >> l, hx = sx / 2, hy = sy / 2;
-        const u64 bandN = u64(hx) * hy;
-        // assemble [LL | HL ; LH | HH] of this level then invert
-        CC_TRY_CUDA(cudaMemcpy2DAsync(coef, sx * sizeof(i16), cur, hx * sizeof(i16), hx * sizeof(i16), hy,
-                                      cudaMemcpyDeviceToDevice, st), "place lowpass");
-        for (u32 bi = 1; bi < 4; ++bi) {
-            const u32 x = bi % 2, y = bi / 2;
-            rc = cc_unsymbolize(coef + u64(y) * hy * sx + u64(x) * hx, bandAt[l] + (bi - 1) * bandN, hx, hy, 1, sx, 0, st);
-            if (rc) return rc;
-        }
-        rc = cc_dwt_int_inverse(l == 0 ? out : cur, tmp, coef, int(sx), int(sy), 1, 0, 0, 0, 0, st);
-        if (rc) return rc;
+        const u32 sx = nx >> l, sy = ny >> l;
+        const u64 bandN = u64(sx / 2) * (sy / 2);
+        u16* const band[3] = {bandAt[l], bandAt[l] + bandN, bandAt[l] + 2 * bandN};
+        liftInverseFromBands(l == 0 ? out : cur, band, tmp, cur, int(sx), int(sy), st);
     }
+    CC_TRY_CUDA(cudaGetLastError(), "decompressHeightfield transform");
     CC_TRY_CUDA(cudaStreamSynchronize(st), "decompressHeightfield");
     return cc_decode_status(I);
 }
