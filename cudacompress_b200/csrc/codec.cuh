@@ -116,7 +116,6 @@ struct TableMeta {
     u32 codeBits;     // total codeword bits
     u32 blocks;       // coding blocks
     u32 histSize;     // histogram bins of this table
-    u32 actOff;       // first of its coding blocks in the call's list of used blocks
     u32 runOff;       // first of its runs (kRunSymbols symbols of coding blocks) in the call's run list
     u64 histOff;      // offset of its histogram and code table
     u64 leafOff;      // offset of its table-builder arrays (by leaf)
@@ -242,7 +241,6 @@ struct cc_instance {
     ccb::u32* headers = nullptr;       // [capHdr]
     ccb::u32* blockBits = nullptr;     // [capBlocks]
     ccb::u32* blockOff = nullptr;      // [capBlocks]
-    ccb::u32* blockTable = nullptr;    // [capBlocks]: table of each coding block of a call
     ccb::u32* runTable = nullptr;      // [capBlocks]: table of each run of coding blocks of a call
     ccb::u32* tileStream = nullptr;    // [capTiles]: stream of each run-length tile of a call
     ccb::SegmentLayout* layout = nullptr;  // [capStreams]

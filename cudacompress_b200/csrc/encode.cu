@@ -38,8 +38,7 @@ struct EncParams {
     u32* headers;
     u32* blockBits;
     u32* blockOff;
-    u32* blockTable;  // [used blocks] table of each coding block in use (k_usedBlocks)
-    u32* runTable;    // [runs] table of each run of coding blocks (k_usedBlocks)
+    u32* runTable;    // [runs] table of each run of coding blocks (k_planFill)
     u32* tileStream;  // [totalTiles] stream of each run-length tile (k_lookupMaps)
     SegmentLayout* layout;
     u32* out;
@@ -176,27 +175,16 @@ __device__ __forceinline__ RunSum warpInclusiveRun(RunSum r) {
     return r;
 }
 
-// The call's tile map: CTA s writes the stream index over its tiles (the
-// prefix layout of the call's descriptors).
-__global__ void __launch_bounds__(256) k_lookupMaps(EncParams p) {
+// The start of a call: CTA s writes the stream index over its tiles (the
+// prefix layout of the call's descriptors) and clears the stream's largest
+// symbol; the first also the error flags.
+__global__ void __launch_bounds__(256) k_encBegin(EncParams p) {
     const u32 i = blockIdx.x;
+    if (i == 0 && threadIdx.x < 4) p.errors[threadIdx.x] = 0;
+    if (threadIdx.x == 0) p.streamMax[i] = 0;
     const EncStreamDev& sd = p.streams[i];
     const u32 tiles = u32(ceilDiv(sd.n, kRleTile));
     for (u32 k = threadIdx.x; k < tiles; k += 256) p.tileStream[sd.tileOff + k] = i;
-}
-
-// The coding blocks in use (those holding symbols after the run-length
-// step), listed table by table: warp t writes t over its meta.blocks entries
-// from meta.actOff (k_histPlan).  The block-level kernels walk this list
-// instead of every block a table could have.
-__global__ void __launch_bounds__(256) k_usedBlocks(EncParams p) {
-    if (warpFailed(p)) return;
-    const u32 t = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;   // a warp per table
-    if (t >= p.T) return;
-    const TableMeta& m = p.meta[t];
-    for (u32 k = lane; k < m.blocks; k += 32) p.blockTable[m.actOff + k] = t;
-    const u32 runs = blocksOf(m.blocks, kRunLog - p.cbLog);
-    for (u32 k = lane; k < runs; k += 32) p.runTable[m.runOff + k] = t;
 }
 
 // ---------------------------------------------------------------------------
@@ -251,9 +239,7 @@ __global__ void __launch_bounds__(kRleThreads) k_summary(EncParams p) {
 constexpr u32 kScanWarps = 8;   // warps (streams or tables) per CTA of the per-unit scans
 
 // Pass 2: the scan of each stream's tile summaries, a warp per stream.
-__global__ void __launch_bounds__(kScanWarps * 32) k_scan(EncParams p) {
-    const u32 s = blockIdx.x * kScanWarps + (threadIdx.x >> 5);
-    if (s >= p.S) return;
+__device__ __forceinline__ void scanStream(const EncParams& p, u32 s) {
     const u32 lane = threadIdx.x & 31u;
     const EncStreamDev sd = p.streams[s];
     if (sd.kind != KIND_RLHUFF) {
@@ -286,13 +272,18 @@ __global__ void __launch_bounds__(kScanWarps * 32) k_scan(EncParams p) {
     if (lane == 0) p.counts[s] = carry.cnt ? carry.cnt + carry.ext + (carry.firstP1 - 1u) / 256u : 0u;
 }
 
+__global__ void __launch_bounds__(kScanWarps * 32) k_scan(EncParams p) {
+    const u32 s = blockIdx.x * kScanWarps + (threadIdx.x >> 5);
+    if (s < p.S) scanStream(p, s);
+}
+
 // Table builders by leaf count (k_leafTiers sorts the tables, k_tableBuild
 // builds them): the heap merge is a latency-bound chain on one warp, so a
 // smaller table gets a smaller CTA and heap and more of them share an SM.
 //   tier 0: up to 256 leaves, a warp, 5 KB of heap (32 per SM)
 //   tier 1: up to 1024 leaves, 64 threads, 20 KB (10 per SM)
-//   tier 2: up to 2048 leaves, 256 threads, 41 KB (5 per SM)
-//   tier 3: more, 256 threads, the full heap (one per SM)
+//   tier 2: up to 2048 leaves, 128 threads, 41 KB (5 per SM)
+//   tier 3: more, 512 threads, the full heap (one per SM)
 constexpr u32 kTinyLeaves = 256;
 constexpr u32 kSmallLeaves = 1024;
 constexpr u32 kBuildSplitLeaves = 2048;
@@ -320,8 +311,7 @@ __device__ __forceinline__ void planTotals(const EncParams& p, const unsigned lo
     if (c[2] > p.capHist || c[3] > p.capLeaves || c[4] > p.capHdr) atomicOr(p.errors, DEV_ERR_TABLE_CAPACITY);
 }
 
-__global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
-    __shared__ u32 scratch[33 * 7];
+__device__ __forceinline__ void histPlanChunk(const EncParams& p, u32* scratch) {
     const u32 t0 = blockIdx.x * kPlanChunk + threadIdx.x * kPlanPer;
     // per table: (unused), (unused), bins, leaves, header words, blocks, runs
     u32 v[kPlanPer][7];
@@ -369,7 +359,6 @@ __global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
             m[j].histOff = at[2];
             m[j].leafOff = at[3];
             m[j].hdrOff = at[4];
-            m[j].actOff = u32(at[5]);
             m[j].runOff = u32(at[6]);
             p.meta[t] = m[j];
         }
@@ -387,6 +376,21 @@ __global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
             for (u32 k = 0; k < 7; ++k) p.planPart[u64(blockIdx.x) * 8 + k] = tot[k];
         }
     }
+}
+
+__global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
+    __shared__ u32 scratch[33 * 7];
+    histPlanChunk(p, scratch);
+}
+
+// Passes 2 and 3 of a call of few streams in one CTA, two of them per warp.
+constexpr u32 kScanPlanStreams = 64;
+
+__global__ void __launch_bounds__(1024) k_scanPlan(EncParams p) {
+    __shared__ u32 scratch[33 * 7];
+    for (u32 s = threadIdx.x >> 5; s < p.S; s += 32) scanStream(p, s);
+    __syncthreads();   // the CTA's counts
+    histPlanChunk(p, scratch);
 }
 
 // Chunk b = blockIdx.x + 1 of a plan of more than one chunk: the sums of
@@ -418,7 +422,6 @@ __global__ void __launch_bounds__(1024) k_histPlanCarry(EncParams p) {
             m.histOff += sC[2];
             m.leafOff += sC[3];
             m.hdrOff += sC[4];
-            m.actOff += u32(sC[5]);
             m.runOff += u32(sC[6]);
         }
     }
@@ -430,10 +433,19 @@ __global__ void __launch_bounds__(1024) k_histPlanCarry(EncParams p) {
     }
 }
 
-__global__ void __launch_bounds__(256) k_zeroHist(EncParams p) {
-    if (*reinterpret_cast<volatile const u32*>(p.errors)) return;   // no barriers in this kernel
+// After the plan: the call's histograms zeroed, and the runs of coding blocks
+// in use (those holding symbols after the run-length step) listed table by
+// table - warp t writes t over its runs from meta.runOff.  The block-level
+// kernels walk this list instead of every block a table could have.
+__global__ void __launch_bounds__(256) k_planFill(EncParams p) {
+    if (warpFailed(p)) return;
+    const u32 thread = blockIdx.x * 256u + threadIdx.x, threads = gridDim.x * 256u, lane = threadIdx.x & 31u;
     const u64 total = p.totals[1];
-    for (u64 i = u64(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += u64(gridDim.x) * blockDim.x) p.hist[i] = 0;
+    for (u64 i = thread; i < total; i += threads) p.hist[i] = 0;
+    for (u32 t = thread >> 5; t < p.T; t += threads >> 5) {
+        const u32 runs = blocksOf(p.meta[t].blocks, kRunLog - p.cbLog), off = p.meta[t].runOff;
+        for (u32 k = lane; k < runs; k += 32) p.runTable[off + k] = t;
+    }
 }
 
 // The leaf count of every table (the nonzero bins of its histogram; a warp
@@ -657,7 +669,10 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
 // more leaves than the shared-memory builder holds run sequentially on
 // global memory (huffman_build.cuh).
 // ---------------------------------------------------------------------------
-constexpr u32 kBuildThreads = 256;
+constexpr u32 kBuildThreads = 256, kMidThreads = 128;
+// the full builder, a CTA of its own on an SM: the merge is one warp's, the
+// sort's deep rounds and the walks over leaves take all
+constexpr u32 kBigThreads = 512;
 
 __device__ __forceinline__ void putBits(u32* words, u32 pos, u32 value, u32 count) {
     // MSB-first, count <= 32, words pre-zeroed; atomics because neighbouring
@@ -863,7 +878,7 @@ __device__ void buildTable(const EncParams& p, u32 t) {
 
 // One table per CTA (kBuildEach), or the CTAs walk the list of one tier.
 template <u32 kThreads, u32 kCap>
-__global__ void __launch_bounds__(kThreads) k_tableBuild(EncParams p) {
+__global__ void __launch_bounds__(kThreads, 1) k_tableBuild(EncParams p) {
     if (p.buildTier == kBuildEach) {
         buildTable<kThreads, kCap>(p, blockIdx.x);
         return;
@@ -886,7 +901,7 @@ static size_t tableBuildSoloSmem(int device) {
         int optin = 0;
         cudaFuncAttributes fa{};
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-        cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, kBuildSmemLeaves>));
+        cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(k_tableBuild<kBigThreads, kBuildSmemLeaves>));
         cached[device] = optin > int(fa.sharedSizeBytes) ? size_t(optin) - fa.sharedSizeBytes : 0;
     }
     return cached[device];
@@ -933,7 +948,7 @@ struct LaneRun {
 };
 
 // Bits of every coding block in use.  Warps walk the call's run list
-// (k_usedBlocks): a run is kRunSymbols consecutive symbols of one table, 32
+// (k_planFill): a run is kRunSymbols consecutive symbols of one table, 32
 // per lane, so cb / 32 lanes share a coding block; each lane sums the code
 // lengths of its symbols and the block's lanes add theirs.
 template <class Sym>
@@ -977,12 +992,22 @@ __global__ void __launch_bounds__(kScanWarps * 32) k_blockScan(EncParams p) {
     if ((threadIdx.x & 31u) == 0) p.meta[t].codeBits = total;
 }
 
+// The same with a CTA per table, for calls of few tables: 512 threads over the
+// 16384 blocks of a 256^3 volume's band take 6 us, a warp 25.
+constexpr u32 kWideScanTables = 4 * 148;
+
+__global__ void __launch_bounds__(512) k_blockScanWide(EncParams p) {
+    __shared__ u32 scratch[40];
+    if (blockFailed(p)) return;
+    const u32 t = blockIdx.x;
+    const u32 off = p.tables[t].blockOff;
+    const u32 total = blockExclusiveScan8<512>(p.blockBits + off, p.blockOff + off, p.meta[t].blocks, scratch);
+    if (threadIdx.x == 0) p.meta[t].codeBits = total;
+}
+
 // Segment layout per stream (a thread per stream), then the exclusive scan
 // of the segments' words over the streams (k_layout, k_layoutCarry).
-__global__ void __launch_bounds__(256) k_layoutSegments(EncParams p) {
-    if (*reinterpret_cast<volatile const u32*>(p.errors)) return;   // no barriers in this kernel
-    const u32 s = blockIdx.x * 256u + threadIdx.x;
-    if (s >= p.S) return;
+__device__ __forceinline__ SegmentLayout segmentOf(const EncParams& p, u32 s) {
     SegmentLayout L{};
     const EncStreamDev sd = p.streams[s];
     const u32 offW = (blocksOf(p.counts[s], p.cbLog) + 1u) / 2u;
@@ -1009,7 +1034,29 @@ __global__ void __launch_bounds__(256) k_layoutSegments(EncParams p) {
     }
     L.words = words;
     L.bitLength = words * 32u;
-    p.layout[s] = L;
+    return L;
+}
+
+__global__ void __launch_bounds__(256) k_layoutSegments(EncParams p) {
+    if (*reinterpret_cast<volatile const u32*>(p.errors)) return;   // no barriers in this kernel
+    const u32 s = blockIdx.x * 256u + threadIdx.x;
+    if (s < p.S) p.layout[s] = segmentOf(p, s);
+}
+
+// Both steps of a call of at most 1024 streams.
+__global__ void __launch_bounds__(1024) k_layoutOne(EncParams p) {
+    __shared__ u32 scratch[40];
+    if (blockFailed(p)) return;
+    const u32 s = threadIdx.x;
+    SegmentLayout L{};
+    if (s < p.S) L = segmentOf(p, s);
+    u32 tot;
+    L.startWord = blockExclusiveSum<1024>(L.words, scratch, &tot);
+    if (s < p.S) p.layout[s] = L;
+    if (threadIdx.x == 0) {
+        p.totals[0] = tot;
+        if (tot > p.outWordsMax) atomicOr(p.errors, DEV_ERR_OUTPUT_CAPACITY);
+    }
 }
 
 // CTA b scans the segment words of streams 1024 b .. 1024 b + 1023; with more
@@ -1083,16 +1130,25 @@ __device__ __forceinline__ void orCodeword(u32* win, u32 wLo, u32 wHi, u32 pos, 
 // register until its bit offset is known.
 constexpr u32 kPackWindowWords = kRunSymbols * 31u / 32u + 2u;
 
+__device__ void writeHeaders(const EncParams& p, u32 s, u32 gt, u32 g);
+
+// The first headCtas CTAs write the streams' headers beside the packing, g
+// threads per stream.
 template <class Sym>
-__global__ void __launch_bounds__(kPackWarps * 32, 3) k_pack(EncParams p) {
+__global__ void __launch_bounds__(kPackWarps * 32, 3) k_pack(EncParams p, u32 headCtas, u32 g) {
     __shared__ u32 winAll[kPackWarps * kPackWindowWords];
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warpFailed(p)) return;
+    if (blockIdx.x < headCtas) {
+        const u32 s = (blockIdx.x * (kPackWarps * 32u) + threadIdx.x) / g;
+        if (s < p.S) writeHeaders(p, s, threadIdx.x & (g - 1u), g);
+        return;
+    }
     u32* win = winAll + warp * kPackWindowWords;
     const u32 runs = u32(p.totals[3]);
     const u32 bpr = kRunSymbols >> p.cbLog;
-    const u32 stride = gridDim.x * kPackWarps;
-    for (u32 r = blockIdx.x * kPackWarps + warp; r < runs; r += stride) {
+    const u32 stride = (gridDim.x - headCtas) * kPackWarps;
+    for (u32 r = (blockIdx.x - headCtas) * kPackWarps + warp; r < runs; r += stride) {
         const u32 t = p.runTable[r];
         const TableMeta m = p.meta[t];
         const EncTableDev td = p.tables[t];
@@ -1179,14 +1235,11 @@ __global__ void __launch_bounds__(kPackWarps * 32, 3) k_pack(EncParams p) {
     }
 }
 
-// Count words, table headers, codeword bit counts and offset increments.  A
-// group of g threads (a power of two, 32 .. 512) writes one stream: a call of
-// many streams packs 512 / g of them into a CTA instead of one (as many as
-// still leave four CTAs per SM).
-__global__ void __launch_bounds__(512) k_headers(EncParams p, u32 g) {
-    if (blockFailed(p)) return;
-    const u32 s = blockIdx.x * (blockDim.x / g) + threadIdx.x / g, gt = threadIdx.x & (g - 1u);
-    if (s >= p.S) return;   // no barriers below
+// Count words, table headers, codeword bit counts and offset increments of
+// stream s, by g threads (a power of two, 32 .. 256; this one gt): a call of
+// many streams packs several into a CTA (as many as still leave four CTAs per
+// SM).
+__device__ void writeHeaders(const EncParams& p, u32 s, u32 gt, u32 g) {
     const EncStreamDev sd = p.streams[s];
     const SegmentLayout L = p.layout[s];
     u32* seg = p.out + L.startWord;
@@ -1298,23 +1351,26 @@ int encodePrepare(cc_instance* I, const EncStream* streams, u32 S, char* slot, s
 template <class Sym>
 static int launchEncode(cc_instance* I, const EncParams& p) {
     cudaStream_t st = I->stream;
-    CC_TRY_CUDA(cudaMemsetAsync(I->errors, 0, 4 * sizeof(u32), st), "memset errors");
-    CC_TRY_CUDA(cudaMemsetAsync(I->streamMax, 0, sizeof(u32) * p.S, st), "memset stream max");
-    if (p.S) { k_lookupMaps<<<p.S, 256, 0, st>>>(p); countLaunch(); }
+    k_encBegin<<<p.S, 256, 0, st>>>(p);   // S > 0: encodeDevice returns early, a batch has volumes
+    countLaunch();
     if (p.totalTiles) { SectionTimer t(I, "enc.summary", st); k_summary<Sym><<<p.totalTiles, kRleThreads, 0, st>>>(p); countLaunch(); }
-    {
-        SectionTimer t(I, "enc.rle_scan", st);
-        k_scan<<<u32(ceilDiv(p.S, kScanWarps)), kScanWarps * 32, 0, st>>>(p);
-        countLaunch();
-    }
-    {
+    const u32 chunks = std::max<u32>(1, u32(ceilDiv(p.T, kPlanChunk)));
+    if (p.S <= kScanPlanStreams) {   // then one chunk
         SectionTimer t(I, "enc.hist_plan", st);
-        const u32 chunks = std::max<u32>(1, u32(ceilDiv(p.T, kPlanChunk)));
+        k_scanPlan<<<1, 1024, 0, st>>>(p);
+        countLaunch();
+    } else {
+        {
+            SectionTimer t(I, "enc.rle_scan", st);
+            k_scan<<<u32(ceilDiv(p.S, kScanWarps)), kScanWarps * 32, 0, st>>>(p);
+            countLaunch();
+        }
+        SectionTimer t(I, "enc.hist_plan", st);
         k_histPlan<<<chunks, 1024, 0, st>>>(p);
         countLaunch();
         if (chunks > 1) { k_histPlanCarry<<<chunks - 1, 1024, 0, st>>>(p); countLaunch(); }
     }
-    { SectionTimer t(I, "enc.hist_zero", st); k_zeroHist<<<2 * 148, 256, 0, st>>>(p); countLaunch(); }
+    { SectionTimer t(I, "enc.hist_zero", st); k_planFill<<<2 * 148, 256, 0, st>>>(p); countLaunch(); }
     if (p.totalTiles) {
         CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_write<Sym>),
                                         sizeof(Sym) == 2 ? kAttrWrite16 : kAttrWrite32, I->device, writeSmem<Sym>()),
@@ -1330,7 +1386,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
     const bool solo = I->tableBuildSoloSM && p.T <= sms;
     size_t buildSmem = hm::Layout<kBuildSmemLeaves>::kBytes;
     if (solo) buildSmem = std::max(buildSmem, tableBuildSoloSmem(I->device));
-    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, kBuildSmemLeaves>),
+    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBigThreads, kBuildSmemLeaves>),
                                     kAttrTableBuild, I->device, buildSmem),
                 "tableBuild smem");
     {
@@ -1367,16 +1423,16 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
                     EncParams big = q;
                     big.buildTier = 3;
                     big.buildLo = kBuildSplitLeaves + 1;
-                    k_tableBuild<kBuildThreads, kBuildSmemLeaves>
-                        <<<std::min(p.T, sms), kBuildThreads, buildSmem, I->buildSide>>>(big);
+                    k_tableBuild<kBigThreads, kBuildSmemLeaves>
+                        <<<std::min(p.T, sms), kBigThreads, buildSmem, I->buildSide>>>(big);
                     countLaunch();
                 }
                 EncParams mid = q;
                 mid.buildTier = 2;
                 mid.buildLo = kSmallLeaves + 1;
                 mid.buildHi = kBuildSplitLeaves;
-                k_tableBuild<kBuildThreads, kBuildSplitLeaves>
-                    <<<std::min(p.T, 5u * sms), kBuildThreads, hm::Layout<kBuildSplitLeaves>::kBytes, I->buildSide>>>(mid);
+                k_tableBuild<kMidThreads, kBuildSplitLeaves>
+                    <<<std::min(p.T, 5u * sms), kMidThreads, hm::Layout<kBuildSplitLeaves>::kBytes, I->buildSide>>>(mid);
                 countLaunch();
                 CC_TRY_CUDA(cudaEventRecord(I->buildJoin, I->buildSide), "table build join");
             }
@@ -1396,13 +1452,11 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
                 k_tableBuild<kBuildThreads, kBuildSplitLeaves>
                     <<<p.T, kBuildThreads, hm::Layout<kBuildSplitLeaves>::kBytes, st>>>(q);
             else
-                k_tableBuild<kBuildThreads, kBuildSmemLeaves><<<p.T, kBuildThreads, buildSmem, st>>>(q);
+                k_tableBuild<kBigThreads, kBuildSmemLeaves><<<p.T, kBigThreads, buildSmem, st>>>(q);
             countLaunch();
         }
     }
-    // used-block list (after the plan, k_histPlan); the block kernels walk it
-    // with a grid of a few CTAs per SM
-    if (p.totalBlocks && p.T) { k_usedBlocks<<<u32(ceilDiv(p.T, 8)), 256, 0, st>>>(p); countLaunch(); }
+    // the block kernels walk the run list (k_planFill) with a few CTAs per SM
     const u32 blockGrid = u32(std::max(1, I->smCount > 0 ? I->smCount : 148)) * 8u;
     // runs of the call: at most the used blocks / blocks per run, plus one per table
     const u32 runBound = u32(ceilDiv(p.totalBlocks, kRunSymbols / p.cb)) + p.T;
@@ -1411,33 +1465,32 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         { SectionTimer t(I, "enc.block_bits", st); k_blockBits<Sym><<<g, kPackWarps * 32, 0, st>>>(p); countLaunch(); }
         {
             SectionTimer t(I, "enc.block_scan", st);
-            k_blockScan<<<u32(ceilDiv(p.T, kScanWarps)), kScanWarps * 32, 0, st>>>(p);
+            if (p.T <= kWideScanTables) k_blockScanWide<<<p.T, 512, 0, st>>>(p);
+            else k_blockScan<<<u32(ceilDiv(p.T, kScanWarps)), kScanWarps * 32, 0, st>>>(p);
             countLaunch();
         }
     }
     {
         SectionTimer t(I, "enc.layout", st);
-        k_layoutSegments<<<u32(ceilDiv(p.S, 256)), 256, 0, st>>>(p);
-        countLaunch();
-        const u32 chunks = std::max<u32>(1, u32(ceilDiv(p.S, 1024)));
-        k_layout<<<chunks, 1024, 0, st>>>(p);
-        countLaunch();
-        if (chunks > 1) { k_layoutCarry<<<chunks - 1, 1024, 0, st>>>(p); countLaunch(); }
-    }
-    if (p.totalBlocks) {
-        const u32 g = std::min<u32>(blockGrid, u32(ceilDiv(runBound, kPackWarps)));
-        SectionTimer t(I, "enc.pack", st);
-        k_pack<Sym><<<g, kPackWarps * 32, 0, st>>>(p);
-        countLaunch();
+        if (p.S <= 1024) {
+            k_layoutOne<<<1, 1024, 0, st>>>(p);
+            countLaunch();
+        } else {
+            k_layoutSegments<<<u32(ceilDiv(p.S, 256)), 256, 0, st>>>(p);
+            const u32 chunks = u32(ceilDiv(p.S, 1024));
+            k_layout<<<chunks, 1024, 0, st>>>(p);
+            k_layoutCarry<<<chunks - 1, 1024, 0, st>>>(p);
+            countLaunch(3);
+        }
     }
     {
-        SectionTimer t(I, "enc.headers", st);
+        SectionTimer t(I, "enc.pack", st);
+        const u32 packCtas = p.totalBlocks ? std::min<u32>(blockGrid, u32(ceilDiv(runBound, kPackWarps))) : 0u;
         // streams per CTA: as few as keep four CTAs per SM busy
-        const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
         u32 per = 1;
-        while (per < 16 && u64(2 * per) * 4 * sms <= p.S) per <<= 1;
-        const u32 g = 512 / per;
-        k_headers<<<u32(ceilDiv(p.S, per)), 512, 0, st>>>(p, g);
+        while (per < 8 && u64(2 * per) * 4 * sms <= p.S) per <<= 1;
+        const u32 headCtas = u32(ceilDiv(p.S, per));
+        k_pack<Sym><<<headCtas + packCtas, kPackWarps * 32, 0, st>>>(p, headCtas, kPackWarps * 32 / per);
         countLaunch();
     }
     CC_TRY_CUDA(cudaGetLastError(), "encode launch");
@@ -1449,7 +1502,7 @@ int prepareDecodeAttributes(cc_instance* I);
 int prepareKernelAttributes(cc_instance* I) {
     size_t buildSmem = hm::Layout<kBuildSmemLeaves>::kBytes;
     if (I->tableBuildSoloSM) buildSmem = std::max(buildSmem, tableBuildSoloSmem(I->device));
-    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBuildThreads, kBuildSmemLeaves>),
+    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBigThreads, kBuildSmemLeaves>),
                                     kAttrTableBuild, I->device, buildSmem),
                 "tableBuild smem");
     if (I->symBytes == 2)
@@ -1495,7 +1548,6 @@ int encodeLaunch(cc_instance* I, const EncPlan& hp, u32* out, u64 outCap) {
     p.headers = I->headers;
     p.blockBits = I->blockBits;
     p.blockOff = I->blockOff;
-    p.blockTable = I->blockTable;
     p.runTable = I->runTable;
     p.tileStream = I->tileStream;
     p.layout = I->layout;

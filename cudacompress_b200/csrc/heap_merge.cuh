@@ -22,14 +22,16 @@
 //    the first sibling below it that became the smaller child, else the path
 //    itself: for the root that is one minimum over the lanes' (level, tail).
 //
-// Measured on B200 (cycles per merge, one table alone on an SM): 390 at every
+// Measured on B200 (cycles per merge, one table alone on an SM): 350 at every
 // size, where a one-thread replay took 1374 at 406 leaves, 1643 at 2012 and
 // 1883 at 8192.  What bounds it is one warp's chain of minimum over the lanes
 // (24 cycles), pair loads (30 and up), clamp and compare, three times per
-// merge, and the issue of some fifty instructions beside each.  Tried: 16-bit
-// ids and tails with comparisons instead of kInf nodes 457; nodes of 8 bytes,
-// whose pair is one 16-byte load, 574; tails stored before the next
-// operation's loads 619.
+// merge, and in-order issue: whatever the next operation does not wait for -
+// ids, tails, parents - is stored after the minimum is under way.  Tried:
+// these stores before it 390; the new tail at the parting of two paths by a
+// second minimum instead of in its lane 399; 16-bit ids and tails with
+// comparisons instead of kInf nodes 457; nodes of 8 bytes, whose pair is one
+// 16-byte load, 574; tails stored before the next operation's loads 619.
 //
 // Shared layout, nodes 1-based (node k's children are 2k and 2k + 1), words:
 // the probabilities (a pair of children is one 8-byte load), the ids, the
@@ -100,9 +102,14 @@ struct Merge {
     // tail, the lane's key and the path's end; the winners' ballot, and the
     // tails on their way to their array.
     struct Path {
-        U node4, sibTail, key, none, from, newTail;
+        U node4, sibTail, key, newTail;
         B holds, win;
         u32 tail4, winners;
+    };
+    // An operation's moves: where, which id, whether.
+    struct Store {
+        U at4, id;
+        B moved;
     };
     U rootP, rootId;   // the root's element, in its lane
 
@@ -148,82 +155,81 @@ struct Merge {
         l.tail4 = key & kKeyTail;
     }
 
-    // The moves of a pop that leaves n elements.  fwdLevel / fwdTail4: the
-    // tail of the node at which this path and the previous operation's part
-    // (not stored yet); prev: that operation, whose tails are stored here.
-    CC_HD void popMove(const Loads& l, u32 n, u32 fwdLevel, u32 fwdTail4, const Path& prev, Path& p) {
+    // The moves of a pop that leaves n elements.  prev: the previous
+    // operation, whose tails are stored here; parting: the level at which this
+    // path leaves its path (the sibling there is its node, with a new tail).
+    CC_HD void popMove(const Loads& l, u32 n, u32 parting, const Path& prev, Path& p, Store& o) {
         const U v = w.all(l.v);
         const U x = w.min(l.px, l.py);
         const U y = w.max(x, w.min3(v, l.nx, l.ny));
         const B isLeft = w.lt(l.px, l.py);
-        const U kk4 = w.sel(isLeft, l.pair4, w.add(l.pair4, w.all(4u)));
-        const B moved = w.le(x, v);
-        const U id = w.sel(w.le(w.min(l.nx, l.ny), v), w.sel(w.lt(l.nx, l.ny), l.ix, l.iy), w.all(l.idv));
+        o.at4 = w.sel(isLeft, l.pair4, w.add(l.pair4, w.all(4u)));
+        o.moved = w.le(x, v);
         w.fence();
-        w.template st<0>(kk4, y, moved);
-        w.template st<At::kIds>(kk4, id, moved);
+        w.template st<0>(o.at4, y, o.moved);
+        rootP = y;
+        // the sibling wins a left node's place on a tie too
+        finish(l, n, y, w.sel(isLeft, w.below(l.py), l.px), parting, prev, p);
+        o.id = w.sel(w.le(w.min(l.nx, l.ny), v), w.sel(w.lt(l.nx, l.ny), l.ix, l.iy), w.all(l.idv));
+    }
+    // The ids of an operation's moves, and the tails of the one before.
+    CC_HD void storeIds(const Store& o, const Path& prev) {
+        w.template st<At::kIds>(o.at4, o.id, o.moved);
         tailsStore(prev);
         w.fence();
-        rootP = y;
-        rootId = id;
-        // the sibling wins a left node's place on a tie too
-        finish(l, n, y, w.sel(isLeft, w.below(l.py), l.px), fwdLevel, fwdTail4, p);
     }
 
-    CC_HD void finish(const Loads& l, u32 n, const U& y, const U& s, u32 fwdLevel, u32 fwdTail4, Path& p) {
-        p.sibTail = w.sel(w.eq(level, w.all(fwdLevel)), w.all(fwdTail4), l.sibTail);
+    CC_HD void finish(const Loads& l, u32 n, const U& y, const U& s, u32 parting, const Path& prev, Path& p) {
+        p.sibTail = w.sel(w.eq(level, w.all(parting)), prev.newTail, l.sibTail);
         p.win = w.lt(s, y);
-        p.none = w.all(kNoKey | l.tail4);
-        p.key = w.sel(p.win, w.orv(levelKey, p.sibTail), p.none);
+        p.key = w.sel(p.win, w.orv(levelKey, p.sibTail), w.all(kNoKey | l.tail4));
         p.node4 = l.node4;
         p.holds = w.le(l.node4, w.all(4u * n));
         p.tail4 = l.tail4;
     }
 
-    // Loads of a push whose path ends in tail4 / 4.
-    CC_HD void pushLoads(Loads& l, u32 tail4) {
+    // Loads of a push whose path ends in tail4 / 4: the probabilities, and once
+    // the pop's ids and tails are stored, the rest.
+    CC_HD void pushValues(Loads& l, u32 tail4) {
         const U t = w.shr(w.all(tail4), sh);
         l.node4 = w.andv(t, nodeMask);
-        const U up4 = w.shr(l.pair4 = w.andv(t, pairMask), 1u);
+        l.pair4 = w.andv(t, pairMask);
         w.template ldPair<0>(w.orv(l.pair4, none), l.px, l.py);
-        l.nx = w.template ld<0>(up4);
-        l.ix = w.template ld<At::kIds>(up4);
-        l.sibTail = w.template ld<At::kTails>(w.xorv(l.node4, w.all(4u)));
+        l.nx = w.template ld<0>(w.shr(l.pair4, 1u));
         l.tail4 = tail4;
+    }
+    CC_HD void pushRest(Loads& l) {
+        l.ix = w.template ld<At::kIds>(w.shr(l.pair4, 1u));
+        l.sibTail = w.template ld<At::kTails>(w.xorv(l.node4, w.all(4u)));
     }
 
     // The moves of a push of c at position q.
-    CC_HD void pushMove(const Loads& l, u32 q, u32 c, u32 id, u32 fwdLevel, u32 fwdTail4, const Path& prev, Path& p) {
+    CC_HD void pushMove(const Loads& l, u32 q, u32 c, u32 id, u32 parting, const Path& prev, Path& p, Store& o) {
         const B odd = w.nz(w.andv(l.node4, w.all(4u)));
         const U e = w.sel(odd, l.py, l.px);
         const U up = w.andv(l.nx, upMask);
         const U cv = w.all(c);
         const U y = w.max(up, w.min(cv, e));
-        const B moved = w.both(w.le(w.orv(l.node4, none), w.all(4u * q)), w.lt(cv, e));
-        const U newId = w.sel(w.lt(cv, up), l.ix, w.all(id));
+        o.at4 = l.node4;
+        o.moved = w.both(w.le(w.orv(l.node4, none), w.all(4u * q)), w.lt(cv, e));
         w.fence();
-        w.template st<0>(l.node4, y, moved);
-        w.template st<At::kIds>(l.node4, newId, moved);
-        tailsStore(prev);
-        w.fence();
+        w.template st<0>(o.at4, y, o.moved);
         rootP = y;
-        rootId = w.sel(moved, newId, rootId);
-        finish(l, q, y, w.sel(odd, l.px, w.below(l.py)), fwdLevel, fwdTail4, p);
+        finish(l, q, y, w.sel(odd, l.px, w.below(l.py)), parting, prev, p);
+        o.id = w.sel(w.lt(cv, up), l.ix, w.all(id));
     }
 
     // Tails of an operation's path nodes, while the next operation waits for
     // its loads: the nearest winning sibling below each node, and its tail
     // (else the path's end).
     CC_HD void tailsFind(Path& p) {
-        p.from = w.andv(w.all(p.winners), deeper);
-        p.newTail = w.shfl(p.sibTail, w.lastSet(p.from));
+        const U from = w.andv(w.all(p.winners), deeper);
+        const U t = w.shfl(p.sibTail, w.lastSet(from));
+        p.newTail = w.sel(w.nz(from), t, w.all(p.tail4));
     }
     CC_HD void tailsStore(const Path& p) {
-        w.template st<At::kTails>(p.node4, w.sel(w.nz(p.from), p.newTail, w.all(p.tail4)), p.holds);
+        w.template st<At::kTails>(p.node4, p.newTail, p.holds);
     }
-    // The minimum over the keys after r.
-    CC_HD u32 keyAfter(u32 r, const Path& p) { return w.reduceMin(w.sel(w.lt(w.all(r), p.key), p.key, p.none)); }
-
     // Merges the heap of L >= 2 elements (the arrays set up: ids and tails of
     // nodes 1 .. L, kInf at the others of the full tree and at kNone); writes
     // the parent of every id but the root's (2L - 2).
@@ -235,14 +241,14 @@ struct Merge {
         pc.sibTail = w.all(0u);
         pc.holds = w.lt(w.all(1u), w.all(0u));
         pc.winners = 0;
-        pc.none = w.all(kNoKey | pc.tail4);
-        pc.key = pc.none;
+        pc.newTail = w.all(pc.tail4);
         rootP = w.all(w.template ldOne<0>(4u));
         rootId = w.all(w.template ldOne<At::kIds>(4u));
         u32 rc = kNoKey | pc.tail4;
         u32 next = L;
         u32 qDepth = D;   // depth of the push's position
         Loads l;
+        Store o;
         takeLast(l, L - 1);
         for (u32 len = L; len > 1; --len, ++next) {
             const u32 q = len - 1;
@@ -250,33 +256,38 @@ struct Merge {
             const u32 tailC = 4u * q << (D - qDepth);
 
             popLoads(l, rc);
-            const u32 rc2 = keyAfter(rc, pc);
             tailsFind(pc);
             w.template stParent<At::kParents>(rootId, next);
             U c = rootP;
-            popMove(l, len - 1, rc >> kKeyLevel, rc2 & kKeyTail, pc, pa);
-            takeLast(l, len - 2);
+            popMove(l, len - 1, rc >> kKeyLevel, pc, pa, o);
             const u32 ra = w.reduceMin(pa.key);
+            rootId = o.id;
+            storeIds(o, pc);
+            takeLast(l, len - 2);
             pa.winners = w.ballot(pa.win);
 
             popLoads(l, ra);
-            const u32 ra2 = keyAfter(ra, pa);
+            tailsFind(pa);
             w.template stParent<At::kParents>(rootId, next);
             c = w.shfl(w.add(c, rootP), w.all(31u));
-            tailsFind(pa);
             // the level at which the push's path leaves this pop's
             const u32 diff = (tailC ^ l.tail4) >> 2;
             const u32 h = diff ? D - log2Floor(diff) : 0x7Eu;
-            popMove(l, len - 2, ra >> kKeyLevel, ra2 & kKeyTail, pa, pb);
+            popMove(l, len - 2, ra >> kKeyLevel, pa, pb, o);
+            w.fence();
 
-            pushLoads(l, tailC);
+            pushValues(l, tailC);
             pb.winners = w.ballot(pb.win);
-            const u32 rb2 = keyAfter((h << kKeyLevel) | kKeyTail, pb);
+            rootId = o.id;
+            storeIds(o, pa);
+            pushRest(l);
             tailsFind(pb);
-            pushMove(l, q, w.first(c), 2u * next, h, rb2 & kKeyTail, pb, pc);
-            takeLast(l, len - 2);
+            pushMove(l, q, w.first(c), 2u * next, h, pb, pc, o);
             rc = w.reduceMin(pc.key);
             pc.winners = w.ballot(pc.win);
+            rootId = w.sel(o.moved, o.id, rootId);
+            storeIds(o, pb);
+            takeLast(l, len - 2);
         }
     }
 };
@@ -329,19 +340,20 @@ struct DeviceWarp {
     template <u32 kArray>
     __device__ __forceinline__ u32 ldOne(u32 off) const { return ld<kArray>(off); }
     // Predicated stores are written out: as conditional statements they became
-    // branches (541 instead of 390 cycles per merge).
+    // branches (541 instead of 390 cycles per merge then).
     __device__ __forceinline__ static u32 window() { return u32(__cvta_generic_to_shared(mem())); }
     template <u32 kArray>
     __device__ __forceinline__ void st(u32 off, u32 v, bool c) const {
-        asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.u32 [%0], %1;\n}"
-                     :: "r"(window() + kArray + off), "r"(v), "r"(u32(c)) : "memory");
+        asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.u32 [%0 + %3], %1;\n}"
+                     :: "r"(window() + off), "r"(v), "r"(u32(c)), "n"(kArray) : "memory");
     }
     template <u32 kArray>
     __device__ __forceinline__ void stAll(u32 off, u32 v) const { *reinterpret_cast<u32*>(mem() + kArray + off) = v; }
     // by the root's lane; id2: the id x 2
     template <u32 kArray>
     __device__ __forceinline__ void stParent(u32 id2, u32 v) const {
-        if (lane() == 31u) *reinterpret_cast<u16*>(mem() + kArray + id2) = u16(v);
+        asm volatile("{\n.reg .pred p;\nsetp.eq.u32 p, %2, 31;\n@p st.shared.u16 [%0 + %3], %1;\n}"
+                     :: "r"(window() + id2), "h"(u16(v)), "r"(lane()), "n"(kArray) : "memory");
     }
 };
 #endif

@@ -155,7 +155,6 @@ void layoutArena(cc_instance* I, char* base, size_t* total) {
     I->headers = c.take<u32>(I->capHdr);
     I->blockBits = c.take<u32>(I->capBlocks + 1);
     I->blockOff = c.take<u32>(I->capBlocks + 1);
-    I->blockTable = c.take<u32>(I->capBlocks + 1);
     I->runTable = c.take<u32>(I->capBlocks + 1);
     I->tileStream = c.take<u32>(I->capTiles + 1);
     I->layout = c.take<SegmentLayout>(I->capStreams);

@@ -112,19 +112,34 @@ __device__ int warpPartition(u32* a, int f, int l, u16* lList, u16* rList) {
     const u32 ltMask = (1u << lane) - 1u;
     const u32 p = keyOf(a[f]);
     int nL = 0, nR = 0;
-    for (int base = f + 1; base < l; base += 32) {
-        const int j = base + int(lane);
-        const bool pred = j < l && !(keyOf(a[j]) < p);
-        const u32 m = __ballot_sync(0xffffffffu, pred);
-        if (pred) lList[f + nL + __popc(m & ltMask)] = u16(j);
-        nL += __popc(m);
+    // four groups of 32 per step, their loads in flight together
+    for (int base = f + 1; base < l; base += 128) {
+        bool pred[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = base + 32 * q + int(lane);
+            pred[q] = j < l && !(keyOf(a[min(j, l - 1)]) < p);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const u32 m = __ballot_sync(0xffffffffu, pred[q]);
+            if (pred[q]) lList[f + nL + __popc(m & ltMask)] = u16(base + 32 * q + int(lane));
+            nL += __popc(m);
+        }
     }
-    for (int top = l - 1; top > f; top -= 32) {
-        const int j = top - int(lane);
-        const bool pred = j > f && !(p < keyOf(a[j]));
-        const u32 m = __ballot_sync(0xffffffffu, pred);
-        if (pred) rList[f + nR + __popc(m & ltMask)] = u16(j);
-        nR += __popc(m);
+    for (int top = l - 1; top > f; top -= 128) {
+        bool pred[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = top - 32 * q - int(lane);
+            pred[q] = j > f && !(p < keyOf(a[max(j, f)]));
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const u32 m = __ballot_sync(0xffffffffu, pred[q]);
+            if (pred[q]) rList[f + nR + __popc(m & ltMask)] = u16(top - 32 * q - int(lane));
+            nR += __popc(m);
+        }
     }
     __syncwarp();
     // K = number of leading k with lList[k] < rList[k] (monotone in k)
