@@ -88,53 +88,86 @@ __device__ __forceinline__ const Sym* tableInput(const EncParams& p, const EncTa
 
 // Run-length tiles: kRleWarps warps x 32 groups x 32 symbols.  Warp w
 // covers symbols [w * 1024, (w + 1) * 1024) of the tile; group k of it is 32
-// consecutive symbols, symbol k * 32 + i held by lane i.  A ballot gives a
-// group's nonzero mask, kept by lane k, so a warp describes its 1024
-// symbols with one mask per lane and the run-length bookkeeping is warp
-// scans over the groups.  Positions are kept +1 so that 0 means "no
-// nonzero".
+// consecutive symbols, lane k's.  They pass through shared memory, a padded
+// row per group, so that global memory is read 16 bytes per lane and a lane
+// has its own symbols at hand: a nonzero mask per lane describes the warp's
+// 1024 symbols, and the run-length bookkeeping is warp scans over the groups.
+// Positions are kept +1 so that 0 means "no nonzero".
 constexpr u32 kRleWarps = kRleThreads / 32;
+constexpr u32 kRlePitch = 36;   // elements per row: a lane's 8 (16-bit: 16 bytes of 4) are free of conflicts
 static_assert(kRleTile == kRleWarps * 1024, "a tile is 32 groups of 32 symbols per warp");
-
-template <class Sym>
-struct WarpSyms {
-    u32 x[16];      // this lane's symbol of groups 2j (low half) and 2j + 1 (high half); u16 symbols
-    u32 y[32];      // 32-bit symbols (Sym = u32)
-    __device__ __forceinline__ u32 at(u32 k) const {   // k a compile-time constant after unrolling
-        return sizeof(Sym) == 2 ? (x[k >> 1] >> (16 * (k & 1))) & 0xFFFFu : y[k];
-    }
-};
 
 // Group data of lane k of the calling warp (its group k).
 struct GroupRuns {
     u32 mask, cnt, firstP1, lastP1;
 };
 
+__device__ __forceinline__ void putRow(u16* row, uint4 v) {   // 8-byte aligned
+    reinterpret_cast<uint2*>(row)[0] = make_uint2(v.x, v.y);
+    reinterpret_cast<uint2*>(row)[1] = make_uint2(v.z, v.w);
+}
+__device__ __forceinline__ void putRow(u32* row, uint4 v) { *reinterpret_cast<uint4*>(row) = v; }
+
 // Loads the warp's 1024 symbols from stream position wbase (zero beyond n)
-// and returns lane k's group k mask data; maxSym receives the warp's largest
-// symbol.
+// into its rows and returns lane k's group k mask data; maxSym receives the
+// warp's largest symbol.
 template <class Sym>
-__device__ __forceinline__ GroupRuns loadGroups(const Sym* in, u32 wbase, u32 n, WarpSyms<Sym>& v, u32& maxSym) {
+__device__ __forceinline__ GroupRuns loadGroups(const Sym* in, u32 wbase, u32 n, Sym* rows, u32& maxSym) {
+    constexpr u32 kVec = 16 / sizeof(Sym), kParts = 32 / kVec;   // elements per access, accesses per group
     const u32 lane = threadIdx.x & 31u;
+    maxSym = 0;
+    if (wbase >= n) return GroupRuns{0u, 0u, 0u, 0u};   // warp-uniform
+    if ((reinterpret_cast<uintptr_t>(in + wbase) & 15u) == 0) {
+        uint4 v[kParts];
 #pragma unroll
-    for (u32 k = 0; k < 32; ++k) {
-        const u32 pos = wbase + 32u * k + lane;
-        const u32 x = pos < n ? u32(in[pos]) : 0u;
-        if (sizeof(Sym) == 2) {
-            if (k & 1) v.x[k >> 1] |= x << 16;
-            else v.x[k >> 1] = x;
-        } else {
-            v.y[k] = x;
+        for (u32 k = 0; k < kParts; ++k) {
+            const u32 at = wbase + (k * 32u + lane) * kVec;
+            v[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (at + kVec <= n) {
+                v[k] = *reinterpret_cast<const uint4*>(in + at);
+            } else if (at < n) {
+                u32 x[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (u32 q = 0; q < kVec; ++q)
+                    if (at + q < n) x[q * sizeof(Sym) / 4] |= u32(in[at + q]) << (sizeof(Sym) == 2 ? 16 * (q & 1) : 0);
+                v[k] = make_uint4(x[0], x[1], x[2], x[3]);
+            }
+        }
+#pragma unroll
+        for (u32 k = 0; k < kParts; ++k) {
+            const u32 c = k * 32u + lane;
+            putRow(rows + (c / kParts) * kRlePitch + (c % kParts) * kVec, v[k]);
+        }
+    } else {
+#pragma unroll 8
+        for (u32 k = 0; k < 32; ++k) {
+            const u32 pos = wbase + 32u * k + lane;
+            rows[k * kRlePitch + lane] = pos < n ? in[pos] : Sym(0);
         }
     }
+    __syncwarp();
     GroupRuns g{0u, 0u, 0u, 0u};
+    const Sym* row = rows + lane * kRlePitch;
     u32 m = 0;
+    if (sizeof(Sym) == 2) {
 #pragma unroll
-    for (u32 k = 0; k < 32; ++k) {
-        const u32 x = v.at(k);
-        m = max(m, x);
-        const u32 b = __ballot_sync(0xffffffffu, x != 0u);
-        if (lane == k) g.mask = b;
+        for (u32 k = 0; k < 8; ++k) {
+            const uint2 x = *reinterpret_cast<const uint2*>(row + 4 * k);
+            m = __vmaxu2(m, __vmaxu2(x.x, x.y));
+            // bit 15 / 31 of each: that half is not zero
+            const u32 a = (((x.x & 0x7FFF7FFFu) + 0x7FFF7FFFu) | x.x) & 0x80008000u;
+            const u32 b = (((x.y & 0x7FFF7FFFu) + 0x7FFF7FFFu) | x.y) & 0x80008000u;
+            const u32 ab = (a >> 15) | (b >> 13);   // bits 0, 16 and 2, 18
+            g.mask |= ((ab | (ab >> 15)) & 15u) << (4 * k);
+        }
+        m = max(m & 0xFFFFu, m >> 16);
+    } else {
+#pragma unroll
+        for (u32 k = 0; k < 8; ++k) {
+            const uint4 x = *reinterpret_cast<const uint4*>(row + 4 * k);
+            m = max(max(m, max(x.x, x.y)), max(x.z, x.w));
+            g.mask |= ((x.x ? 1u : 0u) | (x.y ? 2u : 0u) | (x.z ? 4u : 0u) | (x.w ? 8u : 0u)) << (4 * k);
+        }
     }
     maxSym = __reduce_max_sync(0xffffffffu, m);
     const u32 gb = wbase + 32u * lane;
@@ -198,6 +231,7 @@ template <class Sym>
 __global__ void __launch_bounds__(kRleThreads) k_summary(EncParams p) {
     __shared__ RunSum sRun[kRleWarps];
     __shared__ u32 sStream, sMaxSym;
+    __shared__ __align__(16) Sym sRows[kRleWarps][32 * kRlePitch];
     const u32 tile = blockIdx.x;
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) { sStream = streamOfTile(p, tile); sMaxSym = 0; }
@@ -207,9 +241,8 @@ __global__ void __launch_bounds__(kRleThreads) k_summary(EncParams p) {
     const u32 n = sd.n;
     const Sym* in = reinterpret_cast<const Sym*>(sd.in);
     const u32 wbase = (tile - sd.tileOff) * kRleTile + warp * 1024u;
-    WarpSyms<Sym> v;
     u32 m;
-    const GroupRuns g = loadGroups(in, wbase, n, v, m);
+    const GroupRuns g = loadGroups(in, wbase, n, sRows[warp], m);
     if (lane == 0 && m) atomicMax(&sMaxSym, m);
     if (sd.kind == KIND_RLHUFF) {
         // the warp's summary: (0, 255) entries of the gaps whose previous
@@ -475,36 +508,43 @@ __global__ void __launch_bounds__(256) k_leafTiers(EncParams p) {
 // RLHuff: a tile's run-length entries form one contiguous range of the
 // stream's compact arrays.  Group k of a warp starts its entries after the
 // entries of the tile's groups before it (a warp scan of the groups' counts
-// plus their (0, 255) entries, and a block combine over the warps); inside a
-// group a nonzero's rank is the popcount of the mask below its lane, and its
-// zero count the distance to the set bit below it (or to the nonzero before
-// the group).  Entries are staged in shared memory at their positions within
-// the tile, then copied out with consecutive threads on consecutive entries.
-// Both histograms are counted over the staged entries: the eight most
-// frequent keys of each (zero counts 0..7, symbols 1..8) in per-lane
-// counters, the others with shared-memory atomics.  The stage (dynamic
-// shared memory) holds a whole tile's entries for 16-bit symbols - up to one
-// per symbol, plus the (0, 255) entries of zero runs inside the tile - so
-// only a tile that a zero run of millions of symbols ends in writes its
-// entries directly (and counts them with warp-aggregated atomics).
-constexpr u32 kWriteSymBins = 4096;   // symbol bins counted in shared memory by k_write
+// plus their (0, 255) entries, and a block combine over the warps); its lane
+// then walks its nonzeros, the distance to the one before being the zero
+// count.  Entries are staged in shared memory at their positions within the
+// tile, shifted so that 16-byte chunks there are 16-byte chunks of the compact
+// arrays, and copied out by them.  The eight most frequent keys of each
+// histogram (zero counts 0..7, symbols 1..8) are counted in the lane's
+// registers on the way, the others with shared-memory atomics.  The stage
+// (dynamic shared memory) holds a whole tile's entries for 16-bit symbols - up
+// to one per symbol, plus the (0, 255) entries of zero runs inside the tile -
+// so only a tile that a zero run of millions of symbols ends in writes its
+// entries directly.  Bound: instruction issue; walking a group's nonzeros on
+// its lane instead of a group's lanes together took three 256^3 streams'
+// highpass bands (50 million symbols, 26 million entries) from 191 to 123 us.
+constexpr u32 kWriteSymBins = 2048;   // symbol bins counted in shared memory by k_write
 
 template <class Sym>
 constexpr u32 writeStage() { return sizeof(Sym) == 2 ? kRleTile + kRleTile / 256u : kRleTile / 2u; }
 template <class Sym>
-constexpr size_t writeSmem() { return 2 * sizeof(Sym) * size_t(writeStage<Sym>()); }
+constexpr u32 writeVec() { return 16 / sizeof(Sym); }   // elements of a 16-byte chunk
+// Staged symbols and zero counts (with room for the shift), and the warps' rows.
+template <class Sym>
+constexpr size_t writeSmem() {
+    return sizeof(Sym) * (2 * (size_t(writeStage<Sym>()) + writeVec<Sym>()) + size_t(kRleWarps) * 32 * kRlePitch);
+}
 
 template <class Sym>
 __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
-    constexpr u32 kStage = writeStage<Sym>();
+    constexpr u32 kStage = writeStage<Sym>(), kVec = writeVec<Sym>();
     extern __shared__ __align__(16) unsigned char dynWrite[];
     __shared__ u32 sLast[kRleWarps], sEnt[kRleWarps];
     __shared__ u32 hSym[kWriteSymBins];
     __shared__ u32 hZc[256];
     Sym* const sComp = reinterpret_cast<Sym*>(dynWrite);
-    Sym* const sZcs = sComp + kStage;
+    Sym* const sZcs = sComp + kStage + kVec;
     __shared__ u32 sStream;
     const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    Sym* const rows = sZcs + kStage + kVec + warp * (32 * kRlePitch);
     if (threadIdx.x == 0) sStream = streamOfTile(p, blockIdx.x);
     if (blockFailed(p)) return;   // synchronizes (sStream visible)
     const u32 tile = blockIdx.x;
@@ -517,19 +557,16 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
     hZc[threadIdx.x] = 0;
     const Sym* in = reinterpret_cast<const Sym*>(sd.in);
     const u32 wbase = (tile - sd.tileOff) * kRleTile + warp * 1024u;
-    WarpSyms<Sym> v;
     u32 mUnused;
-    const GroupRuns g = loadGroups(in, wbase, n, v, mUnused);
+    const GroupRuns g = loadGroups(in, wbase, n, rows, mUnused);
     u32* gSym = p.hist + mS.histOff;
     if (sd.kind != KIND_RLHUFF) {
         __syncthreads();
-#pragma unroll
         for (u32 k = 0; k < 32; ++k) {
-            const u32 x = v.at(k);
-            const bool valid = wbase + 32u * k + lane < n;
-            const bool toSmem = valid && x < smemBins;
-            aggregatedIncrement(hSym, toSmem ? x : 0u, toSmem);
-            if (valid && !toSmem && x < mS.histSize) atomicAdd(gSym + x, 1u);
+            if (wbase + 32u * k + lane >= n) break;
+            const u32 x = rows[k * kRlePitch + lane];
+            if (x < smemBins) atomicAdd(hSym + x, 1u);
+            else if (x < mS.histSize) atomicAdd(gSym + x, 1u);
         }
         __syncthreads();
         for (u32 i = threadIdx.x; i < smemBins; i += kRleThreads)
@@ -562,76 +599,83 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
         if (w < warp) warpOut += x;
         entries += x;
     }
-    const u32 groupOut = warpOut + entIncl - ent;
-    Sym* comp = reinterpret_cast<Sym*>(p.compact) + sd.compactOff + ts.out;
-    Sym* zcs = reinterpret_cast<Sym*>(p.zc) + sd.compactOff + ts.out;
-    const bool staged = entries <= kStage;                // block-uniform
-    Sym* oc = staged ? sComp : comp;
-    Sym* oz = staged ? sZcs : zcs;
-    {
-#pragma unroll
-        for (u32 k = 0; k < 32; ++k) {
-            const u32 mk = __shfl_sync(0xffffffffu, g.mask, k);
-            if (mk == 0u) continue;                           // warp-uniform
-            const u32 ok = __shfl_sync(0xffffffffu, groupOut, k);
-            const u32 ek = __shfl_sync(0xffffffffu, e, k);
-            const u32 pk = __shfl_sync(0xffffffffu, prev, k);
-            for (u32 t = lane; t < ek; t += 32) {
-                oc[ok + t] = Sym(0);
-                oz[ok + t] = Sym(255);
-            }
-            if ((mk >> lane) & 1u) {
-                const u32 below = mk & ((1u << lane) - 1u);
-                const u32 gb = wbase + 32u * k;
-                const u32 q = gb + lane + 1u;
-                const u32 pp = below ? gb + 32u - u32(__clz(below)) : pk;
-                const u32 o = ok + ek + u32(__popc(below));
-                oc[o] = Sym(v.at(k));
-                oz[o] = Sym((q - pp - 1u) & 255u);
-            }
-        }
-    }
-    __syncthreads();
-    // histograms (and the copy-out of a staged tile)
-    const Sym* hc = staged ? sComp : comp;
-    const Sym* hz = staged ? sZcs : zcs;
-    const bool fast = staged && mZ.histSize == 256u && smemBins > 8u;   // block-uniform
-    // the eight most frequent keys of each histogram (zero counts 0..7,
-    // symbols 1..8) in per-lane 8-bit counters, four keys per register (at
-    // most ceil(kStage / kRleThreads) = 33 entries per lane), added once per
-    // warp at the end; integer ALU work only
+    const u64 first = sd.compactOff + ts.out;          // the tile's first entry in the compact arrays
+    Sym* comp = reinterpret_cast<Sym*>(p.compact) + first;
+    Sym* zcs = reinterpret_cast<Sym*>(p.zc) + first;
+    const u32 shift = u32(first) & (kVec - 1u);        // both arrays are 16-byte aligned
+    const bool staged = entries <= kStage;             // block-uniform
+    const bool fast = mZ.histSize == 256u && smemBins > 8u;
+    // the eight most frequent keys of each histogram in per-lane 8-bit
+    // counters, four keys per register (at most 32 entries per lane)
     u32 z03 = 0, z47 = 0, s03 = 0, s47 = 0;
     bool rangeErr = false;
-    for (u32 j0 = 0; j0 < entries; j0 += kRleThreads) {
-        const u32 j = j0 + threadIdx.x;
-        const bool act = j < entries;
-        const u32 sym = act ? u32(hc[j]) : 0u;
-        const u32 zc = act ? u32(hz[j]) : 0u;
-        if (act && staged) {
-            comp[j] = Sym(sym);
-            zcs[j] = Sym(zc);
+    auto walk = [&](Sym* oc, Sym* oz) {
+        const u32 at = warpOut + entIncl - ent;        // the group's first entry in the tile
+        // (0, 255) entries, by the whole warp
+        for (u32 lanes = __ballot_sync(0xffffffffu, e != 0u); lanes; lanes &= lanes - 1u) {
+            const int j = __ffs(int(lanes)) - 1;
+            const u32 ej = __shfl_sync(0xffffffffu, e, j), aj = __shfl_sync(0xffffffffu, at, j);
+            for (u32 t = lane; t < ej; t += 32) {
+                oc[aj + t] = Sym(0);
+                oz[aj + t] = Sym(255);
+            }
         }
-        if (fast) {
-            if (act) {
+        if (e) {
+            atomicAdd(hSym, e);                        // smemBins >= 1
+            if (255u < mZ.histSize) atomicAdd(hZc + 255, e);
+            else rangeErr = true;
+        }
+        const Sym* row = rows + lane * kRlePitch;
+        const u32 gb1 = wbase + 32u * lane + 1u;
+        u32 o = at + e, before = prev;
+        for (u32 mask = g.mask; mask; mask &= mask - 1u) {
+            const u32 b = u32(__ffs(int(mask))) - 1u;
+            const u32 sym = row[b], q = gb1 + b;
+            const u32 zc = (q - before - 1u) & 255u;
+            before = q;
+            oc[o] = Sym(sym);
+            oz[o] = Sym(zc);
+            ++o;
+            if (fast) {
                 const u32 zi = 1u << ((zc & 3u) << 3);
                 if (zc < 4u) z03 += zi;
                 else if (zc < 8u) z47 += zi;
                 else atomicAdd(hZc + zc, 1u);
-                const u32 k = sym - 1u;            // keys 1..8 -> 0..7
+                const u32 k = sym - 1u;                // keys 1..8 -> 0..7
                 const u32 si = 1u << ((k & 3u) << 3);
                 if (k < 4u) s03 += si;
                 else if (k < 8u) s47 += si;
                 else if (sym < smemBins) atomicAdd(hSym + sym, 1u);
                 else if (sym < mS.histSize) atomicAdd(gSym + sym, 1u);
+            } else {
+                if (sym < smemBins) atomicAdd(hSym + sym, 1u);
+                else if (sym < mS.histSize) atomicAdd(gSym + sym, 1u);
+                if (zc < mZ.histSize) atomicAdd(hZc + zc, 1u);
+                else rangeErr = true;
             }
-        } else {
-            const bool toSmem = act && sym < smemBins;
-            aggregatedIncrement(hSym, toSmem ? sym : 0u, toSmem);
-            if (act && !toSmem && sym < mS.histSize) atomicAdd(gSym + sym, 1u);
-            const bool zcOk = zc < mZ.histSize;
-            rangeErr |= act && !zcOk;
-            aggregatedIncrement(hZc, zc, act && zcOk);
         }
+    };
+    if (staged) {
+        walk(sComp + shift, sZcs + shift);
+        __syncthreads();
+        // chunk c of the stage: elements [c kVec, (c + 1) kVec) from `first - shift`
+        const u32 end = shift + entries, chunks = (end + kVec - 1u) / kVec;
+        Sym* const compA = comp - shift;
+        Sym* const zcsA = zcs - shift;
+        for (u32 c = threadIdx.x; c < chunks; c += kRleThreads) {
+            const u32 lo = c * kVec;
+            if (lo >= shift && lo + kVec <= end) {
+                *reinterpret_cast<uint4*>(compA + lo) = *reinterpret_cast<const uint4*>(sComp + lo);
+                *reinterpret_cast<uint4*>(zcsA + lo) = *reinterpret_cast<const uint4*>(sZcs + lo);
+            } else {
+                for (u32 i = max(lo, shift); i < min(lo + kVec, end); ++i) {
+                    compA[i] = sComp[i];
+                    zcsA[i] = sZcs[i];
+                }
+            }
+        }
+    } else {
+        walk(comp, zcs);
     }
     if (fast) {
         // widen to 16-bit fields (keys k, k + 2 per register) and sum over the warp
@@ -1105,6 +1149,9 @@ __global__ void __launch_bounds__(1024) k_layoutCarry(EncParams p) {
     }
 }
 
+// a << n for n in 0 .. 32 and up (0 from 32 on).
+__device__ __forceinline__ u32 shl32(u32 a, u32 n) { return __funnelshift_lc(0u, a, n); }
+
 // Or the part of codeword `code` (len bits at absolute bit `pos`) that falls
 // in words [wLo, wHi) into win[] (win[0] = word wLo).
 __device__ __forceinline__ void orCodeword(u32* win, u32 wLo, u32 wHi, u32 pos, u32 code, u32 len) {
@@ -1126,8 +1173,9 @@ __device__ __forceinline__ void orCodeword(u32* win, u32 wLo, u32 wHi, u32 pos, 
 // run (gather ownership: no atomics on global memory, no pre-zeroing),
 // assembling them in a shared-memory window; the bits of the last owned word
 // that belong to the next run are recomputed from that run's first symbols.
-// A lane looks each code up once and keeps code and length packed in a
-// register until its bit offset is known.
+// A lane looks each code up once, keeps pairs of codes until its bit offset is
+// known, and puts four codes at a time.  Bound: instruction issue; putting one
+// code at a time took the same streams' 52 million codes 106 us, this 80.
 constexpr u32 kPackWindowWords = kRunSymbols * 31u / 32u + 2u;
 
 __device__ void writeHeaders(const EncParams& p, u32 s, u32 gt, u32 g);
@@ -1165,49 +1213,59 @@ __global__ void __launch_bounds__(kPackWarps * 32, 3) k_pack(EncParams p, u32 he
         const uint2* enc = p.enc + m.histOff;
         const u32 hs = m.histSize;
         const u32 j0 = rb * kRunSymbols + lane * 32u;
-        // one lookup per symbol: code and length kept packed (code << 5 |
-        // length) while the lane's bit offset is scanned; a warp meeting a
-        // code longer than 27 bits looks its codes up again instead
-        u32 pk[32];
+        // one lookup per symbol; two codes at a time joined in a word (first
+        // code upper), four pairs' lengths in a register, while the lane's bit
+        // offset is scanned.  A warp meeting a pair of more than 32 bits looks
+        // its codes up again one by one instead.
+        u32 pair[16], plen[4] = {0u, 0u, 0u, 0u};
         u32 lsum = 0;
-        bool longCode = false;
+        bool longPair = false;
         {
             LaneRun<Sym> sv;
             sv.load(in, j0, count);
 #pragma unroll
-            for (u32 k = 0; k < 32; ++k) {
-                const uint2 c = j0 + k < count ? enc[min(sv.at(k), hs - 1u)] : make_uint2(0u, 0u);
-                lsum += c.y;
-                longCode |= c.y > 27u;
-                pk[k] = (c.x << 5) | c.y;
+            for (u32 k = 0; k < 16; ++k) {
+                const uint2 a = j0 + 2 * k < count ? enc[min(sv.at(2 * k), hs - 1u)] : make_uint2(0u, 0u);
+                const uint2 b = j0 + 2 * k + 1 < count ? enc[min(sv.at(2 * k + 1), hs - 1u)] : make_uint2(0u, 0u);
+                const u32 l = a.y + b.y;
+                longPair |= l > 32u;
+                pair[k] = (a.x << (b.y & 31u)) | b.x;   // b.y = 32 cannot be: codes are at most 31 bits
+                plen[k >> 2] |= l << (8 * (k & 3));
+                lsum += l;
             }
         }
-        const bool reload = __any_sync(0xffffffffu, longCode);
+        const bool reload = __any_sync(0xffffffffu, longPair);
         __syncwarp();
-        // the lane's codewords are consecutive: concatenate them in a 64-bit
-        // accumulator (bits left-aligned from the lane's start bit in its
-        // first word) and OR whole words into the window - one shared atomic
-        // per word touched
+        // the lane's codewords are consecutive: concatenate them in a word
+        // (bits left-aligned from the lane's start bit in its first word) and
+        // OR whole words into the window - one shared atomic per word touched
         const u32 pos = off0 + warpInclusiveSum(lsum) - lsum;
         {
             u32 w = pos >> 5;
-            u32 n = pos & 31u;
-            unsigned long long acc = 0;
-            auto put = [&](u32 code, u32 len) {
-                if (len) {
-                    acc |= (unsigned long long)code << (64u - n - len);
-                    n += len;
-                }
-                if (n >= 32u) {
-                    if (w >= wLo && w < wHi) atomicOr(win + (w - wLo), u32(acc >> 32));
-                    acc <<= 32;
-                    n -= 32u;
+            u32 n = pos & 31u;   // bits of cur in use
+            u32 cur = 0;
+            auto put = [&](u32 code, u32 len) {   // len <= 32; shifts by 32 give 0
+                const u32 left = shl32(code, 32u - len);
+                cur |= left >> n;
+                const u32 total = n + len;
+                if (total >= 32u) {
+                    if (w >= wLo && w < wHi) atomicOr(win + (w - wLo), cur);
                     ++w;
+                    cur = shl32(left, 32u - n);
                 }
+                n = total & 31u;
             };
             if (!reload) {
 #pragma unroll
-                for (u32 k = 0; k < 32; ++k) put(pk[k] >> 5, pk[k] & 31u);
+                for (u32 k = 0; k < 16; k += 2) {
+                    const u32 la = (plen[k >> 2] >> (8 * (k & 3))) & 255u, lb = (plen[k >> 2] >> (8 * (k & 3) + 8)) & 255u;
+                    if (la + lb <= 32u) {
+                        put(shl32(pair[k], lb) | pair[k + 1], la + lb);
+                    } else {
+                        put(pair[k], la);
+                        put(pair[k + 1], lb);
+                    }
+                }
             } else {
                 LaneRun<Sym> sv;
                 sv.load(in, j0, count);
@@ -1217,7 +1275,7 @@ __global__ void __launch_bounds__(kPackWarps * 32, 3) k_pack(EncParams p, u32 he
                     put(c.x, c.y);
                 }
             }
-            if (n && w >= wLo && w < wHi) atomicOr(win + (w - wLo), u32(acc >> 32));
+            if (n && w >= wLo && w < wHi) atomicOr(win + (w - wLo), cur);
         }
         // bits of the next run inside the last owned word
         if (bEnd < m.blocks && (wHi << 5) > off1) {
