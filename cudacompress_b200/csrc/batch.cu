@@ -16,7 +16,7 @@
 //
 // Work areas (one allocation): per level l a dense level-l volume for every
 // brick (forward coefficients, and the reconstructions on the way back),
-// two transform temporaries, the symbols (per brick: lowpass, then the 7
+// a transform temporary, the symbols (per brick: lowpass, then the 7
 // bands of each level coarse -> fine, every band 16-byte aligned), the
 // descriptors, the bricks' streams, and per brick the word offset and bit
 // size of its stream there.
@@ -68,13 +68,13 @@ struct cc_volume_batch {
     ccb::u64* bitSize = nullptr;
     // launch lists
     // per volume v: descriptors and CTAs of volumes 0..v (prefix launches)
-    struct Rows { const ccb::BRowDesc* d; const ccb::u32* map; ccb::u32 n, ctas; std::vector<ccb::u32> descEnd, ctaEnd; };
+    struct Planes { const ccb::BPlaneDesc* d; const ccb::u32* map; ccb::u32 n, ctas; std::vector<ccb::u32> descEnd, ctaEnd; };
     struct Cols { const ccb::BColDesc* d; const ccb::u32* map; ccb::u32 n, ctas; std::vector<ccb::u32> descEnd, ctaEnd; };
     struct Quant { const ccb::BQuantDesc* d; const ccb::u32* map; ccb::u32 n, ctas; std::vector<ccb::u32> descEnd, ctaEnd; };
     struct Levels { const ccb::BLevelDesc* d; const ccb::u32* map; ccb::u32 n, ctas; std::vector<ccb::u32> descEnd, ctaEnd; };
     std::vector<Levels> fwdLevel;              // per level: the fused forward pass
-    std::vector<Rows> fwdRows, invRows;        // per level
-    std::vector<Cols> fwdY, fwdZ, invZ, invY;  // per level
+    std::vector<Cols> invZ;                    // per level: Z from symbols
+    std::vector<Planes> invPlanes;             // per level: Y and X
     Quant quant{}, dequantLP{};
     ccb::EncPlan enc, encLP;           // highpass streams (I), lowpass streams (ILP)
     ccb::DecPlan dec;
@@ -110,10 +110,10 @@ struct Arena {
 
 u64 vol3(u32 x, u32 y, u32 z) { return u64(x) * y * z; }
 
-void addRows(std::vector<BRowDesc>& v, u32& ctas, BRowDesc d) {
-    batchRowPlan(d);
+void addPlanes(std::vector<BPlaneDesc>& v, u32& ctas, BPlaneDesc d) {
+    const u32 n = batchPlanePlan(d);
     d.ctaOff = ctas;
-    ctas += u32(d.tilesX) * u32(ceilDiv(u64(d.ny) * d.nz, d.R));
+    ctas += n;
     v.push_back(d);
 }
 
@@ -355,11 +355,9 @@ static int batchEnqueueDecompress(cc_volume_batch* b) {
     for (int l = int(b->levels) - 1; l >= 0; --l) {
         SectionTimer t(I, "batch.dwt_inverse", st);
         prefixOf(b->invZ[l], k, nd, ctas);
-        launchBatchCols(b->invZ[l].d, b->invZ[l].map, ctas, true, true, st);
-        prefixOf(b->invY[l], k, nd, ctas);
-        launchBatchCols(b->invY[l].d, b->invY[l].map, ctas, true, false, st);
-        prefixOf(b->invRows[l], k, nd, ctas);
-        launchBatchRows(b->invRows[l].d, b->invRows[l].map, ctas, true, b->inTab, b->outTab, st);
+        launchBatchSymbolCols(b->invZ[l].d, b->invZ[l].map, ctas, st);
+        prefixOf(b->invPlanes[l], k, nd, ctas);
+        launchBatchPlanes(b->invPlanes[l].d, b->invPlanes[l].map, ctas, b->outTab, st);
     }
     CC_TRY_CUDA(cudaGetLastError(), "batch decompress");
     return CC_OK;
@@ -501,8 +499,7 @@ int cc_volume_batch_create(cc_instance* user, uint32_t count, const uint32_t* si
 int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t* sizes, uint32_t levels,
                               const float* quantSteps, uint32_t zChunk, cc_volume_batch** out) {
     if (!out) { setError("cc_volume_batch_create: out is NULL"); return CC_ERR_INVALID_ARGUMENT; }
-    if (zChunk == 0) zChunk = kLvZCDefault;
-    if (zChunk < 8 || zChunk > 256 || (zChunk & 1)) {
+    if (zChunk != 0 && (zChunk < 8 || zChunk > 256 || (zChunk & 1))) {
         setError("cc_volume_batch_create_ex: z_chunk must be 0 (default) or even in 8..256 (got %u)", zChunk);
         *out = nullptr;
         return CC_ERR_INVALID_ARGUMENT;
@@ -591,7 +588,7 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
     std::vector<u64> tOff(count);
     u64 tTot = 0;
     for (u32 v = 0; v < count; ++v) { tOff[v] = tTot; tTot += alignUp(vol3(b->nx[v], b->ny[v], b->nz[v]), 64); }
-    const size_t t1At = A.take(tTot * sizeof(float)), t2At = A.take(tTot * sizeof(float));
+    const size_t tAt = A.take(tTot * sizeof(float));
     std::vector<SymLayout> sl(count);
     std::vector<u64> symOff(count);
     u64 symTot = 0;
@@ -607,14 +604,28 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
 
     // ---- descriptors (host) ----
     auto lev = [&](u32 l, u32 v) { return reinterpret_cast<float*>(levAt[l]) + levOff[l][v]; };   // offsets, rebased below
-    auto t1 = [&](u32 v) { return reinterpret_cast<float*>(t1At) + tOff[v]; };
-    auto t2 = [&](u32 v) { return reinterpret_cast<float*>(t2At) + tOff[v]; };
+    auto t = [&](u32 v) { return reinterpret_cast<float*>(tAt) + tOff[v]; };
     auto sy = [&](u32 v) { return reinterpret_cast<u16*>(symAt) + symOff[v]; };
     std::vector<std::vector<BLevelDesc>> fl(L);
     std::vector<u32> flC(L, 0);
-    std::vector<std::vector<BRowDesc>> fr(L), ir(L);
-    std::vector<std::vector<BColDesc>> fy(L), fz(L), iz(L), iy(L);
-    std::vector<u32> frC(L, 0), irC(L, 0), fyC(L, 0), fzC(L, 0), izC(L, 0), iyC(L, 0);
+    // the forward level's tile depth, unless the caller gives one
+    std::vector<u32> depth(L, zChunk);
+    if (zChunk == 0) {
+        const u32 sms = u32(std::max(1, b->ILP->smCount > 0 ? b->ILP->smCount : 148));
+        for (u32 l = 0; l < L; ++l) {
+            auto ctas = [&](u32 zc) {
+                u64 n = 0;
+                for (u32 v = 0; v < count; ++v)
+                    n += ceilDiv(b->nx[v] >> l, kLvTX) * ceilDiv(b->ny[v] >> l, kLvTY) * ceilDiv(b->nz[v] >> l, zc);
+                return n;
+            };
+            depth[l] = kLvZCDefault;
+            while (depth[l] > kLvZCLeast && ctas(depth[l]) < 2ull * sms) depth[l] /= 2;
+        }
+    }
+    std::vector<std::vector<BColDesc>> iz(L);
+    std::vector<std::vector<BPlaneDesc>> ip(L);
+    std::vector<u32> izC(L, 0), ipC(L, 0);
     std::vector<BQuantDesc> qd, dq;
     u32 qC = 0, dqC = 0;
     std::vector<EncStream> es;
@@ -642,45 +653,12 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
             fd.inv = 1.0f / (b->q0[v] / float(1u << l));              // Quantize.cu:90: reciprocal on the host
             fd.invLP = 1.0f / (b->q0[v] / float(1u << (L - 1)));
             fd.lastLevel = l + 1 == L ? 1 : 0;
-            fd.zChunk = int(zChunk);
+            fd.zChunk = int(depth[l]);
             addLevel(fl[l], flC[l], fd);
-            // X: input (level 0: the caller's volume, tight; else the LLL octant of level l-1) -> t1
-            BRowDesc r{};
-            r.vol = int(v);
-            r.src = l == 0 ? nullptr : lev(l - 1, v);
-            r.dst = t1(v);
-            r.nx = sx; r.ny = syz; r.nz = sz;
-            r.srcRow = l == 0 ? int(X) : int(X >> (l - 1));
-            r.srcSlice = l == 0 ? int(X * Y) : int((X >> (l - 1)) * (Y >> (l - 1)));
-            r.dstRow = sx; r.dstSlice = sx * syz;
-            addRows(fr[l], frC[l], r);
-            // Y: t1 -> t2 (dense level l)
-            BColDesc c{};
-            c.src = t1(v); c.dst = t2(v);
-            c.nx = sx; c.na = syz; c.nc = sz;
-            c.sa = sx; c.sc = sx * syz;
-            c.da = sx; c.dc = sx * syz;
-            addCols(fy[l], fyC[l], c);
-            // Z: t2 -> level l coefficients, quantized in the store: the LLL
-            // octant stays float (next level's input) except at the coarsest
-            // level, where it is the lowpass band
-            BColDesc cz = c;
-            cz.src = t2(v); cz.dst = lev(l, v);
-            cz.na = sz; cz.nc = syz;
-            cz.sa = sx * syz; cz.sc = sx;
-            cz.da = sx * syz; cz.dc = sx;
-            cz.symOut = sy(v) + sl[v].level[l];
-            cz.lpSymOut = sy(v) + sl[v].lp;
-            cz.bandStride = sl[v].bandStride[l];
-            cz.hx = sx / 2; cz.hy = syz / 2; cz.hz = sz / 2;
-            cz.inv = 1.0f / (b->q0[v] / float(1u << l));              // Quantize.cu:90: reciprocal on the host
-            cz.invLP = 1.0f / (b->q0[v] / float(1u << (L - 1)));
-            cz.lastLevel = l + 1 == L ? 1 : 0;
-            addCols(fz[l], fzC[l], cz);
-            // inverse of level l: Z from symbols (lowpass = level l+1 reconstruction) -> t2, Y -> t1, X -> level l
+            // inverse of level l: Z from symbols (lowpass = level l+1 reconstruction) -> t, Y and X -> level l
             BColDesc ic{};
             ic.src = lev(l + 1, v);
-            ic.dst = t2(v);
+            ic.dst = t(v);
             ic.nx = sx; ic.na = sz; ic.nc = syz;
             ic.da = sx * syz; ic.dc = sx;
             ic.bands = sy(v) + sl[v].level[l];
@@ -689,20 +667,14 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
             ic.hx = sx / 2; ic.hy = syz / 2; ic.hz = sz / 2;
             ic.lpRow = sx / 2; ic.lpSlice = (sx / 2) * (syz / 2);
             addCols(iz[l], izC[l], ic);
-            BColDesc iyd{};
-            iyd.src = t2(v); iyd.dst = t1(v);
-            iyd.nx = sx; iyd.na = syz; iyd.nc = sz;
-            iyd.sa = sx; iyd.sc = sx * syz;
-            iyd.da = sx; iyd.dc = sx * syz;
-            addCols(iy[l], iyC[l], iyd);
-            BRowDesc irw{};
-            irw.vol = int(v);
-            irw.src = t1(v);
-            irw.dst = l == 0 ? nullptr : lev(l, v);
-            irw.nx = sx; irw.ny = syz; irw.nz = sz;
-            irw.srcRow = sx; irw.srcSlice = sx * syz;
-            irw.dstRow = sx; irw.dstSlice = sx * syz;
-            addRows(ir[l], irC[l], irw);
+            BPlaneDesc pl{};
+            pl.vol = int(v);
+            pl.src = t(v);
+            pl.dst = l == 0 ? nullptr : lev(l, v);
+            pl.nx = sx; pl.ny = syz; pl.nz = sz;
+            pl.srcRow = sx; pl.srcSlice = sx * syz;
+            pl.dstRow = sx; pl.dstSlice = sx * syz;
+            addPlanes(ip[l], ipC[l], pl);
         }
         // quantization: lowpass (step q0 / 2^(L-1)), then levels coarse -> fine (step q0 / 2^l)
         const u32 Lx = X >> (L - 1), Ly = Y >> (L - 1);
@@ -745,16 +717,12 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
 
     // ---- device plan ----
     auto bytesOf = [](size_t n, size_t e) { return n * e; };
-    std::vector<size_t> flAt(L), frAt(L), irAt(L), fyAt(L), fzAt(L), izAt(L), iyAt(L);
+    std::vector<size_t> flAt(L), izAt(L), ipAt(L);
     A.off = alignUp(A.off, 256);
     for (u32 l = 0; l < L; ++l) {
         flAt[l] = A.take(bytesOf(fl[l].size(), sizeof(BLevelDesc)), 64);
-        frAt[l] = A.take(bytesOf(fr[l].size(), sizeof(BRowDesc)), 64);
-        irAt[l] = A.take(bytesOf(ir[l].size(), sizeof(BRowDesc)), 64);
-        fyAt[l] = A.take(bytesOf(fy[l].size(), sizeof(BColDesc)), 64);
-        fzAt[l] = A.take(bytesOf(fz[l].size(), sizeof(BColDesc)), 64);
+        ipAt[l] = A.take(bytesOf(ip[l].size(), sizeof(BPlaneDesc)), 64);
         izAt[l] = A.take(bytesOf(iz[l].size(), sizeof(BColDesc)), 64);
-        iyAt[l] = A.take(bytesOf(iy[l].size(), sizeof(BColDesc)), 64);
     }
     const size_t qAt = A.take(bytesOf(qd.size(), sizeof(BQuantDesc)), 64);
     const size_t dqAt = A.take(bytesOf(dq.size(), sizeof(BQuantDesc)), 64);
@@ -766,15 +734,11 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
         maps.push_back(std::move(m));
         return maps.size() - 1;
     };
-    std::vector<size_t> flMap(L), frMap(L), irMap(L), fyMap(L), fzMap(L), izMap(L), iyMap(L);
+    std::vector<size_t> flMap(L), izMap(L), ipMap(L);
     for (u32 l = 0; l < L; ++l) {
         flMap[l] = addMap(ctaMapOf(fl[l], flC[l]));
-        frMap[l] = addMap(ctaMapOf(fr[l], frC[l]));
-        irMap[l] = addMap(ctaMapOf(ir[l], irC[l]));
-        fyMap[l] = addMap(ctaMapOf(fy[l], fyC[l]));
-        fzMap[l] = addMap(ctaMapOf(fz[l], fzC[l]));
+        ipMap[l] = addMap(ctaMapOf(ip[l], ipC[l]));
         izMap[l] = addMap(ctaMapOf(iz[l], izC[l]));
-        iyMap[l] = addMap(ctaMapOf(iy[l], iyC[l]));
     }
     const size_t qMap = addMap(ctaMapOf(qd, qC)), dqMap = addMap(ctaMapOf(dq, dqC));
     // the encodes' streams: the lowpass streams, and the highpass streams with
@@ -811,16 +775,12 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
             d.symOut = rebaseS(d.symOut);
             d.lpSymOut = rebaseS(d.lpSymOut);
         }
-        for (auto& d : fr[l]) { d.src = rebaseF(d.src); d.dst = rebaseF(d.dst); }
-        for (auto& d : ir[l]) { d.src = rebaseF(d.src); d.dst = rebaseF(d.dst); }
-        for (auto* vv : {&fy[l], &fz[l], &iz[l], &iy[l]})
-            for (auto& d : *vv) {
-                d.src = rebaseF(d.src);
-                d.dst = rebaseF(d.dst);
-                d.bands = rebaseS(d.bands);
-                d.symOut = rebaseS(d.symOut);
-                d.lpSymOut = rebaseS(d.lpSymOut);
-            }
+        for (auto& d : ip[l]) { d.src = rebaseF(d.src); d.dst = rebaseF(d.dst); }
+        for (auto& d : iz[l]) {
+            d.src = rebaseF(d.src);
+            d.dst = rebaseF(d.dst);
+            d.bands = rebaseS(d.bands);
+        }
     }
     for (auto& d : qd) { d.src = rebaseF(d.src); d.sym = rebaseS(d.sym); }
     for (auto& d : dq) { d.sym = rebaseS(d.sym); d.dstF = rebaseF(d.dstF); }
@@ -853,12 +813,8 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
     e = cudaMemset(b->mem, 0, b->memBytes);
     for (u32 l = 0; l < L && e == cudaSuccess; ++l) {
         e = up(flAt[l], fl[l].data(), fl[l].size() * sizeof(BLevelDesc));
-        if (e == cudaSuccess) e = up(frAt[l], fr[l].data(), fr[l].size() * sizeof(BRowDesc));
-        if (e == cudaSuccess) e = up(irAt[l], ir[l].data(), ir[l].size() * sizeof(BRowDesc));
-        if (e == cudaSuccess) e = up(fyAt[l], fy[l].data(), fy[l].size() * sizeof(BColDesc));
-        if (e == cudaSuccess) e = up(fzAt[l], fz[l].data(), fz[l].size() * sizeof(BColDesc));
+        if (e == cudaSuccess) e = up(ipAt[l], ip[l].data(), ip[l].size() * sizeof(BPlaneDesc));
         if (e == cudaSuccess) e = up(izAt[l], iz[l].data(), iz[l].size() * sizeof(BColDesc));
-        if (e == cudaSuccess) e = up(iyAt[l], iy[l].data(), iy[l].size() * sizeof(BColDesc));
     }
     for (size_t m = 0; m < maps.size() && e == cudaSuccess; ++m) e = up(mapAt[m], maps[m].data(), maps[m].size() * sizeof(u32));
     if (e == cudaSuccess) e = up(qAt, qd.data(), qd.size() * sizeof(BQuantDesc));
@@ -878,16 +834,12 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
     b->qdHost = qd;
     b->dqHost = dq;
     b->fwdLevel.resize(L);
-    b->fwdRows.resize(L); b->invRows.resize(L); b->fwdY.resize(L); b->fwdZ.resize(L); b->invZ.resize(L); b->invY.resize(L);
+    b->invZ.resize(L); b->invPlanes.resize(L);
     auto mapPtr = [&](size_t m) { return reinterpret_cast<const u32*>(base + mapAt[m]); };
     for (u32 l = 0; l < L; ++l) {
         b->fwdLevel[l] = {reinterpret_cast<const BLevelDesc*>(base + flAt[l]), mapPtr(flMap[l]), u32(fl[l].size()), flC[l]};
-        b->fwdRows[l] = {reinterpret_cast<const BRowDesc*>(base + frAt[l]), mapPtr(frMap[l]), u32(fr[l].size()), frC[l]};
-        b->invRows[l] = {reinterpret_cast<const BRowDesc*>(base + irAt[l]), mapPtr(irMap[l]), u32(ir[l].size()), irC[l]};
-        b->fwdY[l] = {reinterpret_cast<const BColDesc*>(base + fyAt[l]), mapPtr(fyMap[l]), u32(fy[l].size()), fyC[l]};
-        b->fwdZ[l] = {reinterpret_cast<const BColDesc*>(base + fzAt[l]), mapPtr(fzMap[l]), u32(fz[l].size()), fzC[l]};
+        b->invPlanes[l] = {reinterpret_cast<const BPlaneDesc*>(base + ipAt[l]), mapPtr(ipMap[l]), u32(ip[l].size()), ipC[l]};
         b->invZ[l] = {reinterpret_cast<const BColDesc*>(base + izAt[l]), mapPtr(izMap[l]), u32(iz[l].size()), izC[l]};
-        b->invY[l] = {reinterpret_cast<const BColDesc*>(base + iyAt[l]), mapPtr(iyMap[l]), u32(iy[l].size()), iyC[l]};
     }
     b->quant = {reinterpret_cast<const BQuantDesc*>(base + qAt), mapPtr(qMap), u32(qd.size()), qC};
     b->dequantLP = {reinterpret_cast<const BQuantDesc*>(base + dqAt), mapPtr(dqMap), u32(dq.size()), dqC};
@@ -903,12 +855,8 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
     };
     for (u32 l = 0; l < L; ++l) {
         prefix(b->fwdLevel[l], fl[l], 1);
-        prefix(b->fwdRows[l], fr[l], 1);
-        prefix(b->invRows[l], ir[l], 1);
-        prefix(b->fwdY[l], fy[l], 1);
-        prefix(b->fwdZ[l], fz[l], 1);
+        prefix(b->invPlanes[l], ip[l], 1);
         prefix(b->invZ[l], iz[l], 1);
-        prefix(b->invY[l], iy[l], 1);
     }
     prefix(b->quant, qd, 1 + 7 * L);
     prefix(b->dequantLP, dq, 1);

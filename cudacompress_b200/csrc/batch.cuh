@@ -35,17 +35,28 @@ struct BColDesc {
     u64 bandStride;
     float step;
     int hx, hy, hz, lpRow, lpSlice;
-    // last forward pass of a level (axis Z) with quantization fused into the
-    // store: the 7 highpass octants go to symOut (band b-1 at b-1 bandStride)
-    // quantized with inv; the LLL octant stays float in dst, or - at the
-    // coarsest level - goes to lpSymOut quantized with invLP
-    u16* symOut;
-    u16* lpSymOut;
-    float inv, invLP;
-    int lastLevel;
     u32 tilesX, tilesA;
     u32 ctaOff;
 };
+
+// Both axes of a plane in one pass: tx x ty outputs of tz slices per CTA, staged
+// with their 4-sample mirrored halos in shared memory; the inverse filters
+// along Y, then X (its order), the forward along X, then Y.
+struct BPlaneDesc {
+    const float* src;
+    float* dst;             // nullptr: the volume's entry of the output pointer table
+    int vol;
+    int nx, ny, nz;
+    int srcRow, srcSlice, dstRow, dstSlice;
+    int tx, ty, tz, pitch;  // tile, multiples of 8 (tz slices); floats per staged row
+    int tilesX, tilesY;
+    int vec;                // nx and the destination pitches allow float4 rows
+    u32 ctaOff;
+};
+constexpr int kPlaneThreads = 288;
+constexpr int kPlaneTile = 64;
+constexpr int kPlaneFloats = (kPlaneTile + 8) * (kPlaneTile + 12);   // staged floats of a CTA
+constexpr int kPlaneLoads = (kPlaneTile + 8) * (kPlaneTile + 8) / 2 / kPlaneThreads;   // pairs per thread
 
 // One band: deadzone quantization to u16 symbols (src strided -> sym dense),
 // or (dstF set) dequantization of dense symbols to a dense float block.
@@ -81,7 +92,11 @@ struct BLevelDesc {
     u32 ctaOff;
 };
 constexpr int kLvTX = 64, kLvTY = 16;
-constexpr int kLvZCDefault = 32;   // default Z extent of a tile (cc_volume_batch_create_ex: 8..256)
+// Z extent of a tile (cc_volume_batch_create_ex: 8..256).  By default 32, halved
+// down to 8 while the level has fewer than two CTAs per SM: a tile streams its
+// slices and 8 of halo one after the other, so a level of few tiles takes as
+// long as one of them (32^3: 26 us at 32, 13 at 8).
+constexpr u32 kLvZCDefault = 32, kLvZCLeast = 8;
 
 constexpr int kBRowOutputs = 4096;    // outputs per row-pass CTA
 constexpr int kBRowMaxWidth = 2048;   // row tile width
@@ -92,10 +107,8 @@ constexpr int kBColTileA = 64;
 constexpr int kBQuantPerCta = 4096;
 
 // Descriptor arrays and CTA maps are device pointers; ctas = CTA count.
-void launchBatchRows(const BRowDesc* d, const u32* map, u32 ctas, bool inverse, const float* const* inTab,
-                     float* const* outTab, cudaStream_t st);
-void launchBatchCols(const BColDesc* d, const u32* map, u32 ctas, bool inverse, bool fromSymbols, cudaStream_t st,
-                     bool quantizeStore = false);
+void launchBatchSymbolCols(const BColDesc* d, const u32* map, u32 ctas, cudaStream_t st);
+void launchBatchPlanes(const BPlaneDesc* d, const u32* map, u32 ctas, float* const* outTab, cudaStream_t st);
 void launchBatchQuant(const BQuantDesc* d, const u32* map, u32 ctas, bool dequantize, cudaStream_t st);
 void launchBatchLevelFwd(const BLevelDesc* d, const u32* map, u32 ctas, const float* const* inTab, cudaStream_t st);
 
@@ -113,6 +126,28 @@ inline void batchRowPlan(BRowDesc& d) {
     d.tilesX = int(ceilDiv(d.nx, d.W));
     d.vec = (d.nx % 8 == 0 && d.W % 8 == 0 && d.srcRow % 4 == 0 && d.srcSlice % 4 == 0 && d.dstRow % 4 == 0 &&
              d.dstSlice % 4 == 0) ? 1 : 0;
+}
+
+// Tiles of a plane pass: at most kPlaneTile wide and high, balanced over the
+// extents, and as many slices as the CTA's shared memory and threads hold - a
+// thread takes one column pair of eight rows (Y) and at most two groups of
+// eight columns of a staged row (X).  Returns the CTAs.
+inline u32 batchPlanePlan(BPlaneDesc& d) {
+    auto tile = [](int n) { return int(alignUp(ceilDiv(n, ceilDiv(n, kPlaneTile)), 8)); };
+    d.tx = tile(d.nx);
+    d.ty = tile(d.ny);
+    d.pitch = d.tx + 12;
+    d.tilesX = int(ceilDiv(d.nx, d.tx));
+    d.tilesY = int(ceilDiv(d.ny, d.ty));
+    auto fits = [&](int tz) {
+        const int rows = tz * (d.ty + 8), pairs = (d.tx + 8) / 2;
+        return rows * d.pitch <= kPlaneFloats && rows <= kPlaneLoads * (kPlaneThreads / pairs) &&
+               tz * (d.ty / 8) * pairs <= kPlaneThreads && rows * (d.tx / 8) <= 2 * kPlaneThreads;
+    };
+    d.tz = 1;
+    while (d.tz < d.nz && fits(d.tz + 1)) ++d.tz;
+    d.vec = d.nx % 8 == 0 && d.dstRow % 4 == 0 && d.dstSlice % 4 == 0 ? 1 : 0;
+    return u32(d.tilesX) * u32(d.tilesY) * u32(ceilDiv(d.nz, d.tz));
 }
 
 // One 2D level of the integer transform between samples and symbol bands (dwt.cu).

@@ -13,6 +13,8 @@
 // Int: CDF 5/3 lifting on shorts (DWTIntKernels.cui:14-1188) with the
 // reference's rounding (DWTCommon.cuh:133-142), including the narrowing of
 // every intermediate to 16 bits.
+#include <type_traits>
+
 #include "batch.cuh"
 
 namespace ccb {
@@ -520,6 +522,23 @@ template <bool kInverse>
 static void colPassFloat(float* dst, const float* src, int nx, int ny, int nz, int axis, int srcRow, int srcSlice,
                          int dstRow, int dstSlice, cudaStream_t st);
 
+template <bool kInverse>
+static void planePass(float* dst, const float* src, int nx, int ny, int nz, int srcRow, int srcSlice, int dstRow,
+                      int dstSlice, cudaStream_t st);
+
+// The plane pass's byte pitches are 32-bit.
+static bool planeFits(int row, int slice) { return row < (1 << 29) && slice < (1 << 29); }
+
+// Whether two arrays of a transform's extents share memory: the two passes
+// that a plane pass replaces go through a buffer, so their source may lie in
+// their destination.
+static bool overlap(const float* a, int rowA, int sliceA, const float* b, int rowB, int sliceB, int nx, int ny, int nz) {
+    auto end = [&](const float* p, int row, int slice) {
+        return reinterpret_cast<uintptr_t>(p + size_t(nz - 1) * slice + size_t(ny - 1) * row + nx);
+    };
+    return reinterpret_cast<uintptr_t>(a) < end(b, rowB, sliceB) && reinterpret_cast<uintptr_t>(b) < end(a, rowA, sliceA);
+}
+
 // A column pass between float arrays of the same pitches.
 template <bool kInverse>
 static void floatCols(float* dst, const float* src, int nx, int ny, int nz, int axis, int row, int slice, cudaStream_t st) {
@@ -552,6 +571,33 @@ void inverseRows<float>(float* dst, const float* src, int nx, int ny, int nz, in
     else rowPass<float, float, true>(dst, src, nx, ny, nz, 1, srcRow, srcSlice, ch, dstRow, dstSlice, st);
 }
 
+// X and Y of a forward level (src -> dst, the X result through buf when they
+// run as two passes) and Y and X of an inverse one.
+template <class TIn>
+static void forwardPlane(float* dst, float* buf, const TIn* src, int nx, int ny, int nz, int ch, int srcRow, int srcSlice,
+                         int dstRow, int dstSlice, cudaStream_t st) {
+    if constexpr (std::is_same<TIn, float>::value) {
+        if (ch == 1 && planeFits(srcRow, srcSlice) && !overlap(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz)) {
+            planePass<false>(dst, src, nx, ny, nz, srcRow, srcSlice, dstRow, dstSlice, st);
+            return;
+        }
+    }
+    forwardRows<TIn>(buf, src, nx, ny, nz, ch, srcRow, srcSlice, dstRow, dstSlice, st);
+    floatCols<false>(dst, buf, nx, ny, nz, 1, dstRow, dstSlice, st);
+}
+template <class TOut>
+static void inversePlane(TOut* dst, float* buf, const float* src, int nx, int ny, int nz, int ch, int srcRow, int srcSlice,
+                         int dstRow, int dstSlice, cudaStream_t st) {
+    if constexpr (std::is_same<TOut, float>::value) {
+        if (ch == 1 && planeFits(srcRow, srcSlice) && !overlap(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz)) {
+            planePass<true>(dst, src, nx, ny, nz, srcRow, srcSlice, dstRow, dstSlice, st);
+            return;
+        }
+    }
+    floatCols<true>(buf, src, nx, ny, nz, 1, srcRow, srcSlice, st);
+    inverseRows<TOut>(dst, buf, nx, ny, nz, ch, srcRow, srcSlice, dstRow, dstSlice, st);
+}
+
 static bool checkSizes(int sx, int sy, int sz, const char* what) {
     bool ok = sx >= 8 && sy >= 8 && sz >= 1 && (sx % 2 == 0) && (sy % 2 == 0) && (sz == 1 || (sz >= 8 && sz % 2 == 0));
     if (!ok) setError("%s: sizes must be even and >= 8 (got %d x %d x %d)", what, sx, sy, sz);
@@ -574,9 +620,8 @@ static int floatForward(float* dst, float* buf2, float* buf1, const TIn* src, in
     if (srcRow <= 0) srcRow = sx * ch;
     if (srcSlice <= 0) srcSlice = sy * srcRow;
     const bool do3D = sz > 1;
-    forwardRows<TIn>(buf1, src, sx, sy, sz, ch, srcRow, srcSlice, dstRow, dstSlice, st);
     float* yDst = do3D ? buf2 : dst;
-    floatCols<false>(yDst, buf1, sx, sy, sz, 1, dstRow, dstSlice, st);
+    forwardPlane<TIn>(yDst, buf1, src, sx, sy, sz, ch, srcRow, srcSlice, dstRow, dstSlice, st);
     if (do3D) floatCols<false>(dst, buf2, sx, sy, sz, 2, dstRow, dstSlice, st);
     CC_TRY_CUDA(cudaGetLastError(), what);
     return CC_OK;
@@ -597,8 +642,7 @@ static int floatInverse(TOut* dst, float* buf2, float* buf1, const float* src, i
         floatCols<true>(buf2, src, sx, sy, sz, 2, srcRow, srcSlice, st);
         ySrc = buf2;
     }
-    floatCols<true>(buf1, ySrc, sx, sy, sz, 1, srcRow, srcSlice, st);
-    inverseRows<TOut>(dst, buf1, sx, sy, sz, ch, srcRow, srcSlice, dstRow, dstSlice, st);
+    inversePlane<TOut>(dst, buf1, ySrc, sx, sy, sz, ch, srcRow, srcSlice, dstRow, dstSlice, st);
     CC_TRY_CUDA(cudaGetLastError(), what);
     return CC_OK;
 }
@@ -633,11 +677,11 @@ static int floatInverseFromSymbols(TOut* dst, float* buf2, float* buf1, const fl
     };
     if (do3D) {
         if (symBytes == 2) first(u16(), buf2, 2); else first(u32(), buf2, 2);
-        floatCols<true>(buf1, buf2, sx, sy, sz, 1, bRow, bSlice, st);
+        inversePlane<TOut>(dst, buf1, buf2, sx, sy, sz, ch, bRow, bSlice, dstRow, dstSlice, st);
     } else {
         if (symBytes == 2) first(u16(), buf1, 1); else first(u32(), buf1, 1);
+        inverseRows<TOut>(dst, buf1, sx, sy, sz, ch, bRow, bSlice, dstRow, dstSlice, st);
     }
-    inverseRows<TOut>(dst, buf1, sx, sy, sz, ch, bRow, bSlice, dstRow, dstSlice, st);
     CC_TRY_CUDA(cudaGetLastError(), what);
     return CC_OK;
 }
@@ -956,14 +1000,7 @@ __device__ __forceinline__ void rowsTile(const BRowDesc& D, const float* src, fl
     }
 }
 
-template <bool kInverse>
-__global__ void __launch_bounds__(256, kInverse ? 8 : 6) k_bRows(const BRowDesc* __restrict__ descs, const u32* __restrict__ map,
-                                               const float* const* inTab, float* const* outTab) {
-    const BRowDesc D = descs[map[blockIdx.x]];
-    rowsTile<kInverse>(D, D.src ? D.src : inTab[D.vol], D.dst ? D.dst : outTab[D.vol], blockIdx.x - D.ctaOff);
-}
-
-// The same pass of one volume, its descriptor a parameter (dwtFloat calls).
+// A row pass of one volume, its descriptor a parameter (dwtFloat calls).
 template <bool kInverse>
 __global__ void __launch_bounds__(256, kInverse ? 8 : 6) k_rowsOne(const __grid_constant__ BRowDesc D) {
     rowsTile<kInverse>(D, D.src, D.dst, blockIdx.x);
@@ -1007,47 +1044,11 @@ __device__ __forceinline__ float2 bandPair(const BColDesc& D, int x, int y, int 
     return make_float2((float(q0) + signI(q0) * 0.5f) * D.step, (float(q1) + signI(q1) * 0.5f) * D.step);
 }
 
-// One sample of the fused store (see BColDesc::symOut): (x, y, z) in the
-// level's [L|H] layout.  Deadzone quantization as k_bQuant's
-// (Quantize.cuh:55-59, reciprocal from the host).
-__device__ __forceinline__ void quantStoreOne(const BColDesc& D, int x, int y, int z, float v) {
-    const int bx = x >= D.hx, by = y >= D.hy, bz = z >= D.hz;
-    const int b = bx + 2 * by + 4 * bz;
-    if (b == 0 && !D.lastLevel) {
-        D.dst[size_t(x) + size_t(z) * D.da + size_t(y) * D.dc] = v;
-        return;
-    }
-    const int lx = x - bx * D.hx, ly = y - by * D.hy, lz = z - bz * D.hz;
-    u16* base = b == 0 ? D.lpSymOut : D.symOut + u64(b - 1) * D.bandStride;
-    base[(u64(lz) * D.hy + ly) * D.hx + lx] = u16(symbolizeI(int(v * (b == 0 ? D.invLP : D.inv))));
-}
-
-// The samples (x, x + 1), x even; with an even half width both lie in one
-// octant at an even offset (one float2 or one 4-byte symbol pair).
-__device__ __forceinline__ void quantStorePair(const BColDesc& D, int x, int y, int z, float2 v) {
-    if (D.hx & 1) {
-        quantStoreOne(D, x, y, z, v.x);
-        quantStoreOne(D, x + 1, y, z, v.y);
-        return;
-    }
-    const int bx = x >= D.hx, by = y >= D.hy, bz = z >= D.hz;
-    const int b = bx + 2 * by + 4 * bz;
-    if (b == 0 && !D.lastLevel) {
-        *reinterpret_cast<float2*>(D.dst + size_t(x) + size_t(z) * D.da + size_t(y) * D.dc) = v;
-        return;
-    }
-    const int lx = x - bx * D.hx, ly = y - by * D.hy, lz = z - bz * D.hz;
-    u16* base = b == 0 ? D.lpSymOut : D.symOut + u64(b - 1) * D.bandStride;
-    const float inv = b == 0 ? D.invLP : D.inv;
-    const u32 s0 = symbolizeI(int(v.x * inv)) & 0xFFFFu, s1 = symbolizeI(int(v.y * inv)) & 0xFFFFu;
-    *reinterpret_cast<u32*>(base + (u64(lz) * D.hy + ly) * D.hx + lx) = s0 | (s1 << 16);
-}
-
 // Eight consecutive outputs of a column pair per thread: the 16 staged
 // samples they use are read from shared memory once into registers (a
 // sliding window) instead of nine reads per output.  The tile's first row
 // is even, so output j has parity j & 1 and its taps are immediates.
-template <bool kInverse, bool kQuantize = false, bool kPacked = false>
+template <bool kInverse, bool kPacked>
 __device__ __forceinline__ void colOutputs8(const BColDesc& D, const float2 (*s)[33], int tx, int ty, int x, int c,
                                             int a0) {
     static_assert(kBColTileA == 64, "eight outputs per thread row of an 8-row block");
@@ -1077,47 +1078,7 @@ __device__ __forceinline__ void colOutputs8(const BColDesc& D, const float2 (*s)
                         : make_float2(fir9c<kInverse, 0>(v0), fir9c<kInverse, 0>(v1));
         }
         const int o = kInverse ? a : splitPos(a, D.na);
-        if (kQuantize) quantStorePair(D, x, c, o, r);   // axis Z: a = z, c = y
-        else *reinterpret_cast<float2*>(D.dst + size_t(x) + size_t(o) * D.da + size_t(c) * D.dc) = r;
-    }
-}
-
-// The same outputs with the quantizer fused into the store (axis Z, a = z,
-// c = y), for an even half width hx and hz = na / 2: the thread's x and y fix
-// its octant up to bz, and output a lands in octant bz = a & 1 at lz = a >> 1
-// (a's split position is a / 2 or hz + a / 2), so every store goes to one of
-// two per-thread bases.  Symbols as quantStorePair computes them.
-__device__ __forceinline__ void colOutputs8Quantize(const BColDesc& D, const float2 (*s)[33], int tx, int ty, int x,
-                                                    int c, int a0) {
-    const int k0 = 8 * ty;
-    if (a0 + k0 >= D.na) return;
-    float2 w[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) w[i] = s[k0 + i][tx];
-    const int bx = x >= D.hx, by = c >= D.hy;
-    const int lx = x - bx * D.hx, ly = c - by * D.hy, be = bx + 2 * by;
-    const u64 slice = u64(D.hy) * D.hx, inPlane = u64(ly) * D.hx + lx;
-    u16* const oddBase = D.symOut + u64(be + 3) * D.bandStride + inPlane;        // octant be + 4
-    u16* const evenSym = be ? D.symOut + u64(be - 1) * D.bandStride + inPlane     // octant be
-                            : D.lpSymOut + inPlane;                               // LLL, coarsest level
-    const bool evenFloat = be == 0 && !D.lastLevel;                              // LLL kept as floats
-    float* const evenF = D.dst + size_t(x) + size_t(c) * D.dc;
-    const float invEven = be ? D.inv : D.invLP;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int a = a0 + k0 + j;
-        if (a >= D.na) break;
-        const float2 r = (j & 1) ? fir9p<false, 1>(w + j) : fir9p<false, 0>(w + j);
-        const u64 lz = u64(a >> 1);
-        if (j & 1) {
-            const u32 s0 = symbolizeI(int(r.x * D.inv)) & 0xFFFFu, s1 = symbolizeI(int(r.y * D.inv)) & 0xFFFFu;
-            *reinterpret_cast<u32*>(oddBase + lz * slice) = s0 | (s1 << 16);
-        } else if (evenFloat) {
-            *reinterpret_cast<float2*>(evenF + size_t(a >> 1) * D.da) = r;
-        } else {
-            const u32 s0 = symbolizeI(int(r.x * invEven)) & 0xFFFFu, s1 = symbolizeI(int(r.y * invEven)) & 0xFFFFu;
-            *reinterpret_cast<u32*>(evenSym + lz * slice) = s0 | (s1 << 16);
-        }
+        *reinterpret_cast<float2*>(D.dst + size_t(x) + size_t(o) * D.da + size_t(c) * D.dc) = r;
     }
 }
 
@@ -1134,7 +1095,7 @@ __device__ __forceinline__ void colOutputs8Quantize(const BColDesc& D, const flo
 // set by the CTAs resident.
 static_assert(kBColTileX == 64, "a column-pass CTA has 32 threads of column pairs per row");
 
-template <bool kInverse, bool kSymbols, bool kQuantize>
+template <bool kInverse, bool kSymbols>
 __device__ __forceinline__ void colsTile(const BColDesc& D, u32 local) {
     __shared__ float2 s[kBColTileA + 8][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -1206,20 +1167,19 @@ __device__ __forceinline__ void colsTile(const BColDesc& D, u32 local) {
     for (int i = 0; i < kLoads; ++i) s[ty + 8 * i][tx] = vals[i];
     __syncthreads();
     if (x >= nx) return;
-    if (kQuantize && !(D.hx & 1) && 2 * D.hz == na) colOutputs8Quantize(D, s, tx, ty, x, c, a0);
-    else colOutputs8<kInverse, kQuantize, kSymbols || kQuantize>(D, s, tx, ty, x, c, a0);
+    colOutputs8<kInverse, kSymbols>(D, s, tx, ty, x, c, a0);
 }
 
-template <bool kInverse, bool kSymbols, bool kQuantize = false>
-__global__ void __launch_bounds__(256, kQuantize ? 4 : 6) k_bCols(const BColDesc* __restrict__ descs, const u32* __restrict__ map) {
+// The batch's inverse Z pass, from symbols.
+__global__ void __launch_bounds__(256, 6) k_bSymbolCols(const BColDesc* __restrict__ descs, const u32* __restrict__ map) {
     const BColDesc D = descs[map[blockIdx.x]];   // a copy: the output stores cannot alias it
-    colsTile<kInverse, kSymbols, kQuantize>(D, blockIdx.x - D.ctaOff);
+    colsTile<true, true>(D, blockIdx.x - D.ctaOff);
 }
 
-// The same pass of one volume, its descriptor a parameter (dwtFloat calls).
+// A column pass of one volume, its descriptor a parameter (dwtFloat calls).
 template <bool kInverse>
 __global__ void __launch_bounds__(256, 6) k_colsOne(const __grid_constant__ BColDesc D) {
-    colsTile<kInverse, false, false>(D, blockIdx.x);
+    colsTile<kInverse, false>(D, blockIdx.x);
 }
 
 // dwtFloat's passes over plain floats.  Rows: any pitch (rowsTile checks its
@@ -1258,6 +1218,218 @@ static void colPassFloat(float* dst, const float* src, int nx, int ny, int nz, i
     d.tilesX = u32(ceilDiv(nx, kBColTileX));
     d.tilesA = u32(ceilDiv(d.na, kBColTileA));
     k_colsOne<kInverse><<<d.tilesX * d.tilesA * u32(d.nc), dim3(32, 8), 0, st>>>(d);
+    countLaunch();
+}
+
+// Output j of a column pair from its window, and the eight outputs of a row
+// window, as scalar chains: their taps are immediates, where packed pairs need
+// every coefficient pair and every odd sample pair moved into registers; the
+// plane pass takes the same time and instructions with either.
+template <bool kInverse>
+__device__ __forceinline__ float2 firPair(const float2* w, int j) {
+    float a[9], b[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        a[i] = w[j + i].x;
+        b[i] = w[j + i].y;
+    }
+    return (j & 1) ? make_float2(fir9c<kInverse, 1>(a), fir9c<kInverse, 1>(b))
+                   : make_float2(fir9c<kInverse, 0>(a), fir9c<kInverse, 0>(b));
+}
+template <bool kInverse>
+__device__ __forceinline__ void firEight(const float* w, float* o) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        o[2 * p] = fir9c<kInverse, 0>(w + 2 * p);
+        o[2 * p + 1] = fir9c<kInverse, 1>(w + 2 * p + 1);
+    }
+}
+
+// A plane pass (BPlaneDesc): X and Y of one level in one read and one write of
+// the volume instead of two of each.  The staged tile is filtered in place:
+// every thread holds the window of its column pair (and, forward, of its row
+// groups) in registers when the barrier lets the outputs overwrite it.  The
+// taps and chains are those of rowsTile and colsTile, in their order, with the
+// intermediate rounded to float as there, so the results are bit-identical.
+// Bound: instruction issue (76% of the slots; 900 per thread for 14 outputs),
+// then DRAM.  256^3: the Y and X passes 54 us, this 44 - 52 before rows were
+// mirrored without branches and addressed by byte pitches.
+template <bool kInverse>
+__device__ __forceinline__ void planeTile(const BPlaneDesc& D, const float* __restrict__ src, float* __restrict__ dst,
+                                          u32 local) {
+    __shared__ __align__(16) float s[kPlaneFloats + 8 * (kPlaneTile + 12)];   // windows of ragged tiles read past their rows
+    const int tid = threadIdx.x;
+    const int xt = int(local % u32(D.tilesX)), rest = int(local / u32(D.tilesX));
+    const int yt = rest % D.tilesY, z0 = rest / D.tilesY * D.tz;
+    const int x0 = xt * D.tx, y0 = yt * D.ty;
+    const int W = min(D.tx, D.nx - x0), H = min(D.ty, D.ny - y0), Z = min(D.tz, D.nz - z0);
+    const int nx = D.nx, ny = D.ny, hn = nx >> 1, P = D.pitch;
+    const int rowsPer = H + 8, pw = (W + 8) >> 1;
+    {
+        // a thread keeps its column pair and takes every R-th staged row; all
+        // of its loads are issued before any is used
+        float2 v[kPlaneLoads];
+        const int R = kPlaneThreads / pw, j0 = quotient(tid, __frcp_rn(float(pw))), pr = tid - j0 * pw;
+        const int rows = j0 < R ? Z * rowsPer : 0;
+        // xa stays even and xb odd under the mirror (nx is even)
+        const int xa = mirrorIdx(x0 - 4 + 2 * pr, nx), xb = mirrorIdx(x0 - 3 + 2 * pr, nx);
+        const char* const pa = reinterpret_cast<const char*>(src + size_t(z0) * D.srcSlice + (kInverse ? xa >> 1 : xa));
+        const char* const pb =
+            reinterpret_cast<const char*>(src + size_t(z0) * D.srcSlice + (kInverse ? hn + (xb >> 1) : xb));
+        // byte pitches: an address is one multiply-add
+        const u32 rowB = 4u * u32(D.srcRow), sliceB = 4u * u32(D.srcSlice);
+        const int yLast = 2 * (ny - 1), hy = ny >> 1;
+        auto rowOf = [&](int y) {   // staged row y's row in the source (mirrored without a branch: -4 <= y <= ny + 3)
+            const int m = min(abs(y), yLast - abs(y));
+            return u32(kInverse ? (m >> 1) + ((m & 1) ? hy : 0) : m);
+        };
+        if (Z == 1) {
+#pragma unroll
+            for (int i = 0; i < kPlaneLoads; ++i) {
+                const int r = j0 + R * i;
+                v[i] = make_float2(0.0f, 0.0f);
+                if (r < rows) {
+                    const u64 off = u64(rowOf(y0 - 4 + r)) * rowB;
+                    v[i].x = *reinterpret_cast<const float*>(pa + off);
+                    v[i].y = *reinterpret_cast<const float*>(pb + off);
+                }
+            }
+        } else {
+            const float rRows = __frcp_rn(float(rowsPer));
+#pragma unroll
+            for (int i = 0; i < kPlaneLoads; ++i) {
+                const int r = j0 + R * i;
+                v[i] = make_float2(0.0f, 0.0f);
+                if (r < rows) {
+                    const int zz = quotient(r, rRows);
+                    const u64 off = u64(rowOf(y0 - 4 + r - zz * rowsPer)) * rowB + u64(u32(zz)) * sliceB;
+                    v[i].x = *reinterpret_cast<const float*>(pa + off);
+                    v[i].y = *reinterpret_cast<const float*>(pb + off);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kPlaneLoads; ++i) {
+            const int r = j0 + R * i;
+            if (r < rows) *reinterpret_cast<float2*>(s + r * P + 2 * pr) = v[i];
+        }
+    }
+    __syncthreads();
+    const int gx = (W + 7) >> 3, gy = (H + 7) >> 3;
+    if (kInverse) {
+        // Y in place: output row y of a slice at its staged row y
+        const int task = tid, perSlice = gy * pw;
+        const bool act = task < Z * perSlice;
+        const int zz = act && Z > 1 ? quotient(task, __frcp_rn(float(perSlice))) : 0, q = task - zz * perSlice;
+        const int g = act ? quotient(q, __frcp_rn(float(pw))) : 0, p = q - g * pw;
+        float* const col = s + (zz * rowsPer + 8 * g) * P + 2 * (act ? p : 0);
+        float2 w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) w[i] = *reinterpret_cast<const float2*>(col + i * P);
+        __syncthreads();
+        if (act) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (8 * g + j < H)
+                    *reinterpret_cast<float2*>(col + j * P) = firPair<true>(w, j);
+        }
+        __syncthreads();
+        const bool vec = D.vec && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+        const int perS = H * gx;
+        const float rPerS = __frcp_rn(float(perS)), rGx = __frcp_rn(float(gx));
+        for (int k = tid; k < Z * perS; k += kPlaneThreads) {
+            const int zq = Z > 1 ? quotient(k, rPerS) : 0, r = k - zq * perS, y = quotient(r, rGx), g8 = r - y * gx;
+            const float* w4 = s + (zq * rowsPer + y) * P + 8 * g8;
+            float wx[16];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float4 v = *reinterpret_cast<const float4*>(w4 + 4 * t);
+                wx[4 * t] = v.x; wx[4 * t + 1] = v.y; wx[4 * t + 2] = v.z; wx[4 * t + 3] = v.w;
+            }
+            float o[8];
+            firEight<true>(wx, o);
+            float* out = dst + size_t(z0 + zq) * D.dstSlice + size_t(y0 + y) * D.dstRow + x0 + 8 * g8;
+            if (vec) {
+                reinterpret_cast<float4*>(out)[0] = make_float4(o[0], o[1], o[2], o[3]);
+                reinterpret_cast<float4*>(out)[1] = make_float4(o[4], o[5], o[6], o[7]);
+            } else {
+#pragma unroll
+                for (int t = 0; t < 8; ++t)
+                    if (8 * g8 + t < W) out[t] = o[t];
+            }
+        }
+    } else {
+        // X in place: output x of a staged row at its column x; two groups per thread
+        float wx[2][16];
+        const int groups = Z * rowsPer * gx;
+        const float rGx = __frcp_rn(float(gx));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int k = tid + kPlaneThreads * i;
+            const int r = k < groups ? quotient(k, rGx) : 0, g8 = k < groups ? k - r * gx : 0;
+            const float* w4 = s + r * P + 8 * g8;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float4 v = *reinterpret_cast<const float4*>(w4 + 4 * t);
+                wx[i][4 * t] = v.x; wx[i][4 * t + 1] = v.y; wx[i][4 * t + 2] = v.z; wx[i][4 * t + 3] = v.w;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int k = tid + kPlaneThreads * i;
+            if (k < groups) {
+                const int r = quotient(k, rGx), g8 = k - r * gx;
+                float v[8];
+                firEight<false>(wx[i], v);
+                float4* o = reinterpret_cast<float4*>(s + r * P + 8 * g8);
+                o[0] = make_float4(v[0], v[1], v[2], v[3]);
+                o[1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        }
+        __syncthreads();
+        const int op = W >> 1, perSlice = gy * op;
+        const float rPer = __frcp_rn(float(perSlice)), rOp = __frcp_rn(float(op));
+        for (int k = tid; k < Z * perSlice; k += kPlaneThreads) {
+            const int zz = Z > 1 ? quotient(k, rPer) : 0, q = k - zz * perSlice, g = quotient(q, rOp), p = q - g * op;
+            const float* col = s + (zz * rowsPer + 8 * g) * P + 2 * p;
+            float2 w[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) w[i] = *reinterpret_cast<const float2*>(col + i * P);
+            float* out = dst + size_t(z0 + zz) * D.dstSlice + ((x0 >> 1) + p);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (8 * g + j >= H) break;
+                const float2 r = firPair<false>(w, j);
+                float* row = out + size_t(splitPos(y0 + 8 * g + j, ny)) * D.dstRow;
+                row[0] = r.x;
+                row[hn] = r.y;
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kPlaneThreads, 4) k_bPlanes(const BPlaneDesc* __restrict__ descs,
+                                                              const u32* __restrict__ map, float* const* outTab) {
+    const BPlaneDesc D = descs[map[blockIdx.x]];
+    planeTile<true>(D, D.src, D.dst ? D.dst : outTab[D.vol], blockIdx.x - D.ctaOff);
+}
+
+// The same pass of one volume, its descriptor a parameter (dwtFloat calls).
+template <bool kInverse>
+__global__ void __launch_bounds__(kPlaneThreads, 4) k_planesOne(const __grid_constant__ BPlaneDesc D) {
+    planeTile<kInverse>(D, D.src, D.dst, blockIdx.x);
+}
+
+template <bool kInverse>
+static void planePass(float* dst, const float* src, int nx, int ny, int nz, int srcRow, int srcSlice, int dstRow,
+                      int dstSlice, cudaStream_t st) {
+    BPlaneDesc d{};
+    d.src = src; d.dst = dst;
+    d.nx = nx; d.ny = ny; d.nz = nz;
+    d.srcRow = srcRow; d.srcSlice = srcSlice; d.dstRow = dstRow; d.dstSlice = dstSlice;
+    const u32 ctas = batchPlanePlan(d);
+    k_planesOne<kInverse><<<ctas, kPlaneThreads, 0, st>>>(d);
     countLaunch();
 }
 
@@ -1574,22 +1746,15 @@ void launchBatchLevelFwd(const BLevelDesc* d, const u32* map, u32 ctas, const fl
     countLaunch();
 }
 
-void launchBatchRows(const BRowDesc* d, const u32* map, u32 ctas, bool inverse, const float* const* inTab,
-                     float* const* outTab, cudaStream_t st) {
+void launchBatchSymbolCols(const BColDesc* d, const u32* map, u32 ctas, cudaStream_t st) {
     if (!ctas) return;
-    if (inverse) k_bRows<true><<<ctas, 256, 0, st>>>(d, map, inTab, outTab);
-    else k_bRows<false><<<ctas, 256, 0, st>>>(d, map, inTab, outTab);
+    k_bSymbolCols<<<ctas, dim3(32, 8), 0, st>>>(d, map);
     countLaunch();
 }
 
-void launchBatchCols(const BColDesc* d, const u32* map, u32 ctas, bool inverse, bool fromSymbols, cudaStream_t st,
-                     bool quantizeStore) {
+void launchBatchPlanes(const BPlaneDesc* d, const u32* map, u32 ctas, float* const* outTab, cudaStream_t st) {
     if (!ctas) return;
-    const dim3 blk(32, 8);
-    if (quantizeStore) k_bCols<false, false, true><<<ctas, blk, 0, st>>>(d, map);
-    else if (fromSymbols) k_bCols<true, true><<<ctas, blk, 0, st>>>(d, map);
-    else if (inverse) k_bCols<true, false><<<ctas, blk, 0, st>>>(d, map);
-    else k_bCols<false, false><<<ctas, blk, 0, st>>>(d, map);
+    k_bPlanes<<<ctas, kPlaneThreads, 0, st>>>(d, map, outTab);
     countLaunch();
 }
 
@@ -1789,9 +1954,8 @@ int cc_dwt_float_forward_static(float* dst, const float* src, int sx, int sy, in
     float* buf2 = scratch + kStaticScratchFloats;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool do3D = sz > 1;
-    forwardRows<float>(buf1, src, sx, sy, sz, ch, srcRow, srcSlice, dstRow, dstSlice, st);
     float* yDst = do3D ? buf2 : dst;
-    floatCols<false>(yDst, buf1, sx, sy, sz, 1, dstRow, dstSlice, st);
+    forwardPlane<float>(yDst, buf1, src, sx, sy, sz, ch, srcRow, srcSlice, dstRow, dstSlice, st);
     if (do3D) floatCols<false>(dst, buf2, sx, sy, sz, 2, dstRow, dstSlice, st);
     CC_TRY_CUDA(cudaGetLastError(), "dwtFloatForwardStatic");
     return CC_OK;

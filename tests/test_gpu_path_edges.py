@@ -1,0 +1,237 @@
+"""Edges of the kernels' size, alignment and length rules, each against the
+oracle, bit for bit: tile borders of the transform passes, sources and streams
+at odd addresses, code words longer than the staged window, and symbol tables
+on both sides of each builder's capacity."""
+import numpy as np
+import pytest
+
+from helpers import Oracle, symbol_streams
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+import cudacompress_b200 as cc  # noqa: E402
+from cudacompress_b200 import fields  # noqa: E402
+
+
+@pytest.fixture(scope="module")
+def oracle():
+    return Oracle()
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def host(t):
+    torch.cuda.synchronize()
+    return t.cpu().numpy()
+
+
+def same(a, b):
+    return a.shape == b.shape and np.ascontiguousarray(a).tobytes() == np.ascontiguousarray(b).tobytes()
+
+
+def pitched(a, row, rows, shift):
+    """A device copy of `a` (z, y, x) whose rows are `row` and slices
+    `row * rows` elements apart, its first element `shift` past an aligned
+    address.  Returns (view to pass on, function reading it back)."""
+    nz, ny, nx = a.shape
+    base = torch.zeros(nz * row * rows + shift, dtype=torch.from_numpy(a[:1, :1, :1]).dtype, device="cuda")
+    view = base[shift:].view(nz, rows, row)
+    view[:, :ny, :nx] = dev(a)
+    return view, lambda: host(view[:, :ny, :nx])
+
+
+# ------------------------------------------------------------- transforms
+# The plane pass works on tiles of 64 x 64 outputs: one below, at and above a
+# tile in x and y, the smallest level, several tiles, and the 2D form.
+FLOAT_SHAPES = [(8, 8, 8), (8, 10, 12), (8, 62, 64), (10, 66, 62), (8, 64, 66), (12, 72, 136), (8, 8, 130), (8, 130, 8),
+                (1, 8, 8), (1, 66, 130), (1, 128, 64), (66, 8, 10)]
+
+
+@pytest.mark.parametrize("shape", FLOAT_SHAPES)
+@pytest.mark.parametrize("pad,shift", [(0, 0), (1, 0), (2, 2), (4, 1)])
+def test_float_transform_at_tile_edges(oracle, shape, pad, shift):
+    """Both directions, with rows padded by `pad` elements and arrays starting
+    `shift` elements past an aligned address."""
+    rng = np.random.default_rng(sum(shape) + pad)
+    a = rng.standard_normal(shape).astype(np.float32)
+    nz, ny, nx = shape
+    row, rows = nx + pad, ny + (1 if pad else 0)
+    pitches = (row, row * rows, row, row * rows)
+    zero = np.zeros_like(a)
+    src, _ = pitched(a, row, rows, shift)
+    dst, read = pitched(zero, row, rows, shift)
+    b1, _ = pitched(zero, row, rows, shift)
+    b2, _ = pitched(zero, row, rows, shift)
+    cc.dwt_float_forward(dst, b2, b1, src, nx, ny, nz, 1, *pitches)
+    fwd = read()
+    assert same(fwd, oracle.dwt_float(a))
+    back, read_back = pitched(zero, row, rows, shift)
+    cc.dwt_float_inverse(back, b2, b1, dst, nx, ny, nz, 1, *pitches)
+    assert same(read_back(), oracle.dwt_float(fwd, inverse=True))
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 8), (1, 66, 130), (1, 200, 72)])
+def test_float_transform_in_place_2d(oracle, shape):
+    """A 2D transform whose destination is its source: tiles overlap their
+    neighbours' inputs, so it goes through the buffer."""
+    rng = np.random.default_rng(3)
+    a = rng.standard_normal(shape).astype(np.float32)
+    _, ny, nx = shape
+    t, b1, b2 = dev(a), dev(np.zeros_like(a)), dev(np.zeros_like(a))
+    cc.dwt_float_forward(t, b2, b1, t, nx, ny, 1)
+    fwd = host(t)
+    assert same(fwd, oracle.dwt_float(a))
+    cc.dwt_float_inverse(t, b2, b1, t, nx, ny, 1)
+    assert same(host(t), oracle.dwt_float(fwd, inverse=True))
+
+
+@pytest.mark.parametrize("shape", [(8, 8, 8), (1, 8, 8), (8, 10, 12), (1, 34, 66), (1, 66, 258), (10, 66, 34), (34, 8, 8),
+                                   (1, 258, 520)])
+@pytest.mark.parametrize("pad,shift", [(0, 0), (1, 1), (2, 2), (4, 4)])
+def test_int_transform_at_tile_edges(oracle, shape, pad, shift):
+    rng = np.random.default_rng(sum(shape) + pad)
+    a = rng.integers(-2000, 8000, shape).astype(np.int16)
+    nz, ny, nx = shape
+    row, rows = nx + pad, ny + (1 if pad else 0)
+    pitches = (row, row * rows, row, row * rows)
+    zero = np.zeros_like(a)
+    src, _ = pitched(a, row, rows, shift)
+    dst, read = pitched(zero, row, rows, shift)
+    buf, _ = pitched(zero, row, rows, shift)
+    cc.dwt_int_forward(dst, buf, src, nx, ny, nz, *pitches)
+    assert same(read(), oracle.dwt_int(a))
+    back, read_back = pitched(zero, row, rows, shift)
+    cc.dwt_int_inverse(back, buf, dst, nx, ny, nz, *pitches)
+    assert same(read_back(), a)
+
+
+@pytest.mark.parametrize("shape,levels", [((20, 28), 1), ((16, 16), 1), ((40, 24), 2), ((64, 136), 2), ((66, 260), 1)])
+def test_heightfield_sizes(oracle, shape, levels):
+    """Band widths that are and are not multiples of four symbols."""
+    img = np.ascontiguousarray(fields.fbm_heightfield(512, seed=31)[: shape[0], : shape[1]])
+    n = max(4096, img.size)
+    with cc.Instance(0, 3, n, 128, 14) as inst:
+        words, bits = cc.compress_heightfield(inst, dev(img), levels)
+        ref_words, ref_bits = oracle.compress_heightfield(img, levels)
+        assert bits == ref_bits
+        assert np.array_equal(host(words)[: (bits + 31) // 32].view(np.uint32), ref_words)
+        out = torch.zeros(shape, dtype=torch.int16, device="cuda")
+        cc.decompress_heightfield(inst, out, levels, words, bits)
+        assert np.array_equal(host(out), img)
+
+
+@pytest.mark.parametrize("z_chunk", [0, 8, 12, 32, 64])
+@pytest.mark.parametrize("shape", [(16, 16, 16), (48, 80, 136), (144, 32, 32)])
+def test_forward_level_depths(oracle, z_chunk, shape):
+    """The forward level's tile depth, chosen by the rule (0) or given, does
+    not show in the streams; levels smaller and larger than a tile."""
+    vol = np.ascontiguousarray(fields.turbulence_field(144, 256, 36, seed=77)[: shape[0], : shape[1], : shape[2]])
+    ref_words, ref_bits = oracle.compress_volume(vol, 1, 0.01)
+    ref = oracle.decompress_volume(ref_words, ref_bits, shape, 1, 0.01)
+    with cc.Instance(0, 8, vol.size, 128, 14) as inst, \
+            cc.VolumeBatch(inst, [shape], 1, [0.01], z_chunk=z_chunk) as batch:
+        batch.compress([dev(vol)])
+        words, bits = batch.read_stream(0)
+        assert bits == ref_bits and np.array_equal(words, ref_words)
+        out = torch.zeros(shape, dtype=torch.float32, device="cuda")
+        batch.decompress([out])
+        batch.status()
+        assert same(host(out), ref)
+
+
+# ---------------------------------------------------------- entropy coder
+def roundtrip(oracle, inst, kind, streams, cb=128, log2max=14, shift=0):
+    """Encodes views `shift` elements into larger buffers, compares with the
+    oracle, decodes the oracle's words into such views."""
+    S, n = streams.shape
+    signed, tsigned = (np.int16, torch.int16) if streams.dtype == np.uint16 else (np.int32, torch.int32)
+    pitch = (n + 16) // 8 * 8
+    buf = torch.zeros(S * pitch + 16, dtype=tsigned, device="cuda")
+    views = [buf[i * pitch + shift: i * pitch + shift + n] for i in range(S)]
+    for v, s in zip(views, streams):
+        v.copy_(dev(s.view(signed)))
+    bs = cc.BitStream()
+    enc, dec = (cc.encode_rlhuff, cc.decode_rlhuff) if kind == 0 else (cc.encode_huff, cc.decode_huff)
+    assert enc(inst, bs, views, n), cc.last_error()
+    words, bits, _ = oracle.encode(kind, streams, cb=cb, log2max=log2max)
+    assert bs.bit_size == bits
+    assert np.array_equal(bs.raw(), words)
+    buf.fill_(-1)
+    assert dec(inst, cc.BitStream(words, bits), views, n), cc.last_error()
+    assert cc.decode_status(inst) == 0
+    for v, s in zip(views, streams):
+        assert np.array_equal(host(v).view(streams.dtype), s)
+    guard = torch.ones_like(buf, dtype=torch.bool)
+    for i in range(S):
+        guard[i * pitch + shift: i * pitch + shift + n] = False
+    assert bool((buf[guard] == -1).all())
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+@pytest.mark.parametrize("n", [31, 33, 1023, 1025, 4097, 20011])
+def test_streams_at_odd_addresses(oracle, kind, shift, n):
+    """Symbol arrays aligned to 16, 2 and 8 bytes; lengths around a lane's
+    group, a warp's and a block's tile."""
+    with cc.Instance(0, 3, 20011, 128, 14) as inst:
+        roundtrip(oracle, inst, kind, symbol_streams("laplace", 3, n, seed=n), shift=shift)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("cb", [32, 64, 128, 256])
+@pytest.mark.parametrize("n", [3000, 40000])
+def test_code_words_longer_than_the_staged_window(oracle, kind, cb, n):
+    """One stream of near-uniform symbols over the whole alphabet (13 to 14
+    bits each: read from global memory), one whose second half is sparse (a
+    stream with both kinds of warps), one of zeros (no code words)."""
+    rng = np.random.default_rng(cb + n)
+    streams = np.zeros((3, n), np.uint16)
+    streams[0] = rng.integers(1, 1 << 14, n)
+    streams[1, : n // 2] = rng.integers(1, 1 << 14, n // 2)
+    streams[1, n // 2:] = (rng.random(n - n // 2) < 0.05) * 3
+    with cc.Instance(0, 3, n, cb, 14) as inst:
+        roundtrip(oracle, inst, kind, streams, cb=cb)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("leaves", [256, 257, 1024, 1025, 2048, 2049, 12287, 12288, 12289, 16383])
+@pytest.mark.parametrize("S", [1, 33])
+def test_table_sizes_around_each_builder(oracle, kind, leaves, S):
+    """A stream of exactly `leaves` distinct symbols, alone (one call's few
+    tables) and with small ones (the tiers by leaf count)."""
+    rng = np.random.default_rng(leaves)
+    n = 20000
+    streams = symbol_streams("laplace", S, n, seed=leaves)
+    v = rng.permutation(np.concatenate([np.arange(1, leaves + 1), rng.integers(1, leaves + 1, n - leaves)]))
+    streams[S // 2] = v
+    assert len(np.unique(streams[S // 2])) == leaves
+    with cc.Instance(0, S, n, 128, 14) as inst:
+        roundtrip(oracle, inst, kind, streams)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("S", [1, 31, 32, 33, 63, 64, 65, 130])
+@pytest.mark.parametrize("cb", [32, 128])
+def test_stream_counts_around_the_plans(oracle, kind, S, cb):
+    """Stream and table counts on both sides of the one-CTA plans' 64."""
+    with cc.Instance(0, S, 5000, cb, 14) as inst:
+        roundtrip(oracle, inst, kind, symbol_streams("sparse", S, 4675, seed=S), cb=cb)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("n", [33, 4097, 20000])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_wide_symbols(oracle, kind, n, shift):
+    """32-bit symbols of a 20-bit alphabet, dense and sparse, at 16- and
+    4-byte aligned addresses."""
+    rng = np.random.default_rng(n)
+    streams = rng.integers(0, 1 << 19, (2, n)).astype(np.uint32)
+    streams[1] *= rng.random(n) < 0.2
+    with cc.Instance(0, 2, 20000, 128, 20) as inst:
+        roundtrip(oracle, inst, kind, streams, log2max=20, shift=shift)
