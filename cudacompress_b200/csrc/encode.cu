@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
 // Table construction: one block per table, all tables of the call at once.
 // Leaf gathering, depths, the sort (an exact warp-parallel replay of
 // std::sort), canonical codes and serialization are block parallel; the heap
-// merge runs in one thread on shared memory (table_build.cuh).  Tables with
+// merge runs on one warp in shared memory (table_build.cuh).  Tables with
 // more leaves than the shared-memory builder holds run sequentially on
 // global memory (huffman_build.cuh).
 // ---------------------------------------------------------------------------
@@ -757,13 +757,15 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     if (es.kind == KIND_RLHUFF)
         for (u32 s = es.groupFirst + threadIdx.x; s < es.groupFirst + es.groupSize; s += kThreads)
             if (p.counts[s]) atomicAnd(&sAllEmpty, 0u);
-    u32 localMax = 0;
-    bool any = false;
-    for (u32 b = threadIdx.x; b < meta.histSize; b += kThreads)
-        if (hist[b]) { localMax = b; any = true; }
-    if (any) atomicMax(&sMax, localMax);
+    if (kThreads > 32) {
+        u32 localMax = 0;
+        bool any = false;
+        for (u32 b = threadIdx.x; b < meta.histSize; b += kThreads)
+            if (hist[b]) { localMax = b; any = true; }
+        if (any) atomicMax(&sMax, localMax);
+    }
     __syncthreads();
-    const u32 symbolMax = count ? sMax : 0u;
+    u32 symbolMax = count ? sMax : 0u;   // kThreads == 32: with the leaves, below
     // Histogram.cu:117-121: with every stream of the reference call empty the
     // reference builds its tables from stale arena words; for zero-count table
     // i that word is the low half of a device pointer when 2+2i < S (nonzero),
@@ -777,7 +779,7 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     u32* heapP = reinterpret_cast<u32*>(dyn);
     u32* heapI = reinterpret_cast<u32*>(dyn + At::kIds);
     const u16* parentS = reinterpret_cast<const u16*>(dyn + At::kParents);
-    u32* orderS = heapP;   // takes the probabilities' place after the merge
+    u32* orderS = heapP;   // takes the probabilities' place after the merge, sorted the ids'
     const u32 smemLeaves = count < hm::kInf - 1u ? kCap : 0u;
     u32 L;
     if (quirkLeaf) {
@@ -790,6 +792,31 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     } else if (count == 0) {
         L = 0;
         if (L < p.buildLo || L > p.buildHi) return;
+    } else if (kThreads == 32) {
+        // one warp: largest symbol and leaves in one pass, 32 bins at a time
+        const u32 below = (1u << threadIdx.x) - 1u;
+        L = 0;
+        u32 next = threadIdx.x < meta.histSize ? hist[threadIdx.x] : 0u;
+        for (u32 base = 0; base < meta.histSize; base += 32) {
+            const u32 b = base + threadIdx.x;
+            u32 h = next;
+            next = b + 32u < meta.histSize ? hist[b + 32u] : 0u;   // in flight over this step's stores
+            const u32 m = __ballot_sync(0xffffffffu, h != 0);
+            if (h) {
+                const u32 off = L + __popc(m & below);
+                if (p.symBytes == 2 && p.bins == 65536u && b == 65535u) h += count & 1u;   // as below
+                leafSym[off] = b;
+                if (!smemLeaves) {
+                    heapG[off] = (u64(h) << 32) | off;
+                } else if (off < kCap) {
+                    heapP[off + 1] = h;
+                    heapI[off + 1] = 2u * off;
+                }
+            }
+            if (m) symbolMax = base + 31u - u32(__clz(int(m)));
+            L += __popc(m);
+        }
+        if (L < p.buildLo || L > p.buildHi) return;   // at most kCap leaves (k_leafTiers)
     } else {
         const u32 nb = symbolMax + 1;
         const u32 per = (nb + kThreads - 1) / kThreads;
@@ -838,8 +865,9 @@ __device__ void buildTable(const EncParams& p, u32 t) {
             // the ids' and the tails' places
             u16* lList = reinterpret_cast<u16*>(heapI);
             u16* rList = lList + kCap;
-            u8* mark = dyn + At::kTails;
-            tb::blockIntrosort<kThreads>(order, int(L), lList, rList, mark, sSegA, sSegB, sSegCount);
+            u32* seg = reinterpret_cast<u32*>(dyn + At::kTails);
+            tb::blockIntrosort<kThreads>(orderS, int(L), lList, rList, seg, sSegA, sSegB, sSegCount, heapI);
+            order = heapI;
         }
     } else if (threadIdx.x == 0) {
         // tables larger than the shared-memory builder: sequential, global memory
@@ -860,8 +888,7 @@ __device__ void buildTable(const EncParams& p, u32 t) {
         if (maxLen <= 31) hb::introsort(order, int(L), hb::LenLess());
         sMaxLen = maxLen;
     }
-    if (threadIdx.x == 0)
-        for (int l = 0; l < 32; ++l) lenCount[l] = 0;
+    if (threadIdx.x < 32) lenCount[threadIdx.x] = 0;
     __syncthreads();
     const u32 maxLen = sMaxLen;
     if (maxLen > 31) {
@@ -874,15 +901,22 @@ __device__ void buildTable(const EncParams& p, u32 t) {
         if (len) atomicAdd(&lenCount[len - 1], 1u);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        u32 idx = 0, code = 0;
-        for (u32 l = 1; l <= 32; ++l) {
-            firstIndex[l] = idx;
-            firstCode[l] = code;
-            u32 c = l <= 31 ? lenCount[l - 1] : 0u;
-            idx += c;
-            code = (code + c) << 1;
+    // first index and code of every length l: index[l + 1] = index[l] + c[l],
+    // code[l + 1] = 2 (code[l] + c[l]), scanned over the lanes (lane l - 1)
+    if (threadIdx.x < 32) {
+        const u32 c = lenCount[threadIdx.x];   // none of length 32
+        u32 idx = c, code = c;
+#pragma unroll
+        for (u32 d = 1; d < 32; d <<= 1) {
+            const u32 i = __shfl_up_sync(0xffffffffu, idx, d), k = __shfl_up_sync(0xffffffffu, code, d);
+            if (threadIdx.x >= d) {
+                idx += i;
+                code += k << d;
+            }
         }
+        code = __shfl_up_sync(0xffffffffu, code, 1) << 1;
+        firstIndex[threadIdx.x + 1] = idx - c;
+        firstCode[threadIdx.x + 1] = threadIdx.x ? code : 0u;
     }
     __syncthreads();
     uint2* enc = p.enc + meta.histOff;
@@ -901,12 +935,11 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     const u32 hdrWords = u32(ceilDiv(headerBits, 32));
     for (u32 w = threadIdx.x; w < hdrWords; w += kThreads) hdr[w] = 0;
     __syncthreads();
+    if (threadIdx.x < maxLen) putBits(hdr, 5 + threadIdx.x * p.log2Max, lenCount[threadIdx.x], p.log2Max);
     if (threadIdx.x == 0) {
-        u32 pos = 0;
-        putBits(hdr, pos, maxLen, 5); pos += 5;
-        for (u32 l = 0; l < maxLen; ++l) { putBits(hdr, pos, lenCount[l], p.log2Max); pos += p.log2Max; }
-        putBits(hdr, pos, L, p.log2Max); pos += p.log2Max;
-        putBits(hdr, pos, symbolBits, longSym ? 5 : 4);
+        putBits(hdr, 0, maxLen, 5);
+        putBits(hdr, 5 + maxLen * p.log2Max, L, p.log2Max);
+        putBits(hdr, 5 + (maxLen + 1) * p.log2Max, symbolBits, longSym ? 5 : 4);
     }
     for (u32 k = threadIdx.x; k < L; k += kThreads)
         putBits(hdr, fixedBits + k * symbolBits, leafSym[order[k] & hb::kLeafMask], symbolBits);
