@@ -23,7 +23,7 @@ namespace ccb {
 enum CodecKind : int { KIND_RLHUFF = 0, KIND_HUFF = 1 };
 
 // Tile of the run-length passes: 256 threads x 8 symbols.
-constexpr u32 kRleThreads = 256;
+constexpr u32 kRleThreads = 128;
 constexpr u32 kRlePerThread = 32;
 constexpr u32 kRleTile = kRleThreads * kRlePerThread;
 // The Huffman block kernels take coding blocks in runs of kRunSymbols symbols

@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
     const TableMeta mS = p.meta[sd.tableFirst];
     const u32 smemBins = min(mS.histSize, kWriteSymBins);
     for (u32 i = threadIdx.x; i < smemBins; i += kRleThreads) hSym[i] = 0;
-    hZc[threadIdx.x] = 0;
+    for (u32 i = threadIdx.x; i < 256u; i += kRleThreads) hZc[i] = 0;
     const Sym* in = reinterpret_cast<const Sym*>(sd.in);
     const u32 wbase = (tile - sd.tileOff) * kRleTile + warp * 1024u;
     u32 mUnused;
@@ -702,7 +702,8 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
     __syncthreads();
     for (u32 i = threadIdx.x; i < smemBins; i += kRleThreads)
         if (hSym[i]) atomicAdd(gSym + i, hSym[i]);
-    if (threadIdx.x < mZ.histSize && hZc[threadIdx.x]) atomicAdd(gZc + threadIdx.x, hZc[threadIdx.x]);
+    for (u32 i = threadIdx.x; i < min(mZ.histSize, 256u); i += kRleThreads)
+        if (hZc[i]) atomicAdd(gZc + i, hZc[i]);
 }
 
 // ---------------------------------------------------------------------------
