@@ -12,7 +12,7 @@
 // kernel covers the batch and all Huffman tables are built concurrently.
 // Launch sequence (no host round trip until the result is read):
 //   summary -> scan -> histPlan -> zeroHist -> write(+histograms)
-//   -> tableBuild -> blockBits -> blockScan -> layout -> pack -> headers
+//   -> tableBuild -> blockBits -> blockScan -> layout -> pack (with the headers)
 #include <cstring>
 
 #include "capi_internal.cuh"
@@ -39,7 +39,7 @@ struct EncParams {
     u32* blockBits;
     u32* blockOff;
     u32* runTable;    // [runs] table of each run of coding blocks (k_planFill)
-    u32* tileStream;  // [totalTiles] stream of each run-length tile (k_lookupMaps)
+    u32* tileStream;  // [totalTiles] stream of each run-length tile (k_encBegin)
     SegmentLayout* layout;
     u32* out;
     u64 outWordsMax;
@@ -70,7 +70,7 @@ __device__ __forceinline__ bool warpFailed(const EncParams& p) {
     return __any_sync(0xffffffffu, *reinterpret_cast<volatile const u32*>(p.errors) != 0);
 }
 
-// Stream owning run-length tile `tile`: one load from the map k_lookupMaps
+// Stream owning run-length tile `tile`: one load from the map k_encBegin
 // writes at the start of a call.
 __device__ __forceinline__ u32 streamOfTile(const EncParams& p, u32 tile) { return p.tileStream[tile]; }
 
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(256) k_leafTiers(EncParams p) {
 // entries directly.  Bound: instruction issue; walking a group's nonzeros on
 // its lane instead of a group's lanes together took three 256^3 streams'
 // highpass bands (50 million symbols, 26 million entries) from 191 to 123 us.
-constexpr u32 kWriteSymBins = 2048;   // symbol bins counted in shared memory by k_write
+constexpr u32 kWriteSymBins = 1024;   // symbol bins counted in shared memory by k_write (4 KB: twelve tiles per SM, not ten)
 
 template <class Sym>
 constexpr u32 writeStage() { return sizeof(Sym) == 2 ? kRleTile + kRleTile / 256u : kRleTile / 2u; }
