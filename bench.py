@@ -420,7 +420,7 @@ SECTION_UNITS = {
     "batch.dwt_forward": "per level (one fused k_bLevelFwd launch): the level's input read once (4 B/voxel) and "
                          "its outputs written once: 7 highpass octants as 2-byte symbols, the lowpass octant as "
                          "float (4 B) or, at the coarsest level, as 2-byte symbols",
-    "batch.dwt_inverse": "per level (three launches: k_bCols from symbols, k_bCols, k_bRows): the level's inputs "
+    "batch.dwt_inverse": "per level (two launches: k_bSymbolCols, k_bPlanes): the level's inputs "
                          "read once (2 B/highpass symbol, 4 B/lowpass voxel) and its output written once "
                          "(4 B/voxel); the intermediate passes' traffic is not credited",
 }
