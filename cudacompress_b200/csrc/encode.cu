@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(256) k_leafTiers(EncParams p) {
 // entries directly.  Bound: instruction issue; walking a group's nonzeros on
 // its lane instead of a group's lanes together took three 256^3 streams'
 // highpass bands (50 million symbols, 26 million entries) from 191 to 123 us.
-constexpr u32 kWriteSymBins = 1024;   // symbol bins counted in shared memory by k_write (4 KB: twelve tiles per SM, not ten)
+constexpr u32 kWriteSymBins = 1024;   // symbol bins counted in shared memory by k_write (4 KB: eleven tiles per SM, not nine)
 
 template <class Sym>
 constexpr u32 writeStage() { return sizeof(Sym) == 2 ? kRleTile + kRleTile / 256u : kRleTile / 2u; }
@@ -955,6 +955,8 @@ __device__ void buildTable(const EncParams& p, u32 t) {
 }
 
 // One table per CTA (kBuildEach), or the CTAs walk the list of one tier.
+// Bounding the one-warp tier to 72 registers (28 CTAs per SM instead of 20)
+// left 4096 bricks at the same time.
 template <u32 kThreads, u32 kCap>
 __global__ void __launch_bounds__(kThreads, 1) k_tableBuild(EncParams p) {
     if (p.buildTier == kBuildEach) {

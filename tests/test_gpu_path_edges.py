@@ -183,6 +183,17 @@ def test_streams_at_odd_addresses(oracle, kind, shift, n):
         roundtrip(oracle, inst, kind, symbol_streams("laplace", 3, n, seed=n), shift=shift)
 
 
+@pytest.mark.parametrize("n", [31 * 2048 + 1, 32 * 2048, 32 * 2048 + 1, 130 * 2048 + 77])
+def test_streams_around_a_step_of_the_tile_scan(oracle, n):
+    """32 run-length tiles of 2048 symbols are one step of a stream's scan;
+    the third stream's only nonzero is its last symbol."""
+    streams = symbol_streams("sparse", 3, n, seed=n)
+    streams[2] = 0
+    streams[2, -1] = 3
+    with cc.Instance(0, 3, n, 128, 14) as inst:
+        roundtrip(oracle, inst, 0, streams)
+
+
 @pytest.mark.parametrize("kind", [0, 1])
 @pytest.mark.parametrize("cb", [32, 64, 128, 256])
 @pytest.mark.parametrize("n", [3000, 40000])
