@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kDecThreads) k_decTables(DecParams p) {
     __shared__ int sFirst[32], sMin[32], sMax[32];
     __shared__ u32 sLim[kLutBits + 1];
     __shared__ u32 sScan[40];
-    __shared__ u32 sCarry, sFail;
+    __shared__ u32 sCarry, sFail, sUsable;   // sUsable: written once, before the barrier that publishes it
     const u32 t = blockIdx.x;
     if (threadIdx.x == 0) sFail = capacityFailed(p) ? 1u : 0u;
     __syncthreads();
@@ -369,10 +369,11 @@ __global__ void __launch_bounds__(kDecThreads) k_decTables(DecParams p) {
         if (d.nLen == 0) ok = ok && d.nSym <= 1;
         else ok = ok && total == d.nSym;
         if (!ok) atomicOr(p.errors, DEV_ERR_CORRUPT);
-        sCarry = ok ? 1u : 0u;
+        sUsable = ok ? 1u : 0u;
+        sCarry = 0;
     }
     __syncthreads();
-    if (!sCarry) {
+    if (!sUsable) {
         if (threadIdx.x == 0) D->nSym = 0xFFFFFFFFu;   // marks the table unusable
         return;
     }
@@ -407,7 +408,6 @@ __global__ void __launch_bounds__(kDecThreads) k_decTables(DecParams p) {
         D->nSym = d.nSym;
         const u32 v0 = d.nSym >= 1 ? ws.bits(symBit, d.symbolBits) : 0u;
         D->single = p.symBytes == 2 ? (v0 & 0xFFFFu) : v0;
-        sCarry = 0;
     }
     // absolute block offsets: inclusive prefix of the u16 increments
     // (PackInc.cu:220-229), eight blocks (four words) per thread per step

@@ -246,3 +246,25 @@ def test_wide_symbols(oracle, kind, n, shift):
     streams[1] *= rng.random(n) < 0.2
     with cc.Instance(0, 2, 20000, 128, 20) as inst:
         roundtrip(oracle, inst, kind, streams, log2max=20, shift=shift)
+
+
+@pytest.mark.parametrize("kind,S", [(0, 7), (0, 296), (0, 297), (1, 1), (1, 592), (1, 593)])
+def test_wide_symbol_tables_of_many_streams(oracle, kind, S):
+    """Decode tables of 32-bit symbols, whose table kernel has no barrier
+    between the symbols and the block offsets: both CTA widths (up to 592
+    tables and more), tables of one leaf to hundreds, several times over.
+    No warp may miss its share of a table: a guard reads the table's state
+    while another warp goes on to its block offsets."""
+    rng = np.random.default_rng(S)
+    n = 700
+    streams = (rng.integers(0, 1 << 18, (S, n)) * (rng.random((S, n)) < rng.random((S, 1)))).astype(np.uint32)
+    streams[0] = 5
+    with cc.Instance(0, S, n, 32, 18) as inst:
+        words, bits, _ = oracle.encode(kind, streams, cb=32, log2max=18)
+        outs = torch.empty((S, n + 4), dtype=torch.int32, device="cuda")
+        dec = cc.decode_rlhuff if kind == 0 else cc.decode_huff
+        for _ in range(8):
+            outs.fill_(-1)
+            assert dec(inst, cc.BitStream(words, bits), [outs[i, :n] for i in range(S)], n), cc.last_error()
+            assert cc.decode_status(inst) == 0
+            assert np.array_equal(host(outs[:, :n]).view(np.uint32), streams)
