@@ -431,6 +431,51 @@ __global__ void __launch_bounds__(128) k_liftCols(i16* __restrict__ dst, const i
     }
 }
 
+// A pass whose source and destination share memory (in-place calls): a CTA
+// stages `lines` whole lines in shared memory behind a barrier before it
+// stores any sample of them.  k_liftRows and k_liftCols keep their windows in
+// registers and would read what their neighbours have stored.  Lines run over
+// the fastest coordinate that is not the axis; alongAxis: the axis is the
+// contiguous one.
+constexpr int kLineSamples = 24576;   // 48 KB
+
+template <bool kInverse>
+__global__ void __launch_bounds__(256) k_liftLines(i16* dst, const i16* src, int nLines, int na, int liftEnd, int lines,
+                                                   bool alongAxis, int sLine, int sAxis, int sOther, int dLine,
+                                                   int dAxis, int dOther) {
+    __shared__ i16 s[kLineSamples];
+    const int l0 = int(blockIdx.x) * lines, nl = min(lines, nLines - l0), hn = na >> 1;
+    const size_t c = blockIdx.y;
+    for (int e = threadIdx.x; e < nl * na; e += 256) {
+        const int l = alongAxis ? e / na : e % nl, k = alongAxis ? e % na : e / nl;
+        // sample order, the [L|H] halves interleaved
+        const int at = !kInverse ? k : k < hn ? 2 * k : 2 * (k - hn) + 1;
+        s[l * na + at] = src[size_t(l0 + l) * sLine + size_t(k) * sAxis + c * sOther];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nl * hn; e += 256) {
+        const int l = alongAxis ? e / hn : e % nl, i = alongAxis ? e % hn : e / nl;
+        const i16* line = s + l * na;
+        auto at = [&](int k) { return line[mirrorIdx(k, na)]; };
+        // the lifted sample of an odd (forward) or even (inverse) position
+        auto first = [&](int k) {
+            const i16 v = at(k);
+            if (mirrorIdx(k, na) >= liftEnd) return v;
+            return kInverse ? unupdate(v, at(k - 1), at(k + 1)) : predict(v, at(k - 1), at(k + 1));
+        };
+        i16* out = dst + size_t(l0 + l) * dLine + c * dOther;
+        if (!kInverse) {
+            const i16 h0 = first(2 * i - 1), h1 = first(2 * i + 1);
+            out[size_t(i) * dAxis] = 2 * i < liftEnd ? update(line[2 * i], h0, h1) : line[2 * i];
+            out[size_t(hn + i) * dAxis] = h1;
+        } else {
+            const i16 a0 = first(2 * i), a1 = first(2 * i + 2);
+            out[size_t(2 * i) * dAxis] = a0;
+            out[size_t(2 * i + 1) * dAxis] = 2 * i + 1 < liftEnd ? unpredict(line[2 * i + 1], a0, a1) : line[2 * i + 1];
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Host-side pass launchers.
 // ---------------------------------------------------------------------------
@@ -463,9 +508,39 @@ static PitchLoad pitchLoad(const float* p, int axis, int row, int slice) {
 
 static bool aligned(const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
 
+// Whether two arrays of a transform's extents share memory.
+template <class T>
+static bool overlap(const T* a, int rowA, int sliceA, const T* b, int rowB, int sliceB, int nx, int ny, int nz) {
+    auto end = [&](const T* p, int row, int slice) {
+        return reinterpret_cast<uintptr_t>(p + size_t(nz - 1) * slice + size_t(ny - 1) * row + nx);
+    };
+    return reinterpret_cast<uintptr_t>(a) < end(b, rowB, sliceB) && reinterpret_cast<uintptr_t>(b) < end(a, rowA, sliceA);
+}
+
+// A lifting pass along axis 0, 1 or 2 by whole lines in shared memory; false
+// if a line is too long for it.
+template <bool kInverse>
+static bool liftLinePass(i16* dst, const i16* src, int nx, int ny, int nz, int axis, int srcRow, int srcSlice,
+                         int dstRow, int dstSlice, cudaStream_t st) {
+    const int na = axis == 0 ? nx : axis == 1 ? ny : nz, nLines = axis == 0 ? ny : nx, nc = axis == 2 ? ny : nz;
+    if (na > kLineSamples) return false;
+    const int lines = std::min(32, kLineSamples / na);
+    const int liftEnd = axis == 0 ? intDwtXLiftEnd(na) : na;
+    const int s[3] = {1, srcRow, srcSlice}, d[3] = {1, dstRow, dstSlice};
+    const int line = axis == 0 ? 1 : 0, other = axis == 2 ? 1 : 2;
+    const dim3 g(u32(ceilDiv(nLines, lines)), u32(nc));
+    k_liftLines<kInverse><<<g, 256, 0, st>>>(dst, src, nLines, na, liftEnd, lines, axis == 0, s[line], s[axis], s[other],
+                                             d[line], d[axis], d[other]);
+    countLaunch();
+    return true;
+}
+
 template <bool kInverse>
 static void liftRowPass(i16* dst, const i16* src, int nx, int ny, int nz, int srcRow, int srcSlice, int dstRow,
                         int dstSlice, cudaStream_t st) {
+    if (overlap<i16>(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz) &&
+        liftLinePass<kInverse>(dst, src, nx, ny, nz, 0, srcRow, srcSlice, dstRow, dstSlice, st))
+        return;
     const u32 groups = u32(ceilDiv(nx, 8)), total = groups * u32(ny) * u32(nz);
     const bool vec = nx % 8 == 0 && ((srcRow | srcSlice | dstRow | dstSlice) & 7) == 0 && aligned(src, 16) &&
                      aligned(dst, 16) && (nx / 2) % 4 == 0;
@@ -478,6 +553,9 @@ static void liftRowPass(i16* dst, const i16* src, int nx, int ny, int nz, int sr
 template <bool kInverse>
 static void liftColPass(i16* dst, const i16* src, int nx, int ny, int nz, int axis, int srcRow, int srcSlice,
                         int dstRow, int dstSlice, const LiftBands* bands, cudaStream_t st) {
+    if (!bands && overlap<i16>(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz) &&
+        liftLinePass<kInverse>(dst, src, nx, ny, nz, axis, srcRow, srcSlice, dstRow, dstSlice, st))
+        return;
     const int na = axis == 1 ? ny : nz, nc = axis == 1 ? nz : ny;
     const int sAxis = axis == 1 ? srcRow : srcSlice, sOther = axis == 1 ? srcSlice : srcRow;
     const int dAxis = axis == 1 ? dstRow : dstSlice, dOther = axis == 1 ? dstSlice : dstRow;
@@ -529,16 +607,6 @@ static void planePass(float* dst, const float* src, int nx, int ny, int nz, int 
 // The plane pass's byte pitches are 32-bit.
 static bool planeFits(int row, int slice) { return row < (1 << 29) && slice < (1 << 29); }
 
-// Whether two arrays of a transform's extents share memory: the two passes
-// that a plane pass replaces go through a buffer, so their source may lie in
-// their destination.
-static bool overlap(const float* a, int rowA, int sliceA, const float* b, int rowB, int sliceB, int nx, int ny, int nz) {
-    auto end = [&](const float* p, int row, int slice) {
-        return reinterpret_cast<uintptr_t>(p + size_t(nz - 1) * slice + size_t(ny - 1) * row + nx);
-    };
-    return reinterpret_cast<uintptr_t>(a) < end(b, rowB, sliceB) && reinterpret_cast<uintptr_t>(b) < end(a, rowA, sliceA);
-}
-
 // A column pass between float arrays of the same pitches.
 template <bool kInverse>
 static void floatCols(float* dst, const float* src, int nx, int ny, int nz, int axis, int row, int slice, cudaStream_t st) {
@@ -572,12 +640,13 @@ void inverseRows<float>(float* dst, const float* src, int nx, int ny, int nz, in
 }
 
 // X and Y of a forward level (src -> dst, the X result through buf when they
-// run as two passes) and Y and X of an inverse one.
+// run as two passes: their source may lie in their destination) and Y and X of
+// an inverse one.
 template <class TIn>
 static void forwardPlane(float* dst, float* buf, const TIn* src, int nx, int ny, int nz, int ch, int srcRow, int srcSlice,
                          int dstRow, int dstSlice, cudaStream_t st) {
     if constexpr (std::is_same<TIn, float>::value) {
-        if (ch == 1 && planeFits(srcRow, srcSlice) && !overlap(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz)) {
+        if (ch == 1 && planeFits(srcRow, srcSlice) && !overlap<float>(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz)) {
             planePass<false>(dst, src, nx, ny, nz, srcRow, srcSlice, dstRow, dstSlice, st);
             return;
         }
@@ -589,7 +658,7 @@ template <class TOut>
 static void inversePlane(TOut* dst, float* buf, const float* src, int nx, int ny, int nz, int ch, int srcRow, int srcSlice,
                          int dstRow, int dstSlice, cudaStream_t st) {
     if constexpr (std::is_same<TOut, float>::value) {
-        if (ch == 1 && planeFits(srcRow, srcSlice) && !overlap(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz)) {
+        if (ch == 1 && planeFits(srcRow, srcSlice) && !overlap<float>(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz)) {
             planePass<true>(dst, src, nx, ny, nz, srcRow, srcSlice, dstRow, dstSlice, st);
             return;
         }

@@ -181,6 +181,9 @@ int cc_dwt_float2d_forward_lowpass_only_from_byte(float* d_dst, float* d_buf, co
 int cc_dwt_float_forward_static(float* d_dst, const float* d_src, int size_x, int size_y, int size_z,
                                 int src_channel_count, int dst_row_pitch, int dst_slice_pitch, int src_row_pitch,
                                 int src_slice_pitch, void* stream);
+/* dwtIntForward, dwtIntInverse.  Any of d_dst, d_buf and d_src
+ * may be the same array with the same pitches, up to 24576 samples along an
+ * axis (a pass in place goes line by line through shared memory). */
 int cc_dwt_int_forward(int16_t* d_dst, int16_t* d_buf, const int16_t* d_src, int size_x, int size_y, int size_z,
                        int dst_row_pitch, int dst_slice_pitch, int src_row_pitch, int src_slice_pitch, void* stream);
 int cc_dwt_int_inverse(int16_t* d_dst, int16_t* d_buf, const int16_t* d_src, int size_x, int size_y, int size_z,

@@ -111,6 +111,30 @@ def test_int_transform_at_tile_edges(oracle, shape, pad, shift):
     assert same(read_back(), a)
 
 
+@pytest.mark.parametrize("shape", [(8, 8, 8), (16, 10, 48), (64, 48, 64), (34, 66, 130), (1, 48, 64), (1, 64, 48), (1, 300, 520),
+                                   (8, 8, 2000)])
+@pytest.mark.parametrize("alias", ["dst=src", "buf=src", "dst=buf", "dst=buf=src"])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_int_transform_in_place(oracle, shape, alias, pad):
+    """A pass whose destination is its source stages whole lines: lines within
+    and across a warp's eight-sample groups, a CTA's rows of pairs, and 32
+    lines to a CTA or fewer."""
+    rng = np.random.default_rng(sum(shape))
+    a = rng.integers(-2000, 8000, shape).astype(np.int16)
+    nz, ny, nx = shape
+    row, rows = nx + pad, ny + (1 if pad else 0)
+    pitches = (row, row * rows, row, row * rows)
+    fwd = oracle.dwt_int(a)
+    for run, given, expect in ((cc.dwt_int_forward, a, fwd), (cc.dwt_int_inverse, fwd, a)):
+        src, read = pitched(given, row, rows, 0)
+        dst, read_dst = (src, read) if "dst" in alias and "src" in alias else pitched(np.zeros_like(a), row, rows, 0)
+        buf = {"dst=src": None, "buf=src": src, "dst=buf": dst, "dst=buf=src": src}[alias]
+        if buf is None:
+            buf, _ = pitched(np.zeros_like(a), row, rows, 0)
+        run(dst, buf, src, nx, ny, nz, *pitches)
+        assert same(read_dst(), expect)
+
+
 @pytest.mark.parametrize("shape,levels", [((20, 28), 1), ((16, 16), 1), ((40, 24), 2), ((64, 136), 2), ((66, 260), 1)])
 def test_heightfield_sizes(oracle, shape, levels):
     """Band widths that are and are not multiples of four symbols."""
