@@ -345,11 +345,11 @@ constexpr int kLiftPairs = 8;
 
 template <bool kInverse, int kV, bool kBands>
 __global__ void __launch_bounds__(128) k_liftCols(i16* __restrict__ dst, const i16* __restrict__ src, int nLines, int na,
-                                                  int sAxis, int sOther, int dAxis, int dOther, LiftBands bands) {
+                                                  int sAxis, int sOther, int dAxis, int dOther, int firstPair, LiftBands bands) {
     union Vec { uint2 v; i16 e[kV == 4 ? 4 : 1]; };
     const int x = int(blockIdx.x * 128u + threadIdx.x) * kV;
     if (x >= nLines) return;
-    const int hn = na >> 1, i0 = int(blockIdx.y) * kLiftPairs, c = blockIdx.z;
+    const int hn = na >> 1, i0 = firstPair + int(blockIdx.y) * kLiftPairs, c = blockIdx.z;
     const i16* in = src + size_t(c) * sOther + x;
     i16* out = dst + size_t(c) * dOther + x;
     const int bx = kBands && x >= bands.hx, lx = kBands ? x - bx * bands.hx : 0;
@@ -541,12 +541,18 @@ static void liftRowPass(i16* dst, const i16* src, int nx, int ny, int nz, int sr
     if (overlap<i16>(dst, dstRow, dstSlice, src, srcRow, srcSlice, nx, ny, nz) &&
         liftLinePass<kInverse>(dst, src, nx, ny, nz, 0, srcRow, srcSlice, dstRow, dstSlice, st))
         return;
-    const u32 groups = u32(ceilDiv(nx, 8)), total = groups * u32(ny) * u32(nz);
+    const u32 groups = u32(ceilDiv(nx, 8));
     const bool vec = nx % 8 == 0 && ((srcRow | srcSlice | dstRow | dstSlice) & 7) == 0 && aligned(src, 16) &&
                      aligned(dst, 16) && (nx / 2) % 4 == 0;
-    k_liftRows<kInverse><<<u32(ceilDiv(total, 256)), 256, 0, st>>>(dst, src, nx, ny, groups, total, intDwtXLiftEnd(nx),
-                                                                   srcRow, srcSlice, dstRow, dstSlice, vec);
-    countLaunch();
+    // threads are numbered in 32 bits: slices in parts
+    const int part = int(std::min<u64>(u64(nz), std::max<u64>(1, (1ull << 31) / (u64(groups) * u32(ny)))));
+    for (int z = 0; z < nz; z += part) {
+        const u32 total = groups * u32(ny) * u32(std::min(part, nz - z));
+        k_liftRows<kInverse><<<u32(ceilDiv(total, 256)), 256, 0, st>>>(
+            dst + size_t(z) * dstSlice, src + size_t(z) * srcSlice, nx, ny, groups, total, intDwtXLiftEnd(nx), srcRow,
+            srcSlice, dstRow, dstSlice, vec);
+        countLaunch();
+    }
 }
 
 // axis 1 (Y, other = Z) or 2 (Z, other = Y); bands: see k_liftCols
@@ -563,16 +569,20 @@ static void liftColPass(i16* dst, const i16* src, int nx, int ny, int nz, int ax
     if (bands)
         vec = vec && bands->hx % 4 == 0 && aligned(bands->band[0], 8) && aligned(bands->band[1], 8) &&
               aligned(bands->band[2], 8);
-    const dim3 g(u32(ceilDiv(nx, vec ? 512 : 128)), u32(ceilDiv(na / 2, kLiftPairs)), u32(nc));
-    const LiftBands none{};
-    if (bands) {
-        if (vec) k_liftCols<kInverse, 4, true><<<g, 128, 0, st>>>(dst, src, nx, na, sAxis, sOther, dAxis, dOther, *bands);
-        else k_liftCols<kInverse, 1, true><<<g, 128, 0, st>>>(dst, src, nx, na, sAxis, sOther, dAxis, dOther, *bands);
-    } else {
-        if (vec) k_liftCols<kInverse, 4, false><<<g, 128, 0, st>>>(dst, src, nx, na, sAxis, sOther, dAxis, dOther, none);
-        else k_liftCols<kInverse, 1, false><<<g, 128, 0, st>>>(dst, src, nx, na, sAxis, sOther, dAxis, dOther, none);
+    const LiftBands lb = bands ? *bands : LiftBands{};
+    // a grid's Y extent ends at 65535: axes of more than 2^20 samples in parts
+    constexpr int kPart = 65535 * kLiftPairs;
+    for (int i0 = 0; i0 < na / 2; i0 += kPart) {
+        const dim3 g(u32(ceilDiv(nx, vec ? 512 : 128)), u32(ceilDiv(std::min(na / 2 - i0, kPart), kLiftPairs)), u32(nc));
+        if (bands) {
+            if (vec) k_liftCols<kInverse, 4, true><<<g, 128, 0, st>>>(dst, src, nx, na, sAxis, sOther, dAxis, dOther, i0, lb);
+            else k_liftCols<kInverse, 1, true><<<g, 128, 0, st>>>(dst, src, nx, na, sAxis, sOther, dAxis, dOther, i0, lb);
+        } else {
+            if (vec) k_liftCols<kInverse, 4, false><<<g, 128, 0, st>>>(dst, src, nx, na, sAxis, sOther, dAxis, dOther, i0, lb);
+            else k_liftCols<kInverse, 1, false><<<g, 128, 0, st>>>(dst, src, nx, na, sAxis, sOther, dAxis, dOther, i0, lb);
+        }
+        countLaunch();
     }
-    countLaunch();
 }
 
 // One 2D level straight to symbols: src (sx x sy, row pitch srcRow) -> the LL

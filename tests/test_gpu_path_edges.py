@@ -135,6 +135,17 @@ def test_int_transform_in_place(oracle, shape, alias, pad):
         assert same(read_dst(), expect)
 
 
+def test_int_transform_of_a_very_tall_image(oracle):
+    """More groups of pairs along Y than a grid has rows (65535)."""
+    shape = (1, 2 * 8 * 65535 + 10, 8)
+    a = np.random.default_rng(4).integers(-2000, 8000, shape).astype(np.int16)
+    src, dst, buf, back = dev(a), dev(a * 0), dev(a * 0), dev(a * 0)
+    cc.dwt_int_forward(dst, buf, src, shape[2], shape[1])
+    assert same(host(dst), oracle.dwt_int(a))
+    cc.dwt_int_inverse(back, buf, dst, shape[2], shape[1])
+    assert same(host(back), a)
+
+
 @pytest.mark.parametrize("shape,levels", [((20, 28), 1), ((16, 16), 1), ((40, 24), 2), ((64, 136), 2), ((66, 260), 1)])
 def test_heightfield_sizes(oracle, shape, levels):
     """Band widths that are and are not multiples of four symbols."""
