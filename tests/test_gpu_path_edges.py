@@ -303,3 +303,22 @@ def test_wide_symbol_tables_of_many_streams(oracle, kind, S):
             assert dec(inst, cc.BitStream(words, bits), [outs[i, :n] for i in range(S)], n), cc.last_error()
             assert cc.decode_status(inst) == 0
             assert np.array_equal(host(outs[:, :n]).view(np.uint32), streams)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("bits", [16, 32])
+def test_counts_of_large_symbols(oracle, kind, bits):
+    """Symbols counted by slots of their low byte: one value throughout, a few
+    neighbours, many that share a low byte, the whole upper range, and both
+    sides of the first symbol that is not counted by bin."""
+    rng = np.random.default_rng(bits + kind)
+    n, top = 9000, 1 << (14 if bits == 16 else 20)
+    streams = np.zeros((6, n), np.uint16 if bits == 16 else np.uint32)
+    streams[0] = 2000
+    streams[1] = 1500 + rng.integers(0, 4, n)
+    streams[2] = 1024 + 7 + 256 * rng.integers(0, (top - 1100) // 256, n)
+    streams[3] = rng.integers(1024, top, n)
+    streams[4] = rng.integers(1016, 1032, n) * (rng.random(n) < 0.5)
+    streams[5] = top - 1 - 256 * (np.arange(n) % 3)
+    with cc.Instance(0, 6, n, 128, 14 if bits == 16 else 20) as inst:
+        roundtrip(oracle, inst, kind, streams, log2max=14 if bits == 16 else 20)
