@@ -521,14 +521,19 @@ __global__ void __launch_bounds__(256) k_leafTiers(EncParams p) {
 // entries directly.  Bound: instruction issue; walking a group's nonzeros on
 // its lane instead of a group's lanes together took three 256^3 streams'
 // highpass bands (50 million symbols, 26 million entries) from 191 to 123 us.
-constexpr u32 kWriteSymBins = 1024;   // symbol bins counted in shared memory by k_write (4 KB: eleven tiles per SM, not nine)
+constexpr u32 kWriteSymBins = 768;   // symbol bins counted in shared memory by k_write
 
-// Counts of the symbols above them: a tile has at most kRleTile, so a word of
-// shared memory holds a count (16 bits) and the upper bits of the symbol that
-// took the slot of its low byte first; others of that byte go to global
-// memory.  Streams whose large symbols are few would queue at a few words of
-// global memory: 8 million symbols of value 2000 take 5670 us without the
-// slots, 215 with them (400 with 4096 bins in shared memory instead).
+// Counts of the symbols above them.  Where these repeat - two of the first
+// symbols of a warp's 32 groups are like others - atomics on global memory
+// would queue at a few words: 8 million symbols of value 2000 took 5670 us.  A
+// word of shared memory then holds a count (a tile has at most kRleTile) and
+// the upper bits of the symbol that took the slot of its low byte first; others
+// of that byte go to global memory (215 us; 400 with 4096 bins in shared
+// memory).  Where they do not, every one goes there directly: a slot's look and
+// claim hold up a warp for some 150 cycles, and the write of the lowpass
+// streams of three 256^3 volumes, on the batch's longest chain, took 12.4 us
+// instead of 7.5.  Bins and slots are 4 KB together, twelve tiles per SM; with
+// 5 KB, eleven, their highpass streams took 125 us instead of 121.
 constexpr u32 kHotSlots = 256;
 static_assert(kRleTile < 65536u && kWriteSymBins >= kHotSlots, "16-bit counts; a symbol's upper bits are not 0");
 
@@ -582,6 +587,19 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
     u32 mUnused;
     const GroupRuns g = loadGroups(in, wbase, n, rows, mUnused);
     u32* gSym = p.hist + mS.histOff;
+    bool slots = false;   // warp-uniform
+    if (large) {
+        const u32 x = g.mask ? u32(rows[lane * kRlePitch + u32(__ffs(int(g.mask))) - 1u]) : 0u;
+        const bool is = x >= kWriteSymBins;
+        const u32 peers = __match_any_sync(0xffffffffu, x);
+        const u32 of = __popc(__ballot_sync(0xffffffffu, is));
+        const u32 distinct = __popc(__ballot_sync(0xffffffffu, is && lane == u32(__ffs(int(peers))) - 1u));
+        slots = of >= distinct + 2u;
+    }
+    auto addLarge = [&](u32 sym) {
+        if (slots) countLarge(hHot, gSym, sym);
+        else atomicAdd(gSym + sym, 1u);
+    };
     auto flush = [&] {
         for (u32 i = threadIdx.x; i < smemBins; i += kRleThreads)
             if (hSym[i]) atomicAdd(gSym + i, hSym[i]);
@@ -595,7 +613,7 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
             if (wbase + 32u * k + lane >= n) break;
             const u32 x = rows[k * kRlePitch + lane];
             if (x < smemBins) atomicAdd(hSym + x, 1u);
-            else if (x < mS.histSize) countLarge(hHot, gSym, x);
+            else if (x < mS.histSize) addLarge(x);
         }
         __syncthreads();
         flush();
@@ -674,10 +692,10 @@ __global__ void __launch_bounds__(kRleThreads) k_write(EncParams p) {
                 if (k < 4u) s03 += si;
                 else if (k < 8u) s47 += si;
                 else if (sym < smemBins) atomicAdd(hSym + sym, 1u);
-                else if (sym < mS.histSize) countLarge(hHot, gSym, sym);
+                else if (sym < mS.histSize) addLarge(sym);
             } else {
                 if (sym < smemBins) atomicAdd(hSym + sym, 1u);
-                else if (sym < mS.histSize) countLarge(hHot, gSym, sym);
+                else if (sym < mS.histSize) addLarge(sym);
                 if (zc < mZ.histSize) atomicAdd(hZc + zc, 1u);
                 else rangeErr = true;
             }

@@ -313,12 +313,13 @@ def test_counts_of_large_symbols(oracle, kind, bits):
     sides of the first symbol that is not counted by bin."""
     rng = np.random.default_rng(bits + kind)
     n, top = 9000, 1 << (14 if bits == 16 else 20)
-    streams = np.zeros((6, n), np.uint16 if bits == 16 else np.uint32)
+    streams = np.zeros((7, n), np.uint16 if bits == 16 else np.uint32)
     streams[0] = 2000
     streams[1] = 1500 + rng.integers(0, 4, n)
     streams[2] = 1024 + 7 + 256 * rng.integers(0, (top - 1100) // 256, n)
     streams[3] = rng.integers(1024, top, n)
     streams[4] = rng.integers(1016, 1032, n) * (rng.random(n) < 0.5)
     streams[5] = top - 1 - 256 * (np.arange(n) % 3)
-    with cc.Instance(0, 6, n, 128, 14 if bits == 16 else 20) as inst:
+    streams[6] = 760 + rng.integers(0, 16, n)
+    with cc.Instance(0, 7, n, 128, 14 if bits == 16 else 20) as inst:
         roundtrip(oracle, inst, kind, streams, log2max=14 if bits == 16 else 20)
