@@ -41,6 +41,7 @@ struct cc_volume_batch {
     cc_instance* ILP = nullptr;        // own instance of the lowpass encode
     cudaStream_t sideStream = nullptr; // the lowpass encode's stream
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
+    cudaEvent_t evBuild = nullptr;     // the lowpass encode has come to its table build
     ccb::u32* words = nullptr;         // device: the bricks' streams
     ccb::u64 wordsCap = 0;
     cc_instance* user = nullptr;
@@ -304,6 +305,14 @@ static int batchEnqueueCompress(cc_volume_batch* b) {
     lp.tiles = b->lpTiles[k - 1];
     lp.blocks = b->lpBlocks[k - 1];
     int rc;
+    // The lowpass tables, built on an SM of their own each, are the longest
+    // chain of few large volumes, and their CTAs wait while the highpass write
+    // fills every SM: then it comes after them.  Started first it delayed them
+    // to its end, 126 us of a 1024 us pass over three 256^3 volumes.
+    const u32 sms = u32(std::max(1, ILP->smCount > 0 ? ILP->smCount : 148));
+    const bool solo = k <= sms && b->encTiles[k - 1] >= sms;
+    ILP->encBuildNext = solo ? b->evBuild : nullptr;
+    I->encFillAfter = ILP->encBuildNext;
     {
         SectionTimer t(I, "batch.lowpass_encode", b->sideStream);
         rc = encodeLaunch(ILP, lp, ILP->out, ILP->outWordsMax);
@@ -324,7 +333,6 @@ static int batchEnqueueCompress(cc_volume_batch* b) {
         const u32 hpPer = 7 * b->levels;
         k_brickOffsets<<<1, 1024, 0, st>>>(ILP->layout, I->layout, hpPer, k, b->wordOff, b->bitSize, ILP->errors,
                                            I->errors);
-        const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
         const u32 parts = std::max<u32>(1, std::min<u32>(1024, u32(ceilDiv(16 * sms, k))));
         k_brickConcat<<<k * parts, 256, 0, st>>>(ILP->out, I->out, ILP->layout, I->layout, hpPer, parts, b->wordOff,
                                                  b->bitSize, b->words);
@@ -567,6 +575,7 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
     cudaError_t ce = cudaStreamCreateWithFlags(&b->sideStream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&b->evFork, cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&b->evJoin, cudaEventDisableTiming);
+    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&b->evBuild, cudaEventDisableTiming);
     if (ce != cudaSuccess) { cc_volume_batch_destroy(b); return cudaFail(ce, "volume batch streams"); }
     b->wordsCap = I->outWordsMax + b->ILP->outWordsMax;
 
@@ -907,6 +916,7 @@ void cc_volume_batch_destroy(cc_volume_batch* b) {
     if (b->captureStream) cudaStreamDestroy(b->captureStream);
     if (b->sideStream) cudaStreamDestroy(b->sideStream);
     if (b->evFork) cudaEventDestroy(b->evFork);
+    if (b->evBuild) cudaEventDestroy(b->evBuild);
     if (b->evJoin) cudaEventDestroy(b->evJoin);
     for (cudaEvent_t ev : b->tabEvent)
         if (ev) cudaEventDestroy(ev);

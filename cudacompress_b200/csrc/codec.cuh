@@ -207,6 +207,9 @@ struct cc_instance {
     // the small-table launch on `stream` (fork / join by the two events)
     cudaStream_t buildSide = nullptr, buildSide2 = nullptr;   // the table builders' other streams
     cudaEvent_t buildFork = nullptr, buildJoin = nullptr, buildJoin2 = nullptr;
+    // a batch's two encodes: recorded before the table build if set, and waited
+    // for before the plan's fill if set (batchEnqueueCompress)
+    cudaEvent_t encBuildNext = nullptr, encFillAfter = nullptr;
     // the decode's zero fill and Huff branch on buildSide2
     cudaEvent_t decFork = nullptr, decZeroed = nullptr, decTablesReady = nullptr, decJoin = nullptr;
 

@@ -23,6 +23,7 @@ namespace ccb {
 struct EncParams {
     u32 S, T;
     u32 totalTiles, totalBlocks;
+    u32 maxTiles;     // of the longest stream
     u32 cb, cbLog, log2Max, bins, symBytes;   // cb = 2^cbLog
     const EncStreamDev* streams;
     const EncTableDev* tables;
@@ -310,6 +311,65 @@ __global__ void __launch_bounds__(kScanWarps * 32) k_scan(EncParams p) {
     if (s < p.S) scanStream(p, s);
 }
 
+// The same with a CTA per stream, for long ones: a warp takes 0.7 us for 32
+// tiles, one step after the other.  63 streams of up to 1024 tiles (three 256^3
+// volumes): 5 us, and 6 for the plan, where two streams per warp of one CTA
+// took 38 with the plan; a 512^3 volume's encode 1729 -> 1531 us, one stream of
+// 64 million symbols 1608 -> 934.
+constexpr u32 kScanThreads = 512;
+
+__global__ void __launch_bounds__(kScanThreads) k_scanWide(EncParams p) {
+    constexpr u32 kWarps = kScanThreads / 32;
+    __shared__ RunSum sWarp[kWarps];
+    const u32 s = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const EncStreamDev sd = p.streams[s];
+    if (sd.kind != KIND_RLHUFF) {   // block-uniform
+        if (threadIdx.x == 0) p.counts[s] = sd.n;
+        return;
+    }
+    const u32 tiles = u32(ceilDiv(sd.n, kRleTile));
+    const RunSum* T = p.tiles + sd.tileOff;
+    TileStart* TS = p.tileStart + sd.tileOff;
+    const RunSum none{0, 0, 0, 0};
+    RunSum carry = none;
+    RunSum next = threadIdx.x < tiles ? T[threadIdx.x] : none;
+    for (u32 base = 0; base < tiles; base += kScanThreads) {
+        const u32 i = base + threadIdx.x;
+        const RunSum inc = warpInclusiveRun(next);
+        next = i + kScanThreads < tiles ? T[i + kScanThreads] : none;   // in flight over this step
+        RunSum ex = shflUpRun(inc, 1);
+        if (lane == 0) ex = none;
+        if (lane == 31) sWarp[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            const RunSum w = warpInclusiveRun(lane < kWarps ? sWarp[lane] : none);
+            if (lane < kWarps) sWarp[lane] = w;
+        }
+        __syncthreads();
+        const RunSum E = runCombine(carry, warp ? runCombine(sWarp[warp - 1], ex) : ex);
+        carry = runCombine(carry, sWarp[kWarps - 1]);
+        if (i < tiles) {
+            TileStart ts;
+            ts.prevP1 = E.cnt ? E.lastP1 : 0u;
+            ts.out = E.cnt ? E.cnt + E.ext + (E.firstP1 - 1u) / 256u : 0u;
+            TS[i] = ts;
+        }
+        __syncthreads();   // sWarp is read
+    }
+    if (threadIdx.x == 0) p.counts[s] = carry.cnt ? carry.cnt + carry.ext + (carry.firstP1 - 1u) / 256u : 0u;
+}
+
+// Which of them.  Up to 64 streams take a CTA each where one CTA's 32 warps
+// would take more than four steps over them all (0.7 us each; a launch of its
+// own for the scan costs 2.5 us): one warp or two per stream, which one CTA
+// then joins with the plan.  More streams: where the longest has more than 64
+// tiles, unless that many CTAs would take longer than its warp (2 us per 1184).
+constexpr u32 kScanPlanStreams = 64;
+static bool scanWide(u32 streams, u32 tiles) {
+    if (streams <= kScanPlanStreams) return ceilDiv(streams, 32) * ceilDiv(tiles, 32) > 4;
+    return tiles > 64 && streams / 16 <= tiles;
+}
+
 // Table builders by leaf count (k_leafTiers sorts the tables, k_tableBuild
 // builds them): the heap merge is a latency-bound chain on one warp, so a
 // smaller table gets a smaller CTA and heap and more of them share an SM.
@@ -416,8 +476,7 @@ __global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
     histPlanChunk(p, scratch);
 }
 
-// Passes 2 and 3 of a call of few streams in one CTA, two of them per warp.
-constexpr u32 kScanPlanStreams = 64;
+// Passes 2 and 3 of a call of few and short streams in one CTA (scanWide).
 
 __global__ void __launch_bounds__(1024) k_scanPlan(EncParams p) {
     __shared__ u32 scratch[33 * 7];
@@ -1494,14 +1553,16 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
     countLaunch();
     if (p.totalTiles) { SectionTimer t(I, "enc.summary", st); k_summary<Sym><<<p.totalTiles, kRleThreads, 0, st>>>(p); countLaunch(); }
     const u32 chunks = std::max<u32>(1, u32(ceilDiv(p.T, kPlanChunk)));
-    if (p.S <= kScanPlanStreams) {   // then one chunk
+    const bool wide = scanWide(p.S, p.maxTiles);
+    if (p.S <= kScanPlanStreams && !wide) {   // then one chunk
         SectionTimer t(I, "enc.hist_plan", st);
         k_scanPlan<<<1, 1024, 0, st>>>(p);
         countLaunch();
     } else {
         {
             SectionTimer t(I, "enc.rle_scan", st);
-            k_scan<<<u32(ceilDiv(p.S, kScanWarps)), kScanWarps * 32, 0, st>>>(p);
+            if (wide) k_scanWide<<<p.S, kScanThreads, 0, st>>>(p);
+            else k_scan<<<u32(ceilDiv(p.S, kScanWarps)), kScanWarps * 32, 0, st>>>(p);
             countLaunch();
         }
         SectionTimer t(I, "enc.hist_plan", st);
@@ -1509,6 +1570,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         countLaunch();
         if (chunks > 1) { k_histPlanCarry<<<chunks - 1, 1024, 0, st>>>(p); countLaunch(); }
     }
+    if (I->encFillAfter) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->encFillAfter, 0), "encode order");
     { SectionTimer t(I, "enc.hist_zero", st); k_planFill<<<2 * 148, 256, 0, st>>>(p); countLaunch(); }
     if (p.totalTiles) {
         CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_write<Sym>),
@@ -1518,6 +1580,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         k_write<Sym><<<p.totalTiles, kRleThreads, writeSmem<Sym>(), st>>>(p);
         countLaunch();
     }
+    if (I->encBuildNext) CC_TRY_CUDA(cudaEventRecord(I->encBuildNext, st), "encode order");
     const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
     // an instance whose tables run beside other kernels (the batched codec's
     // lowpass encode) may ask for an SM of its own per table: the sequential
@@ -1667,6 +1730,7 @@ int encodeLaunch(cc_instance* I, const EncPlan& hp, u32* out, u64 outCap) {
     p.S = hp.S;
     p.T = hp.T;
     p.totalTiles = hp.tiles;
+    p.maxTiles = u32(ceilDiv(hp.maxCount, kRleTile));
     p.totalBlocks = hp.blocks;
     p.cb = I->codingBlockSize;
     p.cbLog = 31u - u32(__builtin_clz(p.cb));

@@ -229,6 +229,26 @@ def test_streams_around_a_step_of_the_tile_scan(oracle, n):
         roundtrip(oracle, inst, 0, streams)
 
 
+@pytest.mark.parametrize("S,tiles", [(1, 128), (1, 129), (2, 511), (2, 512), (2, 513), (1, 1090), (33, 64), (33, 65), (64, 65),
+                                     (65, 64), (65, 65)])
+def test_long_streams_of_the_tile_scan(oracle, S, tiles):
+    """Both sides of the rule for a block per stream, and of a block's step of
+    512 tiles; the first stream is dense, the second has runs across many
+    tiles, the last one nonzero near its end."""
+    n = tiles * 2048 - 5
+    rng = np.random.default_rng(tiles + S)
+    streams = np.zeros((S, n), np.uint16)
+    for i in range(S):
+        at = np.unique(rng.integers(0, n, 37 if i == 1 else 3 * tiles))
+        streams[i, at] = rng.integers(1, 40, len(at))
+    streams[-1] = 0
+    streams[-1, -3] = 7
+    if S > 1:
+        streams[0] = rng.integers(0, 4, n)
+    with cc.Instance(0, S, n, 128, 14) as inst:
+        roundtrip(oracle, inst, 0, streams)
+
+
 @pytest.mark.parametrize("kind", [0, 1])
 @pytest.mark.parametrize("cb", [32, 64, 128, 256])
 @pytest.mark.parametrize("n", [3000, 40000])
