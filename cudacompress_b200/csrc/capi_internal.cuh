@@ -147,6 +147,7 @@ enum SmemAttrKernel {
     kAttrDecHuff32,
     kAttrWrite16,
     kAttrWrite32,
+    kAttrTableBuildWide,
     kAttrDecRl,   // 8 variants
     kAttrCount = kAttrDecRl + 8
 };

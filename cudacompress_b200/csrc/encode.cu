@@ -839,9 +839,17 @@ __device__ __forceinline__ void putBits(u32* words, u32 pos, u32 value, u32 coun
 }
 
 // Builds table t (all kThreads threads of the block; returns uniformly).
-// Tables of up to kCap leaves are built in shared memory.
-template <u32 kThreads, u32 kCap>
-__device__ void buildTable(const EncParams& p, u32 t) {
+// Tables of up to kCap leaves are built in shared memory.  kWide (alphabets of
+// more than kWideBins): the leaves are gathered a range of bins per warp.  A
+// range per thread, which small alphabets keep, reads a cache line per lane,
+// and the full builder's heap leaves 28 KB of L1: seven streams over 300000
+// bins 690 us, 201 so; over 60000 bins 284 and 139; a hundred of them, by one
+// warp with a load in flight, 622 and 446.  The merge loop's time changes by 1
+// to 5% with the code around it, which is why the two are compiled apart.
+constexpr u32 kWideBins = 1u << 14;
+
+template <u32 kThreads, u32 kCap, bool kWide>
+__device__ __forceinline__ void buildTable(const EncParams& p, u32 t) {
     constexpr int kSegs = int(kCap / 17u) + 1;   // the sort's queue: segments longer than 16 keys
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ u32 sScan[40];
@@ -862,7 +870,7 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     if (es.kind == KIND_RLHUFF)
         for (u32 s = es.groupFirst + threadIdx.x; s < es.groupFirst + es.groupSize; s += kThreads)
             if (p.counts[s]) atomicAnd(&sAllEmpty, 0u);
-    if (kThreads > 32) {
+    if (kThreads > 32 && !kWide) {
         u32 localMax = 0;
         bool any = false;
         for (u32 b = threadIdx.x; b < meta.histSize; b += kThreads)
@@ -870,7 +878,7 @@ __device__ void buildTable(const EncParams& p, u32 t) {
         if (any) atomicMax(&sMax, localMax);
     }
     __syncthreads();
-    u32 symbolMax = count ? sMax : 0u;   // kThreads == 32: with the leaves, below
+    u32 symbolMax = count ? sMax : 0u;   // kThreads == 32, kWide: with the leaves, below
     // Histogram.cu:117-121: with every stream of the reference call empty the
     // reference builds its tables from stale arena words; for zero-count table
     // i that word is the low half of a device pointer when 2+2i < S (nonzero),
@@ -897,6 +905,64 @@ __device__ void buildTable(const EncParams& p, u32 t) {
     } else if (count == 0) {
         L = 0;
         if (L < p.buildLo || L > p.buildHi) return;
+    } else if constexpr (kWide) {
+        // large alphabets: a range of bins per warp, 32 bins at a time and
+        // kFlight of them in flight, counted, then written behind the warps
+        // before
+        constexpr u32 kWarps = kThreads / 32, kFlight = 8;
+        const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+        const u32 per = (meta.histSize + 32u * kWarps - 1u) / (32u * kWarps) * 32u;
+        const u32 b0 = min(meta.histSize, warp * per), b1 = min(meta.histSize, b0 + per);
+        u32 c = 0, top = 0;
+        for (u32 b = b0; b < b1; b += 32u * kFlight) {
+            u32 h[kFlight];
+#pragma unroll
+            for (u32 q = 0; q < kFlight; ++q) h[q] = b + 32u * q + lane < b1 ? hist[b + 32u * q + lane] : 0u;
+#pragma unroll
+            for (u32 q = 0; q < kFlight; ++q) {
+                const u32 m = __ballot_sync(0xffffffffu, h[q] != 0);
+                c += __popc(m);
+                if (m) top = b + 32u * q + 31u - u32(__clz(int(m)));
+            }
+        }
+        if (lane == 0) {
+            sScan[warp] = c;
+            if (c) atomicMax(&sMax, top);
+        }
+        __syncthreads();
+        u32 off = 0;
+        L = 0;
+#pragma unroll
+        for (u32 w = 0; w < kWarps; ++w) {
+            if (w < warp) off += sScan[w];
+            L += sScan[w];
+        }
+        symbolMax = sMax;
+        if (L < p.buildLo || L > p.buildHi) return;
+        const bool toSmem = L <= smemLeaves;
+        const bool quirk65535 = p.symBytes == 2 && p.bins == 65536u && symbolMax == 65535u;
+        for (u32 b = b0; b < b1; b += 32u * kFlight) {
+            u32 hs[kFlight];
+#pragma unroll
+            for (u32 q = 0; q < kFlight; ++q) hs[q] = b + 32u * q + lane < b1 ? hist[b + 32u * q + lane] : 0u;
+#pragma unroll
+            for (u32 q = 0; q < kFlight; ++q) {
+                const u32 sym = b + 32u * q + lane, m = __ballot_sync(0xffffffffu, hs[q] != 0);
+                if (hs[q]) {
+                    u32 h = hs[q];
+                    if (quirk65535 && sym == 65535u) h += count & 1u;   // HistogramKernels.cui:165,200 padding word
+                    const u32 to = off + __popc(m & below);
+                    leafSym[to] = sym;
+                    if (toSmem) {
+                        heapP[to + 1] = h;
+                        heapI[to + 1] = 2u * to;
+                    } else {
+                        heapG[to] = (u64(h) << 32) | to;
+                    }
+                }
+                off += __popc(m);
+            }
+        }
     } else if (kThreads == 32) {
         // one warp: largest symbol and leaves in one pass, 32 bins at a time
         const u32 below = (1u << threadIdx.x) - 1u;
@@ -974,24 +1040,33 @@ __device__ void buildTable(const EncParams& p, u32 t) {
             tb::blockIntrosort<kThreads>(orderS, int(L), lList, rList, seg, sSegA, sSegB, sSegCount, heapI);
             order = heapI;
         }
-    } else if (threadIdx.x == 0) {
-        // tables larger than the shared-memory builder: sequential, global memory
+    } else {
+        // tables larger than the shared-memory builder: the merges and the sort
+        // run sequentially, on the same area where it holds the heap (8 bytes
+        // per leaf) and then the sort's keys, else on global memory.  The area
+        // leaves 28 KB of L1, so that 16000 leaves took 47.5 ms on global
+        // memory (44.7 when a smaller builder left more); 34.0 so.
         u32* parent = p.parentWork + 2 * meta.leafOff;
-        u32 maxLen = 0;
-        hb::buildTree(heapG, parent, int(L));
-        const int nodes = int(2 * L - 1);
-        parent[nodes - 1] = 0;
-        for (int id = nodes - 2; id >= 0; --id) {
-            u32 d = parent[parent[id]] + 1u;
-            parent[id] = d > 255u ? 255u : d;
+        u64* heap = heapG;
+        if (sizeof(u64) * L <= At::kBytes) {
+            heap = reinterpret_cast<u64*>(dyn);
+            for (u32 i = threadIdx.x; i < L; i += kThreads) heap[i] = heapG[i];
+            __syncthreads();
         }
-        for (u32 i = 0; i < L; ++i) {
-            u32 d = parent[i];
-            maxLen = max(maxLen, d);
+        if (threadIdx.x == 0) hb::buildTree(heap, parent, int(L));
+        __syncthreads();
+        if (sizeof(u32) * L <= At::kBytes) order = reinterpret_cast<u32*>(dyn);
+        const u32 root = 2 * L - 2;
+        u32 localMax = 0;
+        for (u32 i = threadIdx.x; i < L; i += kThreads) {
+            u32 d = 0, node = i;
+            while (node != root && d < 32) { node = parent[node]; ++d; }
             order[i] = (min(d, 31u) << 27) | i;
+            localMax = max(localMax, d);
         }
-        if (maxLen <= 31) hb::introsort(order, int(L), hb::LenLess());
-        sMaxLen = maxLen;
+        if (localMax) atomicMax(&sMaxLen, localMax);
+        __syncthreads();
+        if (threadIdx.x == 0 && sMaxLen <= 31) hb::introsort(order, int(L), hb::LenLess());
     }
     if (threadIdx.x < 32) lenCount[threadIdx.x] = 0;
     __syncthreads();
@@ -1061,16 +1136,16 @@ __device__ void buildTable(const EncParams& p, u32 t) {
 // One table per CTA (kBuildEach), or the CTAs walk the list of one tier.
 // Bounding the one-warp tier to 72 registers (28 CTAs per SM instead of 20)
 // left 4096 bricks at the same time.
-template <u32 kThreads, u32 kCap>
+template <u32 kThreads, u32 kCap, bool kWide>
 __global__ void __launch_bounds__(kThreads, 1) k_tableBuild(EncParams p) {
     if (p.buildTier == kBuildEach) {
-        buildTable<kThreads, kCap>(p, blockIdx.x);
+        buildTable<kThreads, kCap, kWide>(p, blockIdx.x);
         return;
     }
     const u32 n = u32(p.totals[4 + p.buildTier]);
     const u32* list = p.tierTables + u64(p.buildTier) * p.T;
     for (u32 i = blockIdx.x; i < n; i += gridDim.x) {
-        buildTable<kThreads, kCap>(p, list[i]);
+        buildTable<kThreads, kCap, kWide>(p, list[i]);
         __syncthreads();   // the next table reuses the shared memory
     }
 }
@@ -1078,6 +1153,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tableBuild(EncParams p) {
 // Dynamic shared memory that leaves no room on an SM for another table-build
 // CTA or most other kernels' CTAs: the device's per-block opt-in limit minus
 // the kernel's static shared memory.
+template <bool kWide>
 static size_t tableBuildSoloSmem(int device) {
     static size_t cached[64] = {};
     if (device < 0 || device >= 64) return 0;
@@ -1085,7 +1161,7 @@ static size_t tableBuildSoloSmem(int device) {
         int optin = 0;
         cudaFuncAttributes fa{};
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-        cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(k_tableBuild<kBigThreads, kBuildSmemLeaves>));
+        cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(k_tableBuild<kBigThreads, kBuildSmemLeaves, kWide>));
         cached[device] = optin > int(fa.sharedSizeBytes) ? size_t(optin) - fa.sharedSizeBytes : 0;
     }
     return cached[device];
@@ -1546,6 +1622,95 @@ int encodePrepare(cc_instance* I, const EncStream* streams, u32 S, char* slot, s
     return CC_OK;
 }
 
+// The full builder's dynamic shared memory, allowed for its launch.
+template <bool kWide>
+static cudaError_t tableBuildSmem(const cc_instance* I, bool solo, size_t& bytes) {
+    bytes = hm::Layout<kBuildSmemLeaves>::kBytes;
+    if (solo) bytes = std::max(bytes, tableBuildSoloSmem<kWide>(I->device));
+    return ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBigThreads, kBuildSmemLeaves, kWide>),
+                               kWide ? kAttrTableBuildWide : kAttrTableBuild, I->device, bytes);
+}
+
+template <bool kWide>
+static int launchTableBuild(cc_instance* I, const EncParams& p) {
+    cudaStream_t st = I->stream;
+    const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
+    // an instance whose tables run beside other kernels (the batched codec's
+    // lowpass encode) may ask for an SM of its own per table: the sequential
+    // heap merge is latency-bound and loses issue slots to co-resident CTAs
+    const bool solo = I->tableBuildSoloSM && p.T <= sms;
+    size_t buildSmem;
+    CC_TRY_CUDA(tableBuildSmem<kWide>(I, solo, buildSmem), "tableBuild smem");
+    {
+        SectionTimer t(I, "enc.table_build", st);
+        EncParams q = p;
+        q.buildLo = 0;
+        q.buildHi = ~0u;
+        q.buildTier = kBuildEach;
+        // a call of few tables builds them in one launch, a CTA each (the
+        // tiers' pre-pass, launches and stream forks would cost it more than
+        // they save)
+        if (!solo && p.T > kTierMinTables) {
+            // tables sorted by leaf count, each tier's list walked by its own
+            // builder, at the same time: tier 0 on the instance stream, tier 1
+            // on the second side stream, tiers 3 and 2 on the first
+            k_leafTiers<<<u32(ceilDiv(p.T, 8)), 256, 0, st>>>(q);
+            countLaunch();
+            const bool side = p.heapCap > kSmallLeaves, side2 = p.heapCap > kTinyLeaves;
+            if (side2) {
+                CC_TRY_CUDA(cudaEventRecord(I->buildFork, st), "table build fork");
+                CC_TRY_CUDA(cudaStreamWaitEvent(I->buildSide2, I->buildFork, 0), "table build fork");
+                EncParams small = q;
+                small.buildTier = 1;
+                small.buildLo = kTinyLeaves + 1;
+                small.buildHi = kSmallLeaves;
+                k_tableBuild<64u, kSmallLeaves, kWide>
+                    <<<std::min(p.T, 10u * sms), 64, hm::Layout<kSmallLeaves>::kBytes, I->buildSide2>>>(small);
+                countLaunch();
+                CC_TRY_CUDA(cudaEventRecord(I->buildJoin2, I->buildSide2), "table build join");
+            }
+            if (side) {
+                CC_TRY_CUDA(cudaStreamWaitEvent(I->buildSide, I->buildFork, 0), "table build fork");
+                if (p.heapCap > kBuildSplitLeaves) {
+                    EncParams big = q;
+                    big.buildTier = 3;
+                    big.buildLo = kBuildSplitLeaves + 1;
+                    k_tableBuild<kBigThreads, kBuildSmemLeaves, kWide>
+                        <<<std::min(p.T, sms), kBigThreads, buildSmem, I->buildSide>>>(big);
+                    countLaunch();
+                }
+                EncParams mid = q;
+                mid.buildTier = 2;
+                mid.buildLo = kSmallLeaves + 1;
+                mid.buildHi = kBuildSplitLeaves;
+                k_tableBuild<kMidThreads, kBuildSplitLeaves, kWide>
+                    <<<std::min(p.T, 5u * sms), kMidThreads, hm::Layout<kBuildSplitLeaves>::kBytes, I->buildSide>>>(mid);
+                countLaunch();
+                CC_TRY_CUDA(cudaEventRecord(I->buildJoin, I->buildSide), "table build join");
+            }
+            EncParams tiny = q;
+            tiny.buildTier = 0;
+            tiny.buildHi = kTinyLeaves;
+            k_tableBuild<32u, kTinyLeaves, kWide>
+                <<<std::min(p.T, 32u * sms), 32, hm::Layout<kTinyLeaves>::kBytes, st>>>(tiny);
+            countLaunch();
+            if (side2) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->buildJoin2, 0), "table build join");
+            if (side) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->buildJoin, 0), "table build join");
+        } else {
+            if (!solo && p.heapCap <= kSmallLeaves)
+                k_tableBuild<kBuildThreads, kSmallLeaves, kWide>
+                    <<<p.T, kBuildThreads, hm::Layout<kSmallLeaves>::kBytes, st>>>(q);
+            else if (!solo && p.heapCap <= kBuildSplitLeaves)
+                k_tableBuild<kBuildThreads, kBuildSplitLeaves, kWide>
+                    <<<p.T, kBuildThreads, hm::Layout<kBuildSplitLeaves>::kBytes, st>>>(q);
+            else
+                k_tableBuild<kBigThreads, kBuildSmemLeaves, kWide><<<p.T, kBigThreads, buildSmem, st>>>(q);
+            countLaunch();
+        }
+    }
+    return CC_OK;
+}
+
 template <class Sym>
 static int launchEncode(cc_instance* I, const EncParams& p) {
     cudaStream_t st = I->stream;
@@ -1581,83 +1746,9 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         countLaunch();
     }
     if (I->encBuildNext) CC_TRY_CUDA(cudaEventRecord(I->encBuildNext, st), "encode order");
+    int rc = p.bins > kWideBins ? launchTableBuild<true>(I, p) : launchTableBuild<false>(I, p);
+    if (rc) return rc;
     const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
-    // an instance whose tables run beside other kernels (the batched codec's
-    // lowpass encode) may ask for an SM of its own per table: the sequential
-    // heap merge is latency-bound and loses issue slots to co-resident CTAs
-    const bool solo = I->tableBuildSoloSM && p.T <= sms;
-    size_t buildSmem = hm::Layout<kBuildSmemLeaves>::kBytes;
-    if (solo) buildSmem = std::max(buildSmem, tableBuildSoloSmem(I->device));
-    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBigThreads, kBuildSmemLeaves>),
-                                    kAttrTableBuild, I->device, buildSmem),
-                "tableBuild smem");
-    {
-        SectionTimer t(I, "enc.table_build", st);
-        EncParams q = p;
-        q.buildLo = 0;
-        q.buildHi = ~0u;
-        q.buildTier = kBuildEach;
-        // a call of few tables builds them in one launch, a CTA each (the
-        // tiers' pre-pass, launches and stream forks would cost it more than
-        // they save)
-        if (!solo && p.T > kTierMinTables) {
-            // tables sorted by leaf count, each tier's list walked by its own
-            // builder, at the same time: tier 0 on the instance stream, tier 1
-            // on the second side stream, tiers 3 and 2 on the first
-            k_leafTiers<<<u32(ceilDiv(p.T, 8)), 256, 0, st>>>(q);
-            countLaunch();
-            const bool side = p.heapCap > kSmallLeaves, side2 = p.heapCap > kTinyLeaves;
-            if (side2) {
-                CC_TRY_CUDA(cudaEventRecord(I->buildFork, st), "table build fork");
-                CC_TRY_CUDA(cudaStreamWaitEvent(I->buildSide2, I->buildFork, 0), "table build fork");
-                EncParams small = q;
-                small.buildTier = 1;
-                small.buildLo = kTinyLeaves + 1;
-                small.buildHi = kSmallLeaves;
-                k_tableBuild<64u, kSmallLeaves>
-                    <<<std::min(p.T, 10u * sms), 64, hm::Layout<kSmallLeaves>::kBytes, I->buildSide2>>>(small);
-                countLaunch();
-                CC_TRY_CUDA(cudaEventRecord(I->buildJoin2, I->buildSide2), "table build join");
-            }
-            if (side) {
-                CC_TRY_CUDA(cudaStreamWaitEvent(I->buildSide, I->buildFork, 0), "table build fork");
-                if (p.heapCap > kBuildSplitLeaves) {
-                    EncParams big = q;
-                    big.buildTier = 3;
-                    big.buildLo = kBuildSplitLeaves + 1;
-                    k_tableBuild<kBigThreads, kBuildSmemLeaves>
-                        <<<std::min(p.T, sms), kBigThreads, buildSmem, I->buildSide>>>(big);
-                    countLaunch();
-                }
-                EncParams mid = q;
-                mid.buildTier = 2;
-                mid.buildLo = kSmallLeaves + 1;
-                mid.buildHi = kBuildSplitLeaves;
-                k_tableBuild<kMidThreads, kBuildSplitLeaves>
-                    <<<std::min(p.T, 5u * sms), kMidThreads, hm::Layout<kBuildSplitLeaves>::kBytes, I->buildSide>>>(mid);
-                countLaunch();
-                CC_TRY_CUDA(cudaEventRecord(I->buildJoin, I->buildSide), "table build join");
-            }
-            EncParams tiny = q;
-            tiny.buildTier = 0;
-            tiny.buildHi = kTinyLeaves;
-            k_tableBuild<32u, kTinyLeaves>
-                <<<std::min(p.T, 32u * sms), 32, hm::Layout<kTinyLeaves>::kBytes, st>>>(tiny);
-            countLaunch();
-            if (side2) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->buildJoin2, 0), "table build join");
-            if (side) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->buildJoin, 0), "table build join");
-        } else {
-            if (!solo && p.heapCap <= kSmallLeaves)
-                k_tableBuild<kBuildThreads, kSmallLeaves>
-                    <<<p.T, kBuildThreads, hm::Layout<kSmallLeaves>::kBytes, st>>>(q);
-            else if (!solo && p.heapCap <= kBuildSplitLeaves)
-                k_tableBuild<kBuildThreads, kBuildSplitLeaves>
-                    <<<p.T, kBuildThreads, hm::Layout<kBuildSplitLeaves>::kBytes, st>>>(q);
-            else
-                k_tableBuild<kBigThreads, kBuildSmemLeaves><<<p.T, kBigThreads, buildSmem, st>>>(q);
-            countLaunch();
-        }
-    }
     // the block kernels walk the run list (k_planFill) with a few CTAs per SM
     const u32 blockGrid = u32(std::max(1, I->smCount > 0 ? I->smCount : 148)) * 8u;
     // runs of the call: at most the used blocks / blocks per run, plus one per table
@@ -1702,10 +1793,9 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
 int prepareDecodeAttributes(cc_instance* I);
 
 int prepareKernelAttributes(cc_instance* I) {
-    size_t buildSmem = hm::Layout<kBuildSmemLeaves>::kBytes;
-    if (I->tableBuildSoloSM) buildSmem = std::max(buildSmem, tableBuildSoloSmem(I->device));
-    CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_tableBuild<kBigThreads, kBuildSmemLeaves>),
-                                    kAttrTableBuild, I->device, buildSmem),
+    size_t bytes;
+    CC_TRY_CUDA(I->bins > kWideBins ? tableBuildSmem<true>(I, I->tableBuildSoloSM, bytes)
+                                    : tableBuildSmem<false>(I, I->tableBuildSoloSM, bytes),
                 "tableBuild smem");
     if (I->symBytes == 2)
         CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_write<u16>), kAttrWrite16, I->device,

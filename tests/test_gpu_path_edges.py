@@ -343,3 +343,29 @@ def test_counts_of_large_symbols(oracle, kind, bits):
     streams[6] = 760 + rng.integers(0, 16, n)
     with cc.Instance(0, 7, n, 128, 14 if bits == 16 else 20) as inst:
         roundtrip(oracle, inst, kind, streams, log2max=14 if bits == 16 else 20)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("S", [1, 40])
+@pytest.mark.parametrize("top", [31, 32, 63, 511, 512, 513, 4095, 4096, 4097, 65536, 300001])
+def test_leaves_spread_over_an_alphabet(oracle, kind, S, top):
+    """Few symbols in an alphabet of `top` + 1 bins, at the borders of the
+    warps' ranges and of their steps, the largest in the last bin."""
+    rng = np.random.default_rng(top)
+    at = np.array([1, 30, 31, 32, 33, 255, 256, 257, 511, 512, 1023, 8191, 8192, top // 2, top - 1, top])
+    at = np.unique(at[(at >= 1) & (at <= top)])
+    streams = rng.choice(at, (S, 600)).astype(np.uint32)
+    streams[:, 0] = top
+    with cc.Instance(0, S, 600, 128, 20) as inst:
+        roundtrip(oracle, inst, kind, streams, log2max=20)
+
+
+@pytest.mark.parametrize("leaves", [26626, 26627, 26628, 53254, 53255])
+def test_tables_around_the_sequential_builders_area(oracle, leaves):
+    """Leaf counts around what the builder's shared memory holds as a heap (8
+    bytes each) and as sort keys (4 bytes)."""
+    rng = np.random.default_rng(leaves)
+    n = 60000
+    v = rng.permutation(np.concatenate([np.arange(1, leaves + 1), rng.integers(1, 200, n - leaves)]))
+    with cc.Instance(0, 1, n, 128, 17) as inst:
+        roundtrip(oracle, inst, 1, v.astype(np.uint32)[None], log2max=17)
