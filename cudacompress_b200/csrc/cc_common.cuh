@@ -51,16 +51,6 @@ __device__ __forceinline__ u32 warpInclusiveSum(u32 v) {
     }
     return v;
 }
-__device__ __forceinline__ u32 warpSum(u32 v) {
-#pragma unroll
-    for (u32 o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ u32 warpMax(u32 v) {
-#pragma unroll
-    for (u32 o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 
 // Exclusive scan of in[0, n) into out by one warp (in == out allowed), each
 // lane taking eight consecutive elements per step; returns carry + the total.
@@ -183,15 +173,6 @@ __device__ __forceinline__ int quantizeV(float v, float inv, int type) {
 __device__ __forceinline__ float unquantizeV(int q, float step, int type) {
     if (type == 0) return (float(q) + signI(q) * 0.5f) * step;
     return float(q) * step;
-}
-
-// Warp-aggregated increment of `bins[key]`: lanes with equal keys are merged
-// with match_any so each distinct key issues one shared/global atomic.
-__device__ __forceinline__ void aggregatedIncrement(u32* bins, u32 key, bool active) {
-    const u32 mask = __ballot_sync(0xffffffffu, active);
-    if (!active) return;
-    const u32 peers = __match_any_sync(mask, key);
-    if ((threadIdx.x & 31u) == u32(__ffs(peers) - 1)) atomicAdd(bins + key, u32(__popc(peers)));
 }
 #endif
 

@@ -52,27 +52,9 @@ __device__ __forceinline__ float fir9c(const float* v) {
     return sum;
 }
 
-// Two outputs of one parity at once, their windows at a and b: Blackwell's
-// packed fma.rn.f32x2 does both lanes' fmaf in one instruction, each lane
-// rounded exactly as fir9c's scalar chain.
-template <bool kInverse, int kParity>
-__device__ __forceinline__ float2 fir9x2(const float* a, const float* b) {
-    constexpr float kF[2][9] = {
-        {0.0267488f, -0.0168641f, -0.0782233f, 0.2668641f, 0.6029490f, 0.2668641f, -0.0782233f, -0.0168641f, 0.0267488f},
-        {0.0f, 0.0456359f, -0.0287718f, -0.2956359f, 0.5575435f, -0.2956359f, -0.0287718f, 0.0456359f, 0.0f}};
-    constexpr float kI[2][9] = {
-        {0.0f, 0.0337282f, -0.0575435f, -0.5337281f, 1.1150871f, -0.5337281f, -0.0575435f, 0.0337282f, 0.0f},
-        {0.0534975f, -0.0912718f, -0.1564465f, 0.5912718f, 1.2058980f, 0.5912718f, -0.1564465f, -0.0912718f, 0.0534975f}};
-    float2 sum = make_float2(0.0f, 0.0f);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        const float c = kInverse ? kI[kParity][i] : kF[kParity][i];
-        sum = __ffma2_rn(make_float2(c, c), make_float2(a[i], b[i]), sum);
-    }
-    return sum;
-}
-
-// The same over a window of value pairs (lane x: one output, lane y: the other).
+// Two outputs of one parity at once over a window of value pairs (lane x: one
+// output, lane y: the other): Blackwell's packed fma.rn.f32x2 does both lanes'
+// fmaf in one instruction, each lane rounded exactly as fir9c's scalar chain.
 template <bool kInverse, int kParity>
 __device__ __forceinline__ float2 fir9p(const float2* w) {
     constexpr float kF[2][9] = {

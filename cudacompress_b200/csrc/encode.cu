@@ -359,11 +359,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scanWide(EncParams p) {
     if (threadIdx.x == 0) p.counts[s] = carry.cnt ? carry.cnt + carry.ext + (carry.firstP1 - 1u) / 256u : 0u;
 }
 
-// Which of them.  Up to 64 streams take a CTA each where one CTA's 32 warps
-// would take more than four steps over them all (0.7 us each; a launch of its
-// own for the scan costs 2.5 us): one warp or two per stream, which one CTA
-// then joins with the plan.  More streams: where the longest has more than 64
-// tiles, unless that many CTAs would take longer than its warp (2 us per 1184).
+// Which of them.  Up to 64 streams: one CTA scans them, a warp for one or two
+// streams, and makes the plan in the same launch, as long as its warps take at
+// most four steps (0.7 us each); a scan of its own costs a launch, 2.5 us (an
+// image's nine streams of 96 tiles: 476 us there and back with it, 469
+// without).  More streams: where the longest has more than 64 tiles, unless
+// that many CTAs would take longer than its warp (2 us per 1184).
 constexpr u32 kScanPlanStreams = 64;
 static bool scanWide(u32 streams, u32 tiles) {
     if (streams <= kScanPlanStreams) return ceilDiv(streams, 32) * ceilDiv(tiles, 32) > 4;
@@ -373,7 +374,8 @@ static bool scanWide(u32 streams, u32 tiles) {
 // Table builders by leaf count (k_leafTiers sorts the tables, k_tableBuild
 // builds them): the heap merge is a latency-bound chain on one warp, so a
 // smaller table gets a smaller CTA and heap and more of them share an SM.
-//   tier 0: up to 256 leaves, a warp, 5 KB of heap (32 per SM)
+//   tier 0: up to 256 leaves, a warp, 5 KB of heap (21 per SM, by registers;
+//           the grid has 32, those past the first 21 start as others end)
 //   tier 1: up to 1024 leaves, 64 threads, 20 KB (10 per SM)
 //   tier 2: up to 2048 leaves, 128 threads, 41 KB (5 per SM)
 //   tier 3: more, 512 threads, the full heap (one per SM)
@@ -394,20 +396,22 @@ constexpr u32 kTierMinTables = 64;                       // calls of more tables
 constexpr u32 kPlanPer = 4;
 static_assert(kPlanChunk == 1024 * kPlanPer, "a plan chunk is one 1024-thread CTA's tables");
 
-// The call's totals from the offsets' grand sums c[2..6] (bins, leaves,
+constexpr u32 kPlanSums = 5;   // bins, leaves, header words, coding blocks, runs
+
+// The call's totals from the offsets' grand sums c[0..4] (bins, leaves,
 // header words, coding blocks, runs), and the capacity check.
-__device__ __forceinline__ void planTotals(const EncParams& p, const unsigned long long (&c)[7]) {
-    p.totals[2] = c[5];
-    p.totals[3] = c[6];
+__device__ __forceinline__ void planTotals(const EncParams& p, const unsigned long long (&c)[kPlanSums]) {
+    p.totals[2] = c[3];
+    p.totals[3] = c[4];
     for (u32 k = 4; k < 8; ++k) p.totals[k] = 0;   // the tier lists' counts (k_leafTiers)
-    p.totals[1] = c[2];
-    if (c[2] > p.capHist || c[3] > p.capLeaves || c[4] > p.capHdr) atomicOr(p.errors, DEV_ERR_TABLE_CAPACITY);
+    p.totals[1] = c[0];
+    if (c[0] > p.capHist || c[1] > p.capLeaves || c[2] > p.capHdr) atomicOr(p.errors, DEV_ERR_TABLE_CAPACITY);
 }
 
 __device__ __forceinline__ void histPlanChunk(const EncParams& p, u32* scratch) {
     const u32 t0 = blockIdx.x * kPlanChunk + threadIdx.x * kPlanPer;
-    // per table: (unused), (unused), bins, leaves, header words, blocks, runs
-    u32 v[kPlanPer][7];
+    // per table: bins, leaves, header words, blocks, runs
+    u32 v[kPlanPer][kPlanSums];
     TableMeta m[kPlanPer];
 #pragma unroll
     for (u32 j = 0; j < kPlanPer; ++j) {
@@ -426,60 +430,58 @@ __device__ __forceinline__ void histPlanChunk(const EncParams& p, u32* scratch) 
             m[j].histSize = hs;
             m[j].blocks = blocksOf(count, p.cbLog);
         }
-        v[j][0] = 0;
-        v[j][1] = 0;
-        v[j][2] = hs;
-        v[j][3] = ls;
-        v[j][4] = ws;
-        v[j][5] = m[j].blocks;
-        v[j][6] = blocksOf(m[j].blocks, kRunLog - p.cbLog);
+        v[j][0] = hs;
+        v[j][1] = ls;
+        v[j][2] = ws;
+        v[j][3] = m[j].blocks;
+        v[j][4] = blocksOf(m[j].blocks, kRunLog - p.cbLog);
     }
-    u32 sum[7], ex[7], tot[7];
+    u32 sum[kPlanSums], ex[kPlanSums], tot[kPlanSums];
 #pragma unroll
-    for (u32 k = 0; k < 7; ++k) {
+    for (u32 k = 0; k < kPlanSums; ++k) {
         sum[k] = 0;
 #pragma unroll
         for (u32 j = 0; j < kPlanPer; ++j) sum[k] += v[j][k];
     }
-    blockExclusiveSumN<1024, 7>(sum, ex, tot, scratch);
-    unsigned long long at[7];
+    blockExclusiveSumN<1024, kPlanSums>(sum, ex, tot, scratch);
+    unsigned long long at[kPlanSums];
 #pragma unroll
-    for (u32 k = 0; k < 7; ++k) at[k] = ex[k];
+    for (u32 k = 0; k < kPlanSums; ++k) at[k] = ex[k];
 #pragma unroll
     for (u32 j = 0; j < kPlanPer; ++j) {
         const u32 t = t0 + j;
         if (t < p.T) {
-            m[j].histOff = at[2];
-            m[j].leafOff = at[3];
-            m[j].hdrOff = at[4];
-            m[j].runOff = u32(at[6]);
+            m[j].histOff = at[0];
+            m[j].leafOff = at[1];
+            m[j].hdrOff = at[2];
+            m[j].runOff = u32(at[4]);
             p.meta[t] = m[j];
         }
 #pragma unroll
-        for (u32 k = 0; k < 7; ++k) at[k] += v[j][k];
+        for (u32 k = 0; k < kPlanSums; ++k) at[k] += v[j][k];
     }
     if (threadIdx.x == 0) {
         if (gridDim.x == 1) {
-            unsigned long long c[7];
+            unsigned long long c[kPlanSums];
 #pragma unroll
-            for (u32 k = 0; k < 7; ++k) c[k] = tot[k];
+            for (u32 k = 0; k < kPlanSums; ++k) c[k] = tot[k];
             planTotals(p, c);
         } else {
 #pragma unroll
-            for (u32 k = 0; k < 7; ++k) p.planPart[u64(blockIdx.x) * 8 + k] = tot[k];
+            for (u32 k = 0; k < kPlanSums; ++k) p.planPart[u64(blockIdx.x) * 8 + k] = tot[k];
         }
     }
 }
 
 __global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
-    __shared__ u32 scratch[33 * 7];
+    __shared__ u32 scratch[33 * kPlanSums];
     histPlanChunk(p, scratch);
 }
 
 // Passes 2 and 3 of a call of few and short streams in one CTA (scanWide).
 
 __global__ void __launch_bounds__(1024) k_scanPlan(EncParams p) {
-    __shared__ u32 scratch[33 * 7];
+    __shared__ u32 scratch[33 * kPlanSums];
     for (u32 s = threadIdx.x >> 5; s < p.S; s += 32) scanStream(p, s);
     __syncthreads();   // the CTA's counts
     histPlanChunk(p, scratch);
@@ -489,20 +491,20 @@ __global__ void __launch_bounds__(1024) k_scanPlan(EncParams p) {
 // chunks 0 .. b-1 (a warp over planPart) added to its tables' offsets; the
 // last chunk's CTA forms the call's totals.
 __global__ void __launch_bounds__(1024) k_histPlanCarry(EncParams p) {
-    __shared__ unsigned long long sC[7];
+    __shared__ unsigned long long sC[kPlanSums];
     const u32 b = blockIdx.x + 1;
     if (threadIdx.x < 32) {
-        unsigned long long c[7] = {0, 0, 0, 0, 0, 0, 0};
+        unsigned long long c[kPlanSums] = {0, 0, 0, 0, 0};
         for (u32 i = threadIdx.x; i < b; i += 32)
 #pragma unroll
-            for (u32 k = 2; k < 7; ++k) c[k] += p.planPart[u64(i) * 8 + k];
+            for (u32 k = 0; k < kPlanSums; ++k) c[k] += p.planPart[u64(i) * 8 + k];
 #pragma unroll
-        for (u32 k = 2; k < 7; ++k)
+        for (u32 k = 0; k < kPlanSums; ++k)
 #pragma unroll
             for (u32 o = 16; o > 0; o >>= 1) c[k] += __shfl_xor_sync(0xffffffffu, c[k], o);
         if (threadIdx.x == 0)
 #pragma unroll
-            for (u32 k = 0; k < 7; ++k) sC[k] = c[k];
+            for (u32 k = 0; k < kPlanSums; ++k) sC[k] = c[k];
     }
     __syncthreads();
     const u32 t0 = b * kPlanChunk + threadIdx.x * kPlanPer;
@@ -511,16 +513,16 @@ __global__ void __launch_bounds__(1024) k_histPlanCarry(EncParams p) {
         const u32 t = t0 + j;
         if (t < p.T) {
             TableMeta& m = p.meta[t];
-            m.histOff += sC[2];
-            m.leafOff += sC[3];
-            m.hdrOff += sC[4];
-            m.runOff += u32(sC[6]);
+            m.histOff += sC[0];
+            m.leafOff += sC[1];
+            m.hdrOff += sC[2];
+            m.runOff += u32(sC[4]);
         }
     }
     if (b == gridDim.x && threadIdx.x == 0) {
-        unsigned long long c[7];
+        unsigned long long c[kPlanSums];
 #pragma unroll
-        for (u32 k = 0; k < 7; ++k) c[k] = sC[k] + p.planPart[u64(b) * 8 + k];
+        for (u32 k = 0; k < kPlanSums; ++k) c[k] = sC[k] + p.planPart[u64(b) * 8 + k];
         planTotals(p, c);
     }
 }
@@ -574,11 +576,11 @@ __global__ void __launch_bounds__(256) k_leafTiers(EncParams p) {
 // arrays, and copied out by them.  The eight most frequent keys of each
 // histogram (zero counts 0..7, symbols 1..8) are counted in the lane's
 // registers on the way, the others with shared-memory atomics.  The stage
-// (dynamic shared memory) holds a whole tile's entries for 16-bit symbols - up
-// to one per symbol, plus the (0, 255) entries of zero runs inside the tile -
-// so only a tile that a zero run of millions of symbols ends in writes its
-// entries directly.  Bound: instruction issue; walking a group's nonzeros on
-// its lane instead of a group's lanes together took three 256^3 streams'
+// (dynamic shared memory) holds an entry per symbol and eight more for 16-bit
+// symbols, half as many for 32-bit ones.  A tile of more - all nonzero after a
+// run of 2304 zeros, one nonzero after 526336, 32-bit symbols mostly nonzero -
+// writes its entries directly.  Bound: instruction issue; walking a group's
+// nonzeros on its lane instead of a group's lanes together took three 256^3 streams'
 // highpass bands (50 million symbols, 26 million entries) from 191 to 123 us.
 constexpr u32 kWriteSymBins = 768;   // symbol bins counted in shared memory by k_write
 
@@ -1134,7 +1136,7 @@ __device__ __forceinline__ void buildTable(const EncParams& p, u32 t) {
 }
 
 // One table per CTA (kBuildEach), or the CTAs walk the list of one tier.
-// Bounding the one-warp tier to 72 registers (28 CTAs per SM instead of 20)
+// Bounding the one-warp tier to 72 registers (28 CTAs per SM instead of 21)
 // left 4096 bricks at the same time.
 template <u32 kThreads, u32 kCap, bool kWide>
 __global__ void __launch_bounds__(kThreads, 1) k_tableBuild(EncParams p) {
