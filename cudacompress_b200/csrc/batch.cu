@@ -309,7 +309,7 @@ static int batchEnqueueCompress(cc_volume_batch* b) {
     // chain of few large volumes, and their CTAs wait while the highpass write
     // fills every SM: then it comes after them.  Started first it delayed them
     // to its end, 126 us of a 1024 us pass over three 256^3 volumes.
-    const u32 sms = u32(std::max(1, ILP->smCount > 0 ? ILP->smCount : 148));
+    const u32 sms = ILP->smCount;
     const bool solo = k <= sms && b->encTiles[k - 1] >= sms;
     ILP->encBuildNext = solo ? b->evBuild : nullptr;
     I->encFillAfter = ILP->encBuildNext;
@@ -567,7 +567,6 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
     b->ILP->timing = false;   // follows the user instance's timing on each compress call
     // the lowpass tables are built while the highpass encode runs: one SM each
     b->ILP->tableBuildSoloSM = true;
-    cudaDeviceGetAttribute(&b->ILP->smCount, cudaDevAttrMultiProcessorCount, user->device);
     // kernel attributes set once here, so that captured launches do not set them
     rc = prepareKernelAttributes(I);
     if (!rc) rc = prepareKernelAttributes(b->ILP);
@@ -620,7 +619,7 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
     // the forward level's tile depth, unless the caller gives one
     std::vector<u32> depth(L, zChunk);
     if (zChunk == 0) {
-        const u32 sms = u32(std::max(1, b->ILP->smCount > 0 ? b->ILP->smCount : 148));
+        const u32 sms = b->ILP->smCount;
         for (u32 l = 0; l < L; ++l) {
             auto ctas = [&](u32 zc) {
                 u64 n = 0;
@@ -1019,7 +1018,7 @@ int cc_volume_batch_download_streams(cc_volume_batch* b, uint32_t* hWords, uint6
     cudaStream_t st = b->hasOwnStream ? b->ownStream : b->user->stream;
     b->I->stream = st;
     const bool vec = (reinterpret_cast<uintptr_t>(dW) & 15) == 0;
-    const unsigned g = 148 * 4;
+    const unsigned g = b->I->smCount * 4;
     if (vec) k_streamsToHost<true><<<g, 256, 0, st>>>(b->words, b->wordOff, b->bitSize, b->active, static_cast<u32*>(dW), capacityWords, static_cast<u64*>(dE), b->I->errors);
     else k_streamsToHost<false><<<g, 256, 0, st>>>(b->words, b->wordOff, b->bitSize, b->active, static_cast<u32*>(dW), capacityWords, static_cast<u64*>(dE), b->I->errors);
     countLaunch();
@@ -1038,7 +1037,7 @@ int cc_volume_batch_upload_streams(cc_volume_batch* b, const uint32_t* hWords, c
     cudaStream_t st = b->hasOwnStream ? b->ownStream : b->user->stream;
     b->I->stream = st;
     const bool vec = (reinterpret_cast<uintptr_t>(dW) & 15) == 0;
-    const unsigned g = 148 * 4;
+    const unsigned g = b->I->smCount * 4;
     if (vec) k_streamsFromHost<true><<<g, 256, 0, st>>>(static_cast<const u32*>(dW), static_cast<const u64*>(dE), b->active, b->words, b->wordOff, b->bitSize, b->wordsCap, b->I->errors + 4);
     else k_streamsFromHost<false><<<g, 256, 0, st>>>(static_cast<const u32*>(dW), static_cast<const u64*>(dE), b->active, b->words, b->wordOff, b->bitSize, b->wordsCap, b->I->errors + 4);
     countLaunch();

@@ -39,6 +39,15 @@ constexpr u32 kRunSymbols = 1u << kRunLog;
 // threads, four tables each); a call of more tables runs one CTA per chunk
 // and a carry pass over the chunks' sums (planPart).
 constexpr u32 kPlanChunk = 4096;
+
+// The per-stream scans over coding blocks (block bits, run lengths) take a warp
+// per stream, or 512 threads where the call's longest stream has kLongBlocks
+// blocks or more and all CTAs are resident at once.  Seven streams of 1024
+// blocks: 3.4 us by a warp each, 2.9 wide; of 8192 8.4 and 4.1; 580 tables of
+// six blocks 2.5 and 4.7.
+constexpr u32 kLongBlocks = 1024;
+constexpr u32 kWidePerSM = 4;   // resident CTAs of 512 threads
+inline bool wideScan(u32 streams, u32 longest, u32 sms) { return longest >= kLongBlocks && streams <= kWidePerSM * sms; }
 constexpr u64 planPartWords(u64 tables) { return 8 * ((tables + kPlanChunk - 1) / kPlanChunk + 1); }
 
 // Leaves of a table whose Huffman build runs in shared memory (heap_merge.cuh's
@@ -268,7 +277,7 @@ struct cc_instance {
     ccb::u64 stagedWordsMax = 0;
     ccb::u32* blockSum = nullptr;             // [capBlocks]
     bool tableBuildSoloSM = false;            // table-build CTAs ask for a whole SM (calls of <= smCount tables)
-    int smCount = 148;
+    ccb::u32 smCount = 148;                   // multiprocessors of the device
     ccb::u64* decRlTasks = nullptr;           // [capBlocks / 32 + capStreams + 1]: run-length decode warp tasks, then their count
 
     // host staging: ring of slots for uploads, one buffer for downloads

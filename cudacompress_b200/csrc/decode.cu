@@ -27,7 +27,7 @@ namespace ccb {
 struct DecParams {
     u32 S, T, nSrc, nRl, nH;
     u32 rlBlocks, hBlocks;     // coding blocks (upper bounds) of the RLHuff / Huff streams
-    u32 rlMaxN;                // largest output of an RLHuff stream
+    u32 rlMaxN, maxN;          // largest output of an RLHuff stream, and of any
     u32 cb, cbLog, log2Max, symBytes, leavesMax;   // cb = 2^cbLog
     u64 capLeaves;
     DecStreamDesc* streams;
@@ -312,9 +312,11 @@ __global__ void __launch_bounds__(1024) k_decSymPlanCarry(DecParams p) {
 // One CTA per table: 64 threads in calls of many tables (up to 32 tables per
 // SM: the work per table is a short chain of dependent steps), 512 in calls of
 // few, where the offsets of a long stream's blocks - 8 per thread and step -
-// and the lookup table take the time (129 tables of 256^3 streams: 35 -> 18 us).
+// and the lookup table take the time (129 tables of 256^3 streams: 35 -> 18
+// us): a table per SM, or as wideScan has it.  120 tables of six blocks 7.7 us
+// and 6.2 wide, 580 of them 7.9 and 11.9; 400 of 1024 blocks 8.4 and 8.3, of
+// 2048 10.0 and 8.8.
 constexpr u32 kDecThreads = 64, kDecThreadsWide = 512;
-constexpr u32 kDecWideTables = 4 * 148;   // tables of a call that the wide CTAs hold at once
 
 template <u32 kDecThreads>
 __global__ void __launch_bounds__(kDecThreads) k_decTables(DecParams p) {
@@ -1031,8 +1033,8 @@ __global__ void __launch_bounds__(256) k_decScan(DecParams p) {
     if ((threadIdx.x & 31u) == 0 && total > sd.n) atomicOr(p.errors, DEV_ERR_CORRUPT);
 }
 
-// The same with a CTA per stream, for calls of few: a warp takes 38 us over the
-// 16384 blocks of a 256^3 volume's band, 512 threads 13.
+// The same with a CTA per stream (wideScan): a warp takes 38 us over the 16384
+// blocks of a 256^3 volume's band, 512 threads 13.
 __global__ void __launch_bounds__(512) k_decScanWide(DecParams p) {
     __shared__ u32 scratch[40];
     const DecStreamDesc sd = p.streams[p.rlList[blockIdx.x]];
@@ -1134,6 +1136,7 @@ static int planDecode(cc_instance* I, const u32* kinds, const u32* ns, void* con
         d.out = outs[s];
         d.n = ns[s];
         d.m = ns[s];
+        dc.maxN = std::max<u32>(dc.maxN, ns[s]);
         d.kind = kinds[s];
         d.tableFirst = t;
         d.source = sourceOf[s];
@@ -1240,7 +1243,7 @@ static int launchDecodeBackEnd(cc_instance* I, const DecParams& p) {
     }
     {
         SectionTimer t(I, "dec.tables", st);
-        if (p.T <= kDecWideTables) k_decTables<kDecThreadsWide><<<p.T, kDecThreadsWide, 0, st>>>(p);
+        if (p.T <= I->smCount || wideScan(p.T, u32(ceilDiv(p.maxN, p.cb)), I->smCount)) k_decTables<kDecThreadsWide><<<p.T, kDecThreadsWide, 0, st>>>(p);
         else k_decTables<kDecThreads><<<p.T, kDecThreads, 0, st>>>(p);
         countLaunch();
     }
@@ -1269,7 +1272,7 @@ static int launchDecodeBackEnd(cc_instance* I, const DecParams& p) {
         }
         {
             SectionTimer t(I, "dec.run_scan", st);
-            if (p.nRl <= kDecWideTables) k_decScanWide<<<p.nRl, 512, 0, st>>>(p);
+            if (wideScan(p.nRl, u32(ceilDiv(p.rlMaxN, p.cb)), I->smCount)) k_decScanWide<<<p.nRl, 512, 0, st>>>(p);
             else k_decScan<<<u32(ceilDiv(p.nRl, 8)), 256, 0, st>>>(p);
             countLaunch();
         }
@@ -1299,6 +1302,7 @@ static DecParams makeDecParams(cc_instance* I, const DecPlan& dc) {
     p.nH = dc.nH;
     p.rlBlocks = dc.rlBlocks;
     p.rlMaxN = dc.rlMaxN;
+    p.maxN = dc.maxN;
     p.hBlocks = dc.hBlocks;
     p.cb = I->codingBlockSize;
     p.cbLog = 31u - u32(__builtin_clz(p.cb));

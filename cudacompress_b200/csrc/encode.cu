@@ -23,7 +23,7 @@ namespace ccb {
 struct EncParams {
     u32 S, T;
     u32 totalTiles, totalBlocks;
-    u32 maxTiles;     // of the longest stream
+    u32 maxCount;     // symbols of the longest stream
     u32 cb, cbLog, log2Max, bins, symBytes;   // cb = 2^cbLog
     const EncStreamDev* streams;
     const EncTableDev* tables;
@@ -1254,9 +1254,8 @@ __global__ void __launch_bounds__(kScanWarps * 32) k_blockScan(EncParams p) {
     if ((threadIdx.x & 31u) == 0) p.meta[t].codeBits = total;
 }
 
-// The same with a CTA per table, for calls of few tables: 512 threads over the
-// 16384 blocks of a 256^3 volume's band take 6 us, a warp 25.
-constexpr u32 kWideScanTables = 4 * 148;
+// The same with a CTA per table (wideScan): 512 threads over the 16384 blocks of
+// a 256^3 volume's band take 6 us, a warp 25.
 
 __global__ void __launch_bounds__(512) k_blockScanWide(EncParams p) {
     __shared__ u32 scratch[40];
@@ -1636,7 +1635,7 @@ static cudaError_t tableBuildSmem(const cc_instance* I, bool solo, size_t& bytes
 template <bool kWide>
 static int launchTableBuild(cc_instance* I, const EncParams& p) {
     cudaStream_t st = I->stream;
-    const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
+    const u32 sms = I->smCount;
     // an instance whose tables run beside other kernels (the batched codec's
     // lowpass encode) may ask for an SM of its own per table: the sequential
     // heap merge is latency-bound and loses issue slots to co-resident CTAs
@@ -1720,7 +1719,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
     countLaunch();
     if (p.totalTiles) { SectionTimer t(I, "enc.summary", st); k_summary<Sym><<<p.totalTiles, kRleThreads, 0, st>>>(p); countLaunch(); }
     const u32 chunks = std::max<u32>(1, u32(ceilDiv(p.T, kPlanChunk)));
-    const bool wide = scanWide(p.S, p.maxTiles);
+    const bool wide = scanWide(p.S, u32(ceilDiv(p.maxCount, kRleTile)));
     if (p.S <= kScanPlanStreams && !wide) {   // then one chunk
         SectionTimer t(I, "enc.hist_plan", st);
         k_scanPlan<<<1, 1024, 0, st>>>(p);
@@ -1738,7 +1737,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         if (chunks > 1) { k_histPlanCarry<<<chunks - 1, 1024, 0, st>>>(p); countLaunch(); }
     }
     if (I->encFillAfter) CC_TRY_CUDA(cudaStreamWaitEvent(st, I->encFillAfter, 0), "encode order");
-    { SectionTimer t(I, "enc.hist_zero", st); k_planFill<<<2 * 148, 256, 0, st>>>(p); countLaunch(); }
+    { SectionTimer t(I, "enc.hist_zero", st); k_planFill<<<2 * I->smCount, 256, 0, st>>>(p); countLaunch(); }
     if (p.totalTiles) {
         CC_TRY_CUDA(ensureSmemAttribute(reinterpret_cast<const void*>(k_write<Sym>),
                                         sizeof(Sym) == 2 ? kAttrWrite16 : kAttrWrite32, I->device, writeSmem<Sym>()),
@@ -1750,9 +1749,9 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
     if (I->encBuildNext) CC_TRY_CUDA(cudaEventRecord(I->encBuildNext, st), "encode order");
     int rc = p.bins > kWideBins ? launchTableBuild<true>(I, p) : launchTableBuild<false>(I, p);
     if (rc) return rc;
-    const u32 sms = u32(std::max(1, I->smCount > 0 ? I->smCount : 148));
+    const u32 sms = I->smCount;
     // the block kernels walk the run list (k_planFill) with a few CTAs per SM
-    const u32 blockGrid = u32(std::max(1, I->smCount > 0 ? I->smCount : 148)) * 8u;
+    const u32 blockGrid = sms * 8u;
     // runs of the call: at most the used blocks / blocks per run, plus one per table
     const u32 runBound = u32(ceilDiv(p.totalBlocks, kRunSymbols / p.cb)) + p.T;
     if (p.totalBlocks) {
@@ -1760,7 +1759,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         { SectionTimer t(I, "enc.block_bits", st); k_blockBits<Sym><<<g, kPackWarps * 32, 0, st>>>(p); countLaunch(); }
         {
             SectionTimer t(I, "enc.block_scan", st);
-            if (p.T <= kWideScanTables) k_blockScanWide<<<p.T, 512, 0, st>>>(p);
+            if (wideScan(p.T, u32(ceilDiv(p.maxCount, p.cb)), sms)) k_blockScanWide<<<p.T, 512, 0, st>>>(p);
             else k_blockScan<<<u32(ceilDiv(p.T, kScanWarps)), kScanWarps * 32, 0, st>>>(p);
             countLaunch();
         }
@@ -1822,7 +1821,7 @@ int encodeLaunch(cc_instance* I, const EncPlan& hp, u32* out, u64 outCap) {
     p.S = hp.S;
     p.T = hp.T;
     p.totalTiles = hp.tiles;
-    p.maxTiles = u32(ceilDiv(hp.maxCount, kRleTile));
+    p.maxCount = hp.maxCount;
     p.totalBlocks = hp.blocks;
     p.cb = I->codingBlockSize;
     p.cbLog = 31u - u32(__builtin_clz(p.cb));

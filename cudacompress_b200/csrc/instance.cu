@@ -248,6 +248,8 @@ int createInstance(cc_instance** out, int cudaDevice, u32 streamCountMax, u32 el
     }
     cc_instance* I = new cc_instance();
     I->device = cudaDevice;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cudaDevice) == cudaSuccess && sms > 0) I->smCount = u32(sms);
     I->streamCountMax = streamCountMax;
     I->elemCountPerStreamMax = elemCountPerStreamMax;
     I->codingBlockSize = codingBlockSize;

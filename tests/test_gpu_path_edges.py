@@ -91,6 +91,25 @@ def test_float_transform_in_place_2d(oracle, shape):
     assert same(host(t), oracle.dwt_float(fwd, inverse=True))
 
 
+@pytest.mark.parametrize("shape", [(8, 8, 8), (10, 62, 130), (66, 72, 64)])
+@pytest.mark.parametrize("alias", ["buf2=src", "buf2=dst"])
+def test_float_transform_3d_aliases(oracle, shape, alias):
+    """Arrays that a plane pass would read and write at once: the source in
+    the second buffer (forward), the second buffer in the destination
+    (inverse); X and Y then go through the first one."""
+    rng = np.random.default_rng(sum(shape))
+    a = rng.standard_normal(shape).astype(np.float32)
+    nz, ny, nx = shape
+    fwd = oracle.dwt_float(a)
+    src, dst, b1 = dev(a), dev(np.zeros_like(a)), dev(np.zeros_like(a))
+    if alias == "buf2=src":
+        cc.dwt_float_forward(dst, src, b1, src, nx, ny, nz)
+        assert same(host(dst), fwd)
+    else:
+        cc.dwt_float_inverse(dst, dst, b1, dev(fwd), nx, ny, nz)
+        assert same(host(dst), oracle.dwt_float(fwd, inverse=True))
+
+
 @pytest.mark.parametrize("shape", [(8, 8, 8), (1, 8, 8), (8, 10, 12), (1, 34, 66), (1, 66, 258), (10, 66, 34), (34, 8, 8),
                                    (1, 258, 520)])
 @pytest.mark.parametrize("pad,shift", [(0, 0), (1, 1), (2, 2), (4, 4)])
@@ -229,6 +248,22 @@ def test_streams_around_a_step_of_the_tile_scan(oracle, n):
         roundtrip(oracle, inst, 0, streams)
 
 
+@pytest.mark.parametrize("zeros,dense", [(2303, 2048), (2304, 2048), (2305, 2047), (2056 * 256 - 1, 1), (2056 * 256, 1),
+                                         (2056 * 256 + 255, 1), (1 << 20, 1200)])
+def test_tiles_around_the_write_stage(oracle, zeros, dense):
+    """A tile of 2048 symbols with 2056 entries, which its stage holds, and
+    with more: `dense` nonzeros from its start on after a run of `zeros`."""
+    rng = np.random.default_rng(zeros + dense)
+    start = (zeros + 1 + 2047) // 2048 * 2048
+    n = start + 3 * 2048 + 11
+    streams = np.zeros((2, n), np.uint16)
+    streams[0, start - zeros - 1] = 9
+    streams[0, start:start + dense] = rng.integers(1, 30, dense)
+    streams[1] = np.roll(streams[0], 5)   # compact arrays that start off a 16-byte boundary
+    with cc.Instance(0, 2, n, 128, 14) as inst:
+        roundtrip(oracle, inst, 0, streams)
+
+
 @pytest.mark.parametrize("S,tiles", [(1, 128), (1, 129), (2, 511), (2, 512), (2, 513), (1, 1090), (33, 64), (33, 65), (64, 65),
                                      (65, 64), (65, 65)])
 def test_long_streams_of_the_tile_scan(oracle, S, tiles):
@@ -303,10 +338,11 @@ def test_wide_symbols(oracle, kind, n, shift):
         roundtrip(oracle, inst, kind, streams, log2max=20, shift=shift)
 
 
-@pytest.mark.parametrize("kind,S", [(0, 7), (0, 296), (0, 297), (1, 1), (1, 592), (1, 593)])
+@pytest.mark.parametrize("kind,S", [(0, 7), (0, 74), (0, 75), (0, 296), (0, 297), (1, 1), (1, 148), (1, 149), (1, 592),
+                                    (1, 593)])
 def test_wide_symbol_tables_of_many_streams(oracle, kind, S):
     """Decode tables of 32-bit symbols, whose table kernel has no barrier
-    between the symbols and the block offsets: both CTA widths (up to 592
+    between the symbols and the block offsets: both CTA widths (up to 148
     tables and more), tables of one leaf to hundreds, several times over.
     No warp may miss its share of a table: a guard reads the table's state
     while another warp goes on to its block offsets."""
@@ -369,3 +405,62 @@ def test_tables_around_the_sequential_builders_area(oracle, leaves):
     v = rng.permutation(np.concatenate([np.arange(1, leaves + 1), rng.integers(1, 200, n - leaves)]))
     with cc.Instance(0, 1, n, 128, 17) as inst:
         roundtrip(oracle, inst, 1, v.astype(np.uint32)[None], log2max=17)
+
+
+@pytest.mark.parametrize("cb", [32, 128])
+@pytest.mark.parametrize("streams", [1, 3])
+def test_zero_counts_past_a_byte(oracle, cb, streams):
+    """Streams with zero counts up to 65535, which the encoder does not write
+    (it splits runs at 256) but the format's tables can hold: rounds of 32
+    entries within 65536 positions, and longer ones.  A run-length stream is
+    its entry count and the two arrays' Huff streams."""
+    rng = np.random.default_rng(cb)
+    parts, expect, n = [], [], 1 << 21
+    for k in range(streams):
+        zc = np.concatenate([np.full(32, 2046), [0, 65535], rng.integers(0, 40000, 30), rng.integers(0, 256, 64),
+                             [65535], np.full(31, 0), rng.integers(200, 3000, 77 + k)]).astype(np.uint16)
+        sym = rng.integers(1, 50, len(zc)).astype(np.uint16)
+        at = np.cumsum(zc.astype(np.int64) + 1) - 1
+        assert at[-1] < n and int((zc[:32].astype(int) + 1).sum()) <= 65536 < int((zc[32:64].astype(int) + 1).sum())
+        out = np.zeros(n, np.uint16)
+        out[at] = sym
+        expect.append(out)
+        parts.append(np.array([len(zc)], np.uint32))
+        for a in (sym, zc):
+            words, bits, _ = oracle.encode(1, a[None], cb=cb, log2max=16)
+            parts.append(words[: (bits + 31) // 32])
+    words = np.concatenate(parts).astype(np.uint32)
+    with cc.Instance(0, streams, n, cb, 16) as inst:
+        outs = torch.full((streams, n), -1, dtype=torch.int16, device="cuda")
+        assert cc.decode_rlhuff(inst, cc.BitStream(words, 32 * len(words)), list(outs), n), cc.last_error()
+        assert cc.decode_status(inst) == 0
+        assert np.array_equal(host(outs).view(np.uint16), np.stack(expect))
+
+
+def test_forward_depths_of_uneven_levels(oracle):
+    """Batches whose levels take different tile depths by the rule: with 148
+    multiprocessors 8 volumes of 64^3 and near it 8 slices at every level, 24
+    take 16 at level 0, 40 take 32, 100 also 16 at level 1."""
+    shapes = [(64, 64, 64), (64, 48, 64), (48, 64, 56), (64, 64, 40)]
+    field = fields.turbulence_field(64, 256, 21, seed=5)
+    distinct = [np.ascontiguousarray(field[: s[0], : s[1], : s[2]]) for s in shapes]
+    refs = [oracle.compress_volume(v, 3, 0.01) for v in distinct]
+    for count in (8, 24, 40, 100):
+        vols = [dev(distinct[i % 4]) for i in range(count)]
+        with cc.Instance(0, 8, 64 ** 3, 128, 14) as inst, \
+                cc.VolumeBatch(inst, [tuple(v.shape) for v in vols], 3, [0.01] * count) as batch:
+            batch.compress(vols)
+            batch.status()
+            for i in range(count):
+                words, bits = batch.read_stream(i)
+                assert bits == refs[i % 4][1] and np.array_equal(words, refs[i % 4][0])
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("S,blocks", [(3, 1023), (3, 1024), (80, 5), (160, 5), (300, 5), (2, 9000)])
+def test_block_scans_by_length(oracle, kind, S, blocks):
+    """Both sides of the rules for a block per stream in the scans over coding
+    blocks and in the table kernel: lengths and stream counts."""
+    n = 32 * blocks - 3
+    with cc.Instance(0, S, n, 32, 14) as inst:
+        roundtrip(oracle, inst, kind, symbol_streams("sparse", S, n, seed=S + blocks), cb=32)
