@@ -90,7 +90,7 @@ struct cc_volume_batch {
     bool hasOwnStream = false;
     // graphs
     bool useGraph = false;
-    std::map<ccb::u32, cudaGraphExec_t> gCompress, gDecompress;   // by active count
+    std::map<ccb::u32, cudaGraphExec_t> gCompress, gDecompress;   // by active count and kind of priority (runMaybeGraph)
     cudaStream_t captureStream = nullptr;
     std::map<ccb::u32, unsigned> launchesCompress, launchesDecompress;
 };
@@ -307,8 +307,10 @@ static int batchEnqueueCompress(cc_volume_batch* b) {
     int rc;
     // The lowpass tables, built on an SM of their own each, are the longest
     // chain of few large volumes, and their CTAs wait while the highpass write
-    // fills every SM: then it comes after them.  Started first it delayed them
-    // to its end, 126 us of a 1024 us pass over three 256^3 volumes.
+    // fills every SM: then it comes after them, and their stream has priority
+    // (in most graphs the order alone does, in some the write still came
+    // first).  Started first it delayed them to its end, 126 us of a 1024 us
+    // pass over three 256^3 volumes.
     const u32 sms = ILP->smCount;
     const bool solo = k <= sms && b->encTiles[k - 1] >= sms;
     ILP->encBuildNext = solo ? b->evBuild : nullptr;
@@ -394,8 +396,13 @@ static int runMaybeGraph(cc_volume_batch* b, Enqueue fn, std::map<u32, cudaGraph
                          std::map<u32, unsigned>& counts) {
     cc_instance* I = b->I;
     if (!b->useGraph) return fn(b);
-    cudaGraphExec_t& exec = graphs[b->active];
-    unsigned& launches = counts[b->active];
+    // A graph runs at its nodes' priorities (the side stream's may be the
+    // highest), for a stream of other than the default priority at that stream's.
+    int priority = 0;
+    CC_TRY_CUDA(cudaStreamGetPriority(I->stream, &priority), "stream priority");
+    const u32 key = b->active | (priority ? 1u << 31 : 0u);
+    cudaGraphExec_t& exec = graphs[key];
+    unsigned& launches = counts[key];
     if (!exec) {
         // Capture on the batch's own stream (the instance stream may be the
         // legacy default stream, which cannot be captured); the graph is then
@@ -424,7 +431,7 @@ static int runMaybeGraph(cc_volume_batch* b, Enqueue fn, std::map<u32, cudaGraph
         if (rc) { if (g) cudaGraphDestroy(g); return rc; }
         if (e != cudaSuccess) return cudaFail(e, "end capture");
         launches = unsigned(cc_kernel_launches() - c0);
-        e = cudaGraphInstantiate(&exec, g, 0);
+        e = cudaGraphInstantiate(&exec, g, priority ? 0 : cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) { exec = nullptr; return cudaFail(e, "graph instantiate"); }
     }
@@ -571,7 +578,12 @@ int cc_volume_batch_create_ex(cc_instance* user, uint32_t count, const uint32_t*
     rc = prepareKernelAttributes(I);
     if (!rc) rc = prepareKernelAttributes(b->ILP);
     if (rc) { cc_volume_batch_destroy(b); return rc; }
-    cudaError_t ce = cudaStreamCreateWithFlags(&b->sideStream, cudaStreamNonBlocking);
+    int least = 0, greatest = 0;
+    cudaError_t ce = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    // of the highest priority where every lowpass table has an SM of its own
+    // (4096 bricks, whose highpass encode is the longer, lost 1% by it)
+    if (ce == cudaSuccess)
+        ce = cudaStreamCreateWithPriority(&b->sideStream, cudaStreamNonBlocking, count <= b->ILP->smCount ? greatest : 0);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&b->evFork, cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&b->evJoin, cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&b->evBuild, cudaEventDisableTiming);

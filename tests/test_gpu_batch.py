@@ -241,3 +241,26 @@ def test_tile_depth_out_of_range_is_rejected():
         for bad in (4, 9, 257):
             with pytest.raises(cc.CudaCompressError):
                 cc.VolumeBatch(inst, [v.shape for v in vols], 2, steps, z_chunk=bad)
+
+
+def test_batch_on_a_stream_of_priority(oracle):
+    """Graphs of a batch whose stream changes between the default and another
+    priority, back and forth: the same streams and reconstructions."""
+    vols = [np.ascontiguousarray(fields.turbulence_field(48, 192, 24, seed=s)) for s in (1, 2)]
+    refs = [oracle.compress_volume(v, 2, 0.01) for v in vols]
+    outs = [oracle.decompress_volume(w, b, v.shape, 2, 0.01) for v, (w, b) in zip(vols, refs)]
+    dv = [torch.from_numpy(v).cuda() for v in vols]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream(priority=-1), torch.cuda.Stream()]
+    with cc.Instance(0, 8, 48 ** 3, 128, 14) as inst, \
+            cc.VolumeBatch(inst, [v.shape for v in vols], 2, [0.01, 0.01], graph=True) as batch:
+        for st in streams + streams:
+            batch.set_stream(st)
+            back = [torch.zeros(v.shape, dtype=torch.float32, device="cuda") for v in vols]
+            torch.cuda.synchronize()
+            batch.compress(dv)
+            batch.decompress(back)
+            batch.status()
+            for i, (w, b) in enumerate(refs):
+                words, bits = batch.read_stream(i)
+                assert bits == b and np.array_equal(words, w)
+                assert np.array_equal(back[i].cpu().numpy(), outs[i])
