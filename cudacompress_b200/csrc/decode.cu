@@ -783,9 +783,10 @@ __global__ void __launch_bounds__(256) k_decZero(DecParams p) {
 // zero counts, fetched before its symbols are decoded, become positions in the
 // round by the lane of the block, four per step beside its 31 neighbours.
 // Rows are 36 elements: four 16-bit (8 bytes) per lane are free of conflicts.
-// Bound: instruction issue and shared memory (27 instructions per 32 zero
-// counts, 54 per 32 symbols, 64% and 49% of the issue slots), and the lane's
-// chain per symbol (lookup, length, next word) where a call has few blocks.
+// Bound: instruction issue and shared memory (two 256^3 volumes, 14 million
+// entries: 36 warp instructions per 32 zero counts and 73 per 32 symbols, 56%
+// and 46% of the issue slots), and the lane's chain per symbol (lookup, length,
+// next word) where a call has few blocks.
 // Three 256^3 streams (26 million entries): zero counts 61 -> 53, symbols 145
 // -> 126 us against words read from global memory, a scan over the warp per
 // block and round, and the limits searched in global memory; seven streams of

@@ -1312,7 +1312,8 @@ __device__ __forceinline__ void firEight(const float* w, float* o) {
 // groups) in registers when the barrier lets the outputs overwrite it.  The
 // taps and chains are those of rowsTile and colsTile, in their order, with the
 // intermediate rounded to float as there, so the results are bit-identical.
-// Bound: instruction issue (76% of the slots; 900 per thread for 14 outputs),
+// Bound: instruction issue (75% of the slots; 930 per warp for 14 outputs per
+// thread, of which the taps are 260),
 // then DRAM.  256^3: the Y and X passes 54 us, this 44 - 52 before rows were
 // mirrored without branches and addressed by byte pitches.
 template <bool kInverse>
