@@ -47,7 +47,7 @@ constexpr u32 kPlanChunk = 4096;
 // six blocks 2.5 and 4.7.
 constexpr u32 kLongBlocks = 1024;
 constexpr u32 kWidePerSM = 4;   // resident CTAs of 512 threads
-inline bool wideScan(u32 streams, u32 longest, u32 sms) { return longest >= kLongBlocks && streams <= kWidePerSM * sms; }
+inline bool wideBlockScan(u32 streams, u32 longest, u32 sms) { return longest >= kLongBlocks && streams <= kWidePerSM * sms; }
 constexpr u64 planPartWords(u64 tables) { return 8 * ((tables + kPlanChunk - 1) / kPlanChunk + 1); }
 
 // Leaves of a table whose Huffman build runs in shared memory (heap_merge.cuh's

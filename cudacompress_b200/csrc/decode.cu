@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(1024) k_decSymPlanCarry(DecParams p) {
 // SM: the work per table is a short chain of dependent steps), 512 in calls of
 // few, where the offsets of a long stream's blocks - 8 per thread and step -
 // and the lookup table take the time (129 tables of 256^3 streams: 35 -> 18
-// us): a table per SM, or as wideScan has it.  120 tables of six blocks 7.7 us
+// us): a table per SM, or as wideBlockScan has it.  120 tables of six blocks 7.7 us
 // and 6.2 wide, 580 of them 7.9 and 11.9; 400 of 1024 blocks 8.4 and 8.3, of
 // 2048 10.0 and 8.8.
 constexpr u32 kDecThreads = 64, kDecThreadsWide = 512;
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(256) k_decScan(DecParams p) {
     if ((threadIdx.x & 31u) == 0 && total > sd.n) atomicOr(p.errors, DEV_ERR_CORRUPT);
 }
 
-// The same with a CTA per stream (wideScan): a warp takes 38 us over the 16384
+// The same with a CTA per stream (wideBlockScan): a warp takes 38 us over the 16384
 // blocks of a 256^3 volume's band, 512 threads 13.
 __global__ void __launch_bounds__(512) k_decScanWide(DecParams p) {
     __shared__ u32 scratch[40];
@@ -1244,7 +1244,8 @@ static int launchDecodeBackEnd(cc_instance* I, const DecParams& p) {
     }
     {
         SectionTimer t(I, "dec.tables", st);
-        if (p.T <= I->smCount || wideScan(p.T, u32(ceilDiv(p.maxN, p.cb)), I->smCount)) k_decTables<kDecThreadsWide><<<p.T, kDecThreadsWide, 0, st>>>(p);
+        if (p.T <= I->smCount || wideBlockScan(p.T, u32(ceilDiv(p.maxN, p.cb)), I->smCount))
+            k_decTables<kDecThreadsWide><<<p.T, kDecThreadsWide, 0, st>>>(p);
         else k_decTables<kDecThreads><<<p.T, kDecThreads, 0, st>>>(p);
         countLaunch();
     }
@@ -1273,7 +1274,7 @@ static int launchDecodeBackEnd(cc_instance* I, const DecParams& p) {
         }
         {
             SectionTimer t(I, "dec.run_scan", st);
-            if (wideScan(p.nRl, u32(ceilDiv(p.rlMaxN, p.cb)), I->smCount)) k_decScanWide<<<p.nRl, 512, 0, st>>>(p);
+            if (wideBlockScan(p.nRl, u32(ceilDiv(p.rlMaxN, p.cb)), I->smCount)) k_decScanWide<<<p.nRl, 512, 0, st>>>(p);
             else k_decScan<<<u32(ceilDiv(p.nRl, 8)), 256, 0, st>>>(p);
             countLaunch();
         }

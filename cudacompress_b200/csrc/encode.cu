@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scanWide(EncParams p) {
 // without).  More streams: where the longest has more than 64 tiles, unless
 // that many CTAs would take longer than its warp (2 us per 1184).
 constexpr u32 kScanPlanStreams = 64;
-static bool scanWide(u32 streams, u32 tiles) {
+static bool wideTileScan(u32 streams, u32 tiles) {
     if (streams <= kScanPlanStreams) return ceilDiv(streams, 32) * ceilDiv(tiles, 32) > 4;
     return tiles > 64 && streams / 16 <= tiles;
 }
@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(1024) k_histPlan(EncParams p) {
     histPlanChunk(p, scratch);
 }
 
-// Passes 2 and 3 of a call of few and short streams in one CTA (scanWide).
+// Passes 2 and 3 of a call of few and short streams in one CTA (wideTileScan).
 
 __global__ void __launch_bounds__(1024) k_scanPlan(EncParams p) {
     __shared__ u32 scratch[33 * kPlanSums];
@@ -1254,7 +1254,7 @@ __global__ void __launch_bounds__(kScanWarps * 32) k_blockScan(EncParams p) {
     if ((threadIdx.x & 31u) == 0) p.meta[t].codeBits = total;
 }
 
-// The same with a CTA per table (wideScan): 512 threads over the 16384 blocks of
+// The same with a CTA per table (wideBlockScan): 512 threads over the 16384 blocks of
 // a 256^3 volume's band take 6 us, a warp 25.
 
 __global__ void __launch_bounds__(512) k_blockScanWide(EncParams p) {
@@ -1719,7 +1719,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
     countLaunch();
     if (p.totalTiles) { SectionTimer t(I, "enc.summary", st); k_summary<Sym><<<p.totalTiles, kRleThreads, 0, st>>>(p); countLaunch(); }
     const u32 chunks = std::max<u32>(1, u32(ceilDiv(p.T, kPlanChunk)));
-    const bool wide = scanWide(p.S, u32(ceilDiv(p.maxCount, kRleTile)));
+    const bool wide = wideTileScan(p.S, u32(ceilDiv(p.maxCount, kRleTile)));
     if (p.S <= kScanPlanStreams && !wide) {   // then one chunk
         SectionTimer t(I, "enc.hist_plan", st);
         k_scanPlan<<<1, 1024, 0, st>>>(p);
@@ -1759,7 +1759,7 @@ static int launchEncode(cc_instance* I, const EncParams& p) {
         { SectionTimer t(I, "enc.block_bits", st); k_blockBits<Sym><<<g, kPackWarps * 32, 0, st>>>(p); countLaunch(); }
         {
             SectionTimer t(I, "enc.block_scan", st);
-            if (wideScan(p.T, u32(ceilDiv(p.maxCount, p.cb)), sms)) k_blockScanWide<<<p.T, 512, 0, st>>>(p);
+            if (wideBlockScan(p.T, u32(ceilDiv(p.maxCount, p.cb)), sms)) k_blockScanWide<<<p.T, 512, 0, st>>>(p);
             else k_blockScan<<<u32(ceilDiv(p.T, kScanWarps)), kScanWarps * 32, 0, st>>>(p);
             countLaunch();
         }
